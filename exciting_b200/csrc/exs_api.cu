@@ -75,6 +75,8 @@ exs::OzAtomArgs exs_ctx::oz_atom_args() const
     a.lw = oz_lw;
     a.xs = d_xs;
     a.xsig = d_xsig;
+    a.nb = ring_nb;
+    a.nrows = ring_nrows;
     return a;
 }
 
@@ -381,10 +383,13 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
         return fail(c, EXS_ERR_ARG, "slices must be in 3..9");
     if (mode == EXS_PREC_OZAKI_MOD && slices != 0 && (slices < 6 || slices > exs::OZ_MAX_MODULI))
         return fail(c, EXS_ERR_ARG, "moduli must be 0 (automatic) or in 6..16");
-    const int kp8 = exs::oz_kpad(c->K);
+    const bool mod = mode == EXS_PREC_OZAKI_MOD;
+    const int kp8 = mod ? exs::ring_kpad(c->K) : exs::oz_kpad(c->K);
     exs::OzScheme sch{};
-    if (mode == EXS_PREC_OZAKI_MOD) {
-        if (exs::oz_mod_plan(slices, c->K, std::max(1, c->maxaa), &sch) != 0)
+    exs::OzRing ring{};
+    if (mod) {
+        if (exs::oz_mod_plan(slices, c->K, std::max(1, c->maxaa), &sch) != 0 ||
+            exs::oz_ring_plan(sch.b, sch.bx, &ring) != 0)
             return fail(c, EXS_ERR_SIZE, "no modular plan for this K (K <= 65536, at least 8 bits per operand)");
         slices = sch.n;
     } else {
@@ -396,43 +401,52 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
     cudaSetDevice(c->device);
     EXS_CUDA(cudaStreamSynchronize(c->stream));
     const int narr = c->relativity == EXS_REL_IORA ? 6 : 4;    // + Cr, Ci: O = A^H (I + h1aa) A
-    const size_t slot = exs::oz_slot_bytes(slices, c->npad, kp8, narr);
+    const size_t slot = mod ? exs::ring_slot_bytes(ring, c->npad, kp8, c->relativity)
+                            : exs::oz_slot_bytes(slices, c->npad, kp8, narr);
     if (c->d_oz) { cudaFree(c->d_oz); c->d_oz = nullptr; }
     if (c->d_res) { cudaFree(c->d_res); c->d_res = nullptr; c->res_bytes = 0; }
     if (c->d_pace) { cudaFree(c->d_pace); c->d_pace = nullptr; }
     if (c->d_ozscale) { cudaFree(c->d_ozscale); c->d_ozscale = nullptr; }
     if (c->d_xs) { cudaFree(c->d_xs); c->d_xs = nullptr; }
     if (c->d_xsig) { cudaFree(c->d_xsig); c->d_xsig = nullptr; }
-    // per-atom operands: windows of 128-byte chunks, 64-row blocks of h_a and lo rows
+    // per-atom operands: windows of 128-byte chunks; slices: 64-row blocks of h_a and lo rows, moduli:
+    // blocks of ring_nb rows of both
     int nch = 1;
     for (const AtomDesc &a : c->atoms) nch = std::max(nch, a.oz_nch);
     c->oz_lw = 128 * nch;
     c->oz_nfb = (c->maxaa + 63) / 64;
     c->oz_nxb = c->oz_nfb + (c->maxnlo + 63) / 64;
-    c->oz_xseg = mode == EXS_PREC_OZAKI_MOD ? 1 : exs::oz_seg_pairs(slices, c->oz_lw);
+    c->oz_xseg = mod ? 1 : exs::oz_seg_pairs(slices, c->oz_lw);
     sch.segx = c->oz_xseg;
-    const size_t xgroups = (size_t)c->natmtot * slices * c->oz_nxb;
-    // moduli: the residue tiles of the H/O products of a whole batch, for
-    // either tile width (the upper tiles of ngkmax G+k per k-point)
+    int rows = 1;
+    for (const AtomDesc &a : c->atoms) rows = std::max(rows, a.napw + a.losize);
+    exs::ring_row_blocks(rows, &c->ring_nb, &c->ring_nrows);
+    const size_t xgroups = (size_t)c->natmtot * (mod ? 2 * ring.n : slices * c->oz_nxb);
+    const size_t xs_bytes = xgroups * (mod ? c->ring_nrows : 128) * c->oz_lw;
+    const size_t nxsig = (size_t)c->natmtot * (mod ? c->ring_nrows : c->oz_nxb * 64);
+    // moduli: the residues of the H/O products of a whole batch (the upper tiles of ngkmax G+k per
+    // k-point); the per-atom products run before them in the same buffer, in chunks that fit it, of at
+    // least 256 MB where there is that much
     size_t res = 0;
-    if (mode == EXS_PREC_OZAKI_MOD)
-        for (int q : {0, 1, 8}) {
-            const int bj = exs::oz_res_cols(q), bi = exs::oz_res_rows(q);
-            size_t tiles = 0;      // 128-row residue tiles
-            for (int ib = 0; ib < (c->ngkmax + bi - 1) / bi; ib++)
-                for (int jb = 0; jb < (c->ngkmax + bj - 1) / bj; jb++)
-                    if (jb * bj + bj - 1 >= ib * bi) tiles += bi / 128;
-            res = std::max(res, tiles * exs::oz_res_tile_bytes(slices, q) * c->max_batch);
-        }
+    if (mod) {
+        size_t tiles = 0, atiles = 0;
+        const int nib = (c->ngkmax + 255) / 256;
+        for (int ib = 0; ib < nib; ib++)
+            for (int jb = 0; jb < (c->ngkmax + 127) / 128; jb++)
+                if (jb * 128 + 127 >= ib * 256) tiles++;
+        atiles = (size_t)c->natmtot * nib * (c->ring_nrows / c->ring_nb);
+        res = std::max(tiles * exs::ring_ho_tile_bytes(ring) * c->max_batch,
+                       std::min((size_t)256 << 20, atiles * exs::ring_atom_tile_bytes(ring, c->ring_nb) * c->max_batch));
+    }
     cudaError_t e = cudaMalloc((void **)&c->d_oz, slot * c->max_batch);
     if (e == cudaSuccess && res > 0) {
         e = cudaMalloc((void **)&c->d_res, res);
         if (e == cudaSuccess) c->res_bytes = res;
-        if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_pace, exs::oz_pace_bytes());
+        if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_pace, exs::ring_pace_bytes());
     }
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_ozscale, sizeof(double) * 3 * c->npad * c->max_batch);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_xs, xgroups * 128 * c->oz_lw);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_xsig, sizeof(double) * c->natmtot * c->oz_nxb * 64);
+    if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_xs, xs_bytes);
+    if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_xsig, sizeof(double) * nxsig);
     if (e != cudaSuccess || c->oz_xseg < 1) {
         c->prec_mode = EXS_PREC_FP64;
         return fail(c, e != cudaSuccess ? EXS_ERR_NOMEM : EXS_ERR_SIZE, "split-precision work space");
@@ -440,15 +454,20 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
     c->kp8 = kp8;
     c->oz_seg = seg;
     c->oz_slot_bytes = slot;
-    // the slices of all slots: (slot x slice) groups of 4 arrays x npad rows x kp8 bytes
-    const size_t nss = (size_t)slices * c->max_batch;
     bool maps_ok = true;
-    for (int q = 0; q < exs::OZ_NCFG; q++)
-        maps_ok = maps_ok && exs::make_oz_tensor_maps(c->d_oz, nss, c->npad, kp8, exs::OZ_CFG_KCH[q], narr,
-                                                      &c->oz_mapA[q], &c->oz_mapB[q], &c->oz_mapB2[q]);
-    maps_ok = maps_ok && exs::make_oz_atom_maps(c->d_oz, nss, c->npad, kp8, narr, c->d_xs, xgroups, c->oz_lw,
-                                                &c->oz_mapArow, &c->oz_mapX);
-    maps_ok = maps_ok && exs::make_oz_b64_map(c->d_oz, nss, c->npad, kp8, narr, &c->oz_mapB64, &c->oz_mapB64h);
+    if (mod) {
+        maps_ok = exs::make_ring_maps(c->d_oz, (size_t)2 * ring.n * c->max_batch, c->npad, kp8,
+                                      exs::ring_narr(c->relativity), c->d_xs, xgroups, c->ring_nrows, c->ring_nb,
+                                      c->oz_lw, &c->ring_mapHO, &c->ring_mapA, &c->ring_mapX);
+    } else {
+        // the slices of all slots: (slot x slice) groups of 4 arrays x npad rows x kp8 bytes
+        const size_t nss = (size_t)slices * c->max_batch;
+        for (int q = 0; q < exs::OZ_NCFG; q++)
+            maps_ok = maps_ok && exs::make_oz_tensor_maps(c->d_oz, nss, c->npad, kp8, exs::OZ_CFG_KCH[q], narr,
+                                                          &c->oz_mapA[q], &c->oz_mapB[q], &c->oz_mapB2[q]);
+        maps_ok = maps_ok && exs::make_oz_atom_maps(c->d_oz, nss, c->npad, kp8, narr, c->d_xs, xgroups, c->oz_lw,
+                                                    &c->oz_mapArow, &c->oz_mapX);
+    }
     if (!maps_ok) {
         cudaFree(c->d_oz); c->d_oz = nullptr;
         cudaFree(c->d_ozscale); c->d_ozscale = nullptr;
@@ -456,17 +475,17 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
         return fail(c, EXS_ERR_CUDA, "cuTensorMapEncodeTiled failed for the slice array");
     }
     c->slices = slices;
-    sch.wait = c->oz_wait;
+    sch.wait = ring.wait = c->oz_wait;
     c->oz_sch = sch;
+    c->oz_ring = ring;
     c->prec_mode = mode;
     if (c->have_inputs) {   // slices of the current h_a and loa
-        EXS_CUDA(exs::launch_oz_x(c->params(), c->oz_atom_args(), c->oz_sch, c->stream));
+        EXS_CUDA(exs::launch_x(c, c->stream));
         EXS_CUDA(cudaStreamSynchronize(c->stream));
     }
-    {   // a configuration the autotuner chose earlier for this shape; else, with moduli, the paced
-        // persistent two-SM residue tiles (1.5x the 128 x 64 tiles on the 216-atom cell)
+    {   // a configuration the autotuner chose earlier for this shape
         auto it = c->oz_tuned.find(std::make_tuple((int)mode, c->npad, c->K, slices));
-        c->oz_cfg = it != c->oz_tuned.end() ? it->second : (mode == EXS_PREC_OZAKI_MOD ? 10 : 0);
+        c->oz_cfg = it != c->oz_tuned.end() ? it->second : 0;
     }
     return EXS_OK;
 }
@@ -553,7 +572,7 @@ int exs_set_scf_inputs(exs_ctx *c, const exs_scf_inputs *in)
     if (!c->d_dlu) EXS_CUDA(dalloc(&c->d_dlu, (size_t)nat * (c->lmaxapw + 1) * exs::DLU_STRIDE));
     EXS_CUDA(exs::launch_match_dlu(c->params(), c->d_dlu, s));
     if (c->oz_on())   // slices of the new h_a and loa, in place
-        EXS_CUDA(exs::launch_oz_x(c->params(), c->oz_atom_args(), c->oz_sch, s));
+        EXS_CUDA(exs::launch_x(c, s));
     EXS_CUDA(cudaStreamSynchronize(s));
     c->have_inputs = true;
     return EXS_OK;
@@ -593,7 +612,7 @@ int exs_set_wait_limit(exs_ctx *c, long long cycles)
     if (cycles < 0) return fail(c, EXS_ERR_ARG, "negative wait limit");
     c->gen++;   // captured graphs carry the old limit
     c->oz_wait = cycles;
-    c->oz_sch.wait = cycles;
+    c->oz_sch.wait = c->oz_ring.wait = cycles;
     return EXS_OK;
 }
 
@@ -666,16 +685,15 @@ struct Uploaded {
 };
 
 // Upper tiles (128 rows x 32 columns, 256 x 32 for the two-SM tiles with ib
-// counting pairs of 128-row blocks, 128 x 32, 128 x 64 or 256 x 64 for the
-// residue tiles of the modular mode) of the split-precision contraction, in
-// groups of `group` row blocks x `gcols` column blocks (gcols 0: `group`;
-// row blocks outer, then column blocks, inside a group row blocks outer
-// again): the tiles that run at the same time (one
-// CTA per SM) then read about `group` row blocks of A and `group` column
-// blocks of B instead of one row block and ~148 column blocks, so the L2
-// serves the shared operand chunks and HBM streams each block about
-// (number of groups in its row or column) times instead of once per tile
-// row.  group = 1 is the plain row-major order.
+// counting pairs of 128-row blocks, 256 x 128 in the modular mode) of the
+// split-precision contraction, in groups of `group` row blocks x `gcols`
+// column blocks (gcols 0: `group`; row blocks outer, then column blocks,
+// inside a group row blocks outer again): the tiles that run at the same time
+// then read about `group` row blocks of A and `gcols` column blocks of B
+// instead of one row block and all column blocks, so the L2 serves the shared
+// operand chunks and HBM streams each block about (number of groups in its
+// row or column) times instead of once per tile row.  group = 1 is the plain
+// row-major order.
 void oz_tiles(const std::vector<KDesc> &ks, std::vector<int> &t, int rows, int cols, int group = 1, int gcols = 0)
 {
     t.clear();
@@ -695,20 +713,25 @@ void oz_tiles(const std::vector<KDesc> &ks, std::vector<int> &t, int rows, int c
     }
 }
 
-// Per-atom tiles {k, atom, G block of 128, row block of 64} of the
-// split-precision path: h_a A (row blocks 0..nfb-1) and the APW-lo rows
-// (blocks nfb..).
+// Per-atom tiles {k, atom, G block, row block} of the split-precision path:
+// h_a A and the APW-lo rows.  Slices: 128 G x 64 rows (row blocks 0..nfb-1 of
+// h_a, nfb.. of the lo rows); moduli: 256 G x ring_nb rows (h_a rows, then lo
+// rows).
 void oz_atom_tiles(const exs_ctx *c, const std::vector<KDesc> &ks, std::vector<int> &t)
 {
     for (size_t k = 0; k < ks.size(); k++)
         for (int ias = 0; ias < c->natmtot; ias++) {
             const AtomDesc &a = c->atoms[ias];
-            for (int ib = 0; ib < (ks[k].ngp + 127) / 128; ib++) {
-                for (int xb = 0; xb < (a.napw + 63) / 64; xb++) {
+            const int rows = c->oz_sch.mod ? 256 : 128;
+            for (int ib = 0; ib < (ks[k].ngp + rows - 1) / rows; ib++) {
+                auto add = [&](int xb) {
                     t.push_back((int)k); t.push_back(ias); t.push_back(ib); t.push_back(xb);
-                }
-                for (int lb = 0; lb < (a.losize + 63) / 64; lb++) {
-                    t.push_back((int)k); t.push_back(ias); t.push_back(ib); t.push_back(c->oz_nfb + lb);
+                };
+                if (c->oz_sch.mod) {
+                    for (int xb = 0; xb * c->ring_nb < a.napw + a.losize; xb++) add(xb);
+                } else {
+                    for (int xb = 0; xb < (a.napw + 63) / 64; xb++) add(xb);
+                    for (int lb = 0; lb < (a.losize + 63) / 64; lb++) add(c->oz_nfb + lb);
                 }
             }
         }
@@ -726,17 +749,8 @@ void pack_tables(exs_ctx *c, const std::vector<KDesc> &ks, std::vector<int> &ozt
     ozt.clear();
     std::vector<int> ozat;
     if (c->oz_on()) {
-        if (c->oz_sch.mod && (c->oz_cfg & 8)) {   // 256-row pairs, grouped 6 x 12, as two 128-row tiles each
-            std::vector<int> pairs;
-            oz_tiles(ks, pairs, 256, 64, 6, 12);
-            for (size_t t = 0; t < pairs.size(); t += 3)
-                for (int r = 0; r < 2; r++) {
-                    ozt.push_back(pairs[t]);
-                    ozt.push_back(2 * pairs[t + 1] + r);
-                    ozt.push_back(pairs[t + 2]);
-                }
-        } else if (c->oz_sch.mod)   // grouped 12 x 12 (about one wave of 148 CTAs)
-            oz_tiles(ks, ozt, 128, exs::oz_res_cols(c->oz_cfg), 12);
+        if (c->oz_sch.mod)   // grouped 6 x 12 (1536 x 1536, about one round of 74 clusters)
+            oz_tiles(ks, ozt, 256, 128, 6, 12);
         else
             oz_tiles(ks, ozt, (c->oz_cfg & 8) ? 256 : 128, 32);
         oz_atom_tiles(c, ks, ozat);
@@ -836,11 +850,11 @@ int upload_kdesc(exs_ctx *c, const std::vector<KDesc> &ks, Uploaded &u)
     return EXS_OK;
 }
 
-// Zero the column maxima that the A and B producers raise (split-precision
-// path only; the slots of one call are contiguous).
+// Zero the column maxima that the A and B producers raise (slices only; the
+// slots of one call are contiguous).
 cudaError_t oz_reset_maxima(exs_ctx *c, const std::vector<KDesc> &ks, cudaStream_t s)
 {
-    if (!c->oz_on() || ks.empty()) return cudaSuccess;
+    if (!c->oz_on() || c->oz_sch.mod || ks.empty()) return cudaSuccess;
     double *lo = ks[0].oz_scale, *hi = ks[0].oz_scale;
     for (const KDesc &k : ks) {
         lo = std::min(lo, k.oz_scale);
@@ -866,22 +880,31 @@ int enqueue_setup(exs_ctx *c, const std::vector<KDesc> &ks, const Uploaded &u, b
     if (!have_planes) EXS_CUDA(exs::launch_match_planes(p, u.d_k, (int)ks.size(), ngp_max, s));
     if (c->relativity == EXS_REL_IORA) EXS_CUDA(exs::launch_iora_planes(p, u.d_k, (int)ks.size(), ngp_max, s));
     EXS_EV(1);
-    const bool oz = c->oz_on();
-    if (oz && c->relativity == EXS_REL_IORA) {
-        // C = (I + h1aa) A, the right operand of O: its column bound (maximum or 2-norm), then its slices
-        EXS_CUDA(exs::launch_oz_colnorm(p, u.d_k, (int)ks.size(), 2, c->oz_sch.mod, s));
-        EXS_CUDA(exs::launch_oz_split(p, u.d_k, (int)ks.size(), c->oz_sch, c->kp8, 2, s));
-    }
+    const bool oz = c->oz_on(), mod = oz && c->oz_sch.mod;
+    const int nk = (int)ks.size();
+    // column bounds (2-norms with moduli; with slices the producers raised the maxima, but for C), then the
+    // slices or residues of operand `which`: 0 A, 1 B, 2 C
+    auto split = [&](int which) -> cudaError_t {
+        cudaError_t e = cudaSuccess;
+        if (mod) {
+            e = exs::launch_oz_norm(p, u.d_k, nk, which, s);
+            return e != cudaSuccess ? e : exs::launch_ring_split(p, u.d_k, nk, c->oz_ring, c->kp8, which, s);
+        }
+        if (which == 2) e = exs::launch_oz_colmax(p, u.d_k, nk, s);
+        return e != cudaSuccess ? e : exs::launch_oz_split(p, u.d_k, nk, c->oz_sch, c->kp8, which, s);
+    };
+    // C = (I + h1aa) A, the right operand of O
+    if (oz && c->relativity == EXS_REL_IORA) EXS_CUDA(split(2));
     // configuration bit 4: B = h_a A and the APW-lo rows in native FP64 even
     // when the H/O contraction is split
     const bool b64 = !oz || (c->oz_cfg & 16);
-    // moduli: the columns are scaled by their 2-norms (over the maxima the producers raised)
-    const bool norms = oz && c->oz_sch.mod;
     if (oz) {
-        // slices of A; B = h_a A and the APW-lo rows of H from the slices of h_a and loa
-        if (norms) EXS_CUDA(exs::launch_oz_colnorm(p, u.d_k, (int)ks.size(), 0, 1, s));
-        EXS_CUDA(exs::launch_oz_split(p, u.d_k, (int)ks.size(), c->oz_sch, c->kp8, 0, s));
-        if (!b64)
+        // A; B = h_a A and the APW-lo rows of H from the split h_a and loa
+        EXS_CUDA(split(0));
+        if (!b64 && mod)
+            EXS_CUDA(exs::launch_ring_atom(&c->ring_mapA, &c->ring_mapX, p, u.d_k, u.d_ozatiles, u.nozatiles,
+                                           c->oz_ring, c->oz_atom_args(), c->d_res, c->res_bytes, s));
+        else if (!b64)
             EXS_CUDA(exs::launch_oz_atom(c->oz_cfg, &c->oz_mapArow, &c->oz_mapX, p, u.d_k, u.d_ozatiles,
                                          u.nozatiles, c->oz_sch, c->kp8, c->oz_atom_args(), s));
     }
@@ -891,12 +914,11 @@ int enqueue_setup(exs_ctx *c, const std::vector<KDesc> &ks, const Uploaded &u, b
     }
     EXS_EV(2);
     if (oz) {
-        if (norms) EXS_CUDA(exs::launch_oz_colnorm(p, u.d_k, (int)ks.size(), 1, 1, s));
-        EXS_CUDA(exs::launch_oz_split(p, u.d_k, (int)ks.size(), c->oz_sch, c->kp8, 1, s));
+        EXS_CUDA(split(1));
         const int q = c->oz_cfg;
-        if (c->oz_sch.mod)   // residue tiles (one K chunk per stage: the maps of configuration 1), then the CRT
-            EXS_CUDA(exs::launch_oz_res(q, &c->oz_mapA[1], &c->oz_mapB[1], &c->oz_mapB64, &c->oz_mapB64h, p, u.d_k,
-                                        u.d_oztiles, u.noztiles, c->oz_sch, c->kp8, c->d_res, c->d_pace, s));
+        if (mod)
+            EXS_CUDA(exs::launch_ring_ho(&c->ring_mapHO, p, u.d_k, u.d_oztiles, u.noztiles, c->oz_ring, c->kp8,
+                                         c->d_res, c->d_pace, s));
         else
             EXS_CUDA(exs::launch_oz_mma(q, &c->oz_mapA[q], (q & 8) ? &c->oz_mapB2[q] : &c->oz_mapB[q], p, u.d_k,
                                         u.d_oztiles, u.noztiles, c->oz_sch, c->kp8, s));
@@ -1007,8 +1029,8 @@ int exs_autotune(exs_ctx *c, int nk, const int *ngp, const int *igpig_dev, const
     float best = 0.f;
     int best_q = 0;
     for (int q = 0; q < exs::OZ_NCFG; q++) {
-        if ((q & 8) && (q & 2) && !c->oz_sch.mod) continue;   // the slices' two-SM tiles have no persistent form
-        if ((q & 8) && c->oz_sch.mod && (q & 1)) continue;   // moduli: the two-SM residue tiles are 64 wide
+        if (c->oz_sch.mod && (q & 15)) continue;   // moduli: one H/O and one per-atom kernel
+        if ((q & 8) && (q & 2)) continue;   // the two-SM tiles have no persistent form
         if ((q & 16) && (q & 4)) continue;  // no per-atom int8 kernel to make persistent
         c->oz_cfg = q;
         Uploaded u{};                        // the tile list depends on the configuration

@@ -55,6 +55,9 @@ struct OzAtomArgs {
     int lw;                      // window bytes per row (multiple of 128)
     int8_t *xs;                  // slices [atom][slice][block][re, im][64][lw]
     double *xsig;                // row scales [atom][block][64]
+    // moduli: rows n = h_a rows, then lo rows, in blocks of nb (a multiple of 32); planes
+    // [atom][plane][nrows][lw] in xs, scales [atom][nrows] in xsig
+    int nb, nrows;
 };
 static_assert(OZ_NCFG == EXS_OZ_NCONFIG, "public configuration count");
 
@@ -64,40 +67,36 @@ static_assert(OZ_NCFG == EXS_OZ_NCONFIG, "public configuration count");
 //     segment for the H/O and the per-atom tiles);
 //   moduli (mod = 1): every column of A and B scaled by a power of two above
 //     its 2-norm and rounded to integers (b bits: the scaled column has norm
-//     <= 2^b; bx for the h_a / loa rows, scaled by their row norms), stored
-//     as residues modulo n pairwise coprime odd moduli p[m] (int8 in
-//     [-127, 127]); one int8 product per modulus.  By the Cauchy-Schwarz
-//     inequality an H/O product obeys |X| <= 2^(2b) (1 + eps)^2 with
-//     2^(2b + 2) <= M, and its residues are recombined by 96-bit constants
-//     c96 (residue tiles, oz_res_kernel / oz_crt_kernel): exact but for
-//     2^-64 M.  A per-atom product (|X| <= 2^(b + bx) (1 + eps)^2) is folded in
-//     the kernel into a 64-bit sum t += (v mod p[m]) c[m] (mod 2^64) with
-//     c[m] = round(2^(64+h) y_m / p[m]) mod 2^64 and 2^(b + bx + h + 2) <= M,
-//     so that t / 2^64 = 2^h X / M (mod 1) and t read as a signed integer is
-//     exact but for the rounding of the constants (sum |r| / 2 units of
-//     2^-(64+h) M; the h >= 5 headroom bits divide it by 2^h); the value is t
-//     times finx.  fin is the same factor for the H/O products folded in the
-//     64-bit form (2^(2b + h + 2) <= M does not hold for the plan's b: only
-//     the per-atom products use the fold).
+//     <= 2^b; bx for the h_a / loa rows, scaled by their row norms); the
+//     integer products are formed exactly in the rings of OzRing (oz_ring.cu).
+//     n and h are the plan's (exs_ozaki_moduli).
 constexpr int OZ_MAX_MODULI = 16;
 struct OzScheme {
     int mod, n, seg, segx, b, bx, h;
     long long wait;                    // limit of the pipeline waits in cycles (0: OZ_WAIT_CYCLES)
-    double fin, finx;
-    int p[OZ_MAX_MODULI];
-    int mg[OZ_MAX_MODULI];             // round(2^32 / p): quotient estimate by a multiply-high
-    float fp[OZ_MAX_MODULI], finv[OZ_MAX_MODULI];  // p and 1/p in FP32 (the split kernels)
-    float fc[3][OZ_MAX_MODULI];        // 2^13, 2^26, 2^39 mod p
-    unsigned long long c[OZ_MAX_MODULI];
-    // the H/O products (residue tiles): C_m = round(2^96 y_m / p_m) in 32-bit
-    // words (low first); the recombination reads the 64 bits below the top
-    // crt_shift bits of the 96-bit sum (the bits that |X| <= 2^2b leaves as
-    // sign copies when M is far above 2^2b), exact but for 2^-(64+crt_shift) M;
-    // fin96 = M 2^-(64+crt_shift) 2^-2b
-    unsigned c96[3][OZ_MAX_MODULI];
-    int crt_shift;
-    double fin96;
 };
+
+// The rings Z_p of the modular products (oz_ring.cu): n moduli p[m] in which
+// i_m^2 = -1 has a solution, two planes each.
+constexpr int OZ_RING_MAX = 16;
+struct OzRing {
+    int n, b, bx;
+    long long wait;                    // limit of the pipeline waits in cycles (0: OZ_WAIT_CYCLES)
+    int p[OZ_RING_MAX];
+    int mg[OZ_RING_MAX];               // round(2^32 / p): quotient estimate by a multiply-high
+    float inv[OZ_RING_MAX];            // 1 / p
+    // the split: symmetric residues of 2^(8k) (clo, chi: k = 0..3, 4..6) and of i_m 2^(8k) (ilo, ihi) as
+    // packed signed bytes; the sums' start values
+    int clo[OZ_RING_MAX], chi[OZ_RING_MAX], ilo[OZ_RING_MAX], ihi[OZ_RING_MAX];
+    int base[OZ_RING_MAX], icorr[OZ_RING_MAX];
+    // the recombination (two moduli at a time): weights of the real and imaginary parts, round(2^96 / (p p'))
+    unsigned fre[OZ_RING_MAX], fim[OZ_RING_MAX], d96[3][OZ_RING_MAX / 2];
+    int sh, shx;                       // 64-bit window below the top of the 96-bit sum: H/O, per-atom products
+    double fin, finx;                  // value of its unit: M 2^-(64+sh) 2^-2b, M 2^-(64+shx) 2^-(b+bx)
+};
+
+// Arrays of one plane: B, A, and with iora* (O = A^H C, C = (I + h1aa) A) C.
+__host__ __device__ __forceinline__ int ring_narr(int relativity) { return relativity == EXS_REL_IORA ? 3 : 2; }
 
 // atomicMax for non-negative doubles: their IEEE bit patterns order like
 // unsigned integers.
@@ -134,6 +133,25 @@ struct KDesc {
                              // 2-norms with moduli; the scale is the power of two above; null: FP64 path)
     int oz_slot;             // split-precision path: slot index in the slice tensor maps
 };
+
+// Column scale sigma(G) = 2^e with m < 2^e (frexp) for the column bound m in
+// oz_scale: with slices the column maximum that the producers of the A and B
+// planes raise (the matching kernels for A, the h_a A epilogue for B), with
+// moduli the column 2-norm (oz_norm_kernel).  An all-zero column gets
+// sigma = 1.
+__host__ __device__ __forceinline__ double oz_sigma(double m)
+{
+    int e = 0;
+    if (m > 0.0) frexp(m, &e);
+    return ldexp(1.0, e);
+}
+
+// Planes of operand `which` (0: A, 1: B, 2: C = (I + h1aa) A).
+__device__ __forceinline__ void oz_operand(const KDesc &k, int which, const double *&pr, const double *&pi)
+{
+    pr = which == 0 ? k.ar : (which == 1 ? k.br : k.cr);
+    pi = which == 0 ? k.ai : (which == 1 ? k.bi : k.ci);
+}
 
 // Constant per-context device parameters passed by value to kernels.
 // Per (atom, l) entry of DevParams::dlu: the n x n LU factors of D_l
@@ -294,10 +312,12 @@ struct exs_ctx {
     size_t oz_slot_bytes = 0;
     CUtensorMap oz_mapA[exs::OZ_NCFG], oz_mapB[exs::OZ_NCFG];   // TMA views of d_oz per pipeline configuration
     CUtensorMap oz_mapB2[exs::OZ_NCFG];                            // half-B views (two-SM tiles)
-    CUtensorMap oz_mapB64;                                         // B operand of the 128 x 64 residue tiles
-    CUtensorMap oz_mapB64h;                                        // one CTA's half of it in the 256 x 64 pairs
-    uint8_t *d_res = nullptr;                                      // residue tiles of the modular H/O products
-    int *d_pace = nullptr;                                         // pacing of the persistent pair kernel
+    // moduli: rings, TMA views (H/O operands, A by atom windows, h_a and loa), residues, pacing
+    exs::OzRing oz_ring{};
+    CUtensorMap ring_mapHO, ring_mapA, ring_mapX;
+    int ring_nb = 0, ring_nrows = 0;                               // row blocks of the per-atom tiles
+    uint8_t *d_res = nullptr;                                      // residues of the products of one launch
+    int *d_pace = nullptr;                                         // pacing of the product kernel
     size_t res_bytes = 0;
     int oz_cfg = 0;                   // pipeline configuration of the split-precision kernel
     // per-atom products of the split-precision path (h_a A, loa A)
@@ -356,15 +376,7 @@ cudaError_t launch_interstitial(const DevParams &p, int which, const KDesc *d_k,
 cudaError_t launch_oz_split(const DevParams &p, const KDesc *d_k, int nk, const OzScheme &sch, int kp8, int which,
                             cudaStream_t s);
 cudaError_t launch_oz_x(const DevParams &p, const OzAtomArgs &xa, const OzScheme &sch, cudaStream_t s);
-cudaError_t launch_oz_colnorm(const DevParams &p, const KDesc *d_k, int nk, int which, int norm, cudaStream_t s);
-cudaError_t launch_oz_res(int cfg, const CUtensorMap *mapA, const CUtensorMap *mapB32, const CUtensorMap *mapB64,
-                          const CUtensorMap *mapB64h, const DevParams &p, const KDesc *d_k, const void *d_tiles,
-                          int ntiles, const OzScheme &sch, int kp8, uint8_t *res, int *pace, cudaStream_t s);
-int oz_res_cols(int cfg);
-int oz_res_rows(int cfg);
-size_t oz_pace_bytes();
-size_t oz_res_tile_bytes(int n, int cfg);
-bool make_oz_b64_map(void *base, size_t nss, int npad, int kp8, int narr, CUtensorMap *mapB64, CUtensorMap *mapB64h);
+cudaError_t launch_oz_colmax(const DevParams &p, const KDesc *d_k, int nk, cudaStream_t s);
 cudaError_t launch_oz_atom(int cfg, const CUtensorMap *mapArow, const CUtensorMap *mapX, const DevParams &p,
                            const KDesc *d_k, const void *d_tiles, int ntiles, const OzScheme &sch, int kp8,
                            const OzAtomArgs &xa, cudaStream_t s);
@@ -379,5 +391,30 @@ extern const int OZ_CFG_KCH[OZ_NCFG], OZ_CFG_NST[OZ_NCFG];
 int oz_kpad(int K);
 size_t oz_slot_bytes(int S, int npad, int kp8, int narr);
 int oz_seg_pairs(int S, int kp8);
+// Modular contraction (oz_ring.cu)
 int oz_mod_plan(int n, int K, int kx, OzScheme *sch);
+int oz_ring_plan(int b, int bx, OzRing *out);
+int ring_kpad(int K);
+size_t ring_slot_bytes(const OzRing &rg, int npad, int kp8, int relativity);
+size_t ring_ho_tile_bytes(const OzRing &rg);
+size_t ring_atom_tile_bytes(const OzRing &rg, int nb);
+size_t ring_pace_bytes();
+void ring_row_blocks(int rows, int *nb, int *nrows);
+bool make_ring_maps(void *base, size_t nsp, int npad, int kp8, int narr, void *xbase, size_t xgroups, int nrows,
+                    int nb, int lw, CUtensorMap *ho, CUtensorMap *arow, CUtensorMap *x);
+cudaError_t launch_oz_norm(const DevParams &p, const KDesc *d_k, int nk, int which, cudaStream_t s);
+cudaError_t launch_ring_split(const DevParams &p, const KDesc *d_k, int nk, const OzRing &rg, int kp8, int which,
+                              cudaStream_t s);
+cudaError_t launch_ring_x(const DevParams &p, const OzAtomArgs &xa, const OzRing &rg, cudaStream_t s);
+cudaError_t launch_ring_ho(const CUtensorMap *map, const DevParams &p, const KDesc *d_k, const void *d_tiles,
+                           int ntiles, const OzRing &rg, int kp8, uint8_t *res, int *pace, cudaStream_t s);
+cudaError_t launch_ring_atom(const CUtensorMap *mapA, const CUtensorMap *mapX, const DevParams &p, const KDesc *d_k,
+                             const void *d_tiles, int ntiles, const OzRing &rg, const OzAtomArgs &xa, uint8_t *res,
+                             size_t res_bytes, cudaStream_t s);
+// Operands of h_a and loa for the active split arithmetic.
+inline cudaError_t launch_x(const exs_ctx *c, cudaStream_t s)
+{
+    return c->oz_sch.mod ? launch_ring_x(c->params(), c->oz_atom_args(), c->oz_ring, s)
+                         : launch_oz_x(c->params(), c->oz_atom_args(), c->oz_sch, s);
+}
 }  // namespace exs

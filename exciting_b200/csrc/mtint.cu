@@ -767,7 +767,7 @@ int enqueue_hmlint(exs_ctx *c, MtState &m, int lmaxvr, const double *apwfr, cons
     mt_angular_kernel<<<dim3((m.maxrows + 31) / 32, (m.maxrows + 7) / 8, nat), 256, 0, s>>>(a);
     MT_CUDA(cudaGetLastError());
     if (c->oz_on() && c->d_xs)
-        MT_CUDA(exs::launch_oz_x(c->params(), c->oz_atom_args(), c->oz_sch, s));
+        MT_CUDA(exs::launch_x(c, s));
     return EXS_OK;
 }
 

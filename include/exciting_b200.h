@@ -149,22 +149,26 @@ int exs_fderiv_int(int n, const double *x, const double *f, double *result);
 
 /* Select the MT contraction arithmetic: EXS_PREC_FP64 (native FP64),
  * EXS_PREC_OZAKI_INT8 with `slices` int8 slices per operand (3..9), or
- * EXS_PREC_OZAKI_MOD: the operands as integers modulo `slices` pairwise
- * coprime odd moduli (6..16; 0 = the fewest that keep 41 + log2(K)/2 bits
- * per 2-norm-scaled operand column for this context's K), one int8 product
- * per modulus, recombined by the Chinese remainder theorem.  No reference counterpart (the reference's
+ * EXS_PREC_OZAKI_MOD: the operands as integers of as many bits as `slices`
+ * pairwise coprime odd moduli up to 253 hold (6..16; 0 = the fewest that keep
+ * 41 + log2(K)/2 bits per 2-norm-scaled operand column for this context's K;
+ * exs_ozaki_moduli gives the bits), their products formed by int8 residues
+ * and recombined by the Chinese remainder theorem.  No reference counterpart (the reference's
  * contraction is zgemm in FP64). */
 int exs_set_precision(exs_ctx *ctx, int mode, int slices);
 
 /* The modular plan exs_set_precision(EXS_PREC_OZAKI_MOD, n) would use for a
  * contraction length K (2K products per real sum) and per-atom windows of
- * kx rows: the moduli p[0..n-1], the constants
- * c[m] = round(2^(64+h) y_m / p_m) mod 2^64 with y_m = (M / p_m)^-1 mod p_m,
- * M = prod p, the bits b of the A and B columns (scaled to 2-norm <= 2^b),
- * bx of the h_a / loa rows (likewise) and the headroom h of the 64-bit
- * recombination (2^(2b + h + 2) <= M and 2^(b + bx + h + 2) <= M).  n = 0
- * picks n as exs_set_precision does; *n_out receives it.  Any output pointer
- * may be NULL.  Host only. */
+ * kx rows: the bits b of the A and B columns (scaled to 2-norm <= 2^b), bx of
+ * the h_a / loa rows (likewise), which fix the integer products and with them
+ * H and O; the moduli p[0..n-1] whose product M = prod p sets them, and for a
+ * 64-bit recombination in these moduli the constants
+ * c[m] = round(2^(64+h) y_m / p_m) mod 2^64 with y_m = (M / p_m)^-1 mod p_m
+ * and its headroom h (2^(2b + 2) <= M and 2^(b + bx + h + 2) <= M).  The
+ * device forms the same integer products exactly modulo a second set of
+ * moduli, in which -1 is a square (csrc/oz_ring.cu).  n = 0 picks n as
+ * exs_set_precision does; *n_out receives it.  Any output pointer may be
+ * NULL.  Host only. */
 int exs_ozaki_moduli(int n, int K, int kx, int *n_out, int *p, unsigned long long *c, int *b, int *bx,
                      int *h);
 
@@ -348,21 +352,18 @@ int exs_autotune(exs_ctx *ctx, int nk, const int *ngp_host, const int *igpig_dev
                  exs_complex *const *o_dev, int *choice);
 
 /* Selects the split-precision kernel configuration by index
- * (0 .. EXS_OZ_NCONFIG-1) instead of the autotuner's choice: bit 0 picks the
- * pipeline shape of the H/O tiles (slices: two 96 KB stages or four 48 KB
- * stages; moduli: 128 x 64 or 128 x 32 residue tiles), bit 1 a persistent
- * launch (one block per SM walking the tiles) of the H/O tiles instead of
- * one block per tile, bit 2 the same for the per-atom products (h_a A,
- * APW-lo rows), bit 3 two-SM H/O tiles (a pair of blocks computes 256 x 32,
- * or 256 x 64 residue tiles with moduli, with the B operand split between
- * them; with slices bit 1 is then ignored, with moduli bit 0 is ignored and
- * bit 1 makes the pairs persistent, one cluster per SM pair), bit 4 the products
- * h_a A and the APW-lo rows of H in native FP64 (DMMA) instead of int8
- * slices (bit 2 is then ignored; only the H/O contraction stays split).
- * Configurations with the same bit 4 give bit-identical results; the two
- * arithmetics for h_a A agree to FP64 rounding.  Until the autotuner or
- * this call chooses, exs_set_precision sets 0 for slices and 10 (persistent
- * two-SM residue tiles) for moduli. */
+ * (0 .. EXS_OZ_NCONFIG-1) instead of the autotuner's choice.  Slices: bit 0
+ * picks the pipeline shape of the H/O tiles (two 96 KB stages or four 48 KB
+ * stages), bit 1 a persistent launch (one block per SM walking the tiles) of
+ * the H/O tiles instead of one block per tile, bit 2 the same for the per-atom
+ * products (h_a A, APW-lo rows), bit 3 two-SM H/O tiles (a pair of blocks
+ * computes 256 x 32 with the B operand split between them; bit 1 is then
+ * ignored).  Moduli have one form of each kernel and ignore bits 0-3.  Bit 4
+ * (both): the products h_a A and the APW-lo rows of H in native FP64 (DMMA)
+ * instead of int8 (bit 2 is then ignored; only the H/O contraction stays
+ * split).  Configurations with the same bit 4 give bit-identical results; the
+ * two arithmetics for h_a A agree to FP64 rounding.  Until the autotuner or
+ * this call chooses, exs_set_precision sets 0. */
 #define EXS_OZ_NCONFIG 32
 int exs_set_kernel_config(exs_ctx *ctx, int config);
 
