@@ -431,11 +431,12 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
     if (mod) {
         size_t tiles = 0, atiles = 0;
         const int nib = (c->ngkmax + 255) / 256;
+        const int cols = c->ring_cols = exs::ring_ho_cols(c->K);
         for (int ib = 0; ib < nib; ib++)
-            for (int jb = 0; jb < (c->ngkmax + 127) / 128; jb++)
-                if (jb * 128 + 127 >= ib * 256) tiles++;
+            for (int jb = 0; jb < (c->ngkmax + cols - 1) / cols; jb++)
+                if (jb * cols + cols - 1 >= ib * 256) tiles++;
         atiles = (size_t)c->natmtot * nib * (c->ring_nrows / c->ring_nb);
-        res = std::max(tiles * exs::ring_ho_tile_bytes(ring) * c->max_batch,
+        res = std::max(tiles * exs::ring_ho_tile_bytes(ring, cols) * c->max_batch,
                        std::min((size_t)256 << 20, atiles * exs::ring_atom_tile_bytes(ring, c->ring_nb) * c->max_batch));
     }
     cudaError_t e = cudaMalloc((void **)&c->d_oz, slot * c->max_batch);
@@ -458,7 +459,7 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
     if (mod) {
         maps_ok = exs::make_ring_maps(c->d_oz, (size_t)2 * ring.n * c->max_batch, c->npad, kp8,
                                       exs::ring_narr(c->relativity), c->d_xs, xgroups, c->ring_nrows, c->ring_nb,
-                                      c->oz_lw, &c->ring_mapHO, &c->ring_mapA, &c->ring_mapX);
+                                      c->oz_lw, &c->ring_mapHO1, &c->ring_mapHO2, &c->ring_mapA, &c->ring_mapX);
     } else {
         // the slices of all slots: (slot x slice) groups of 4 arrays x npad rows x kp8 bytes
         const size_t nss = (size_t)slices * c->max_batch;
@@ -749,8 +750,8 @@ void pack_tables(exs_ctx *c, const std::vector<KDesc> &ks, std::vector<int> &ozt
     ozt.clear();
     std::vector<int> ozat;
     if (c->oz_on()) {
-        if (c->oz_sch.mod)   // grouped 6 x 12 (1536 x 1536, about one round of 74 clusters)
-            oz_tiles(ks, ozt, 256, 128, 6, 12);
+        if (c->oz_sch.mod)   // grouped 6 x 12 or 9 x 9 tiles, about one round of 74 clusters
+            oz_tiles(ks, ozt, 256, c->ring_cols, c->ring_cols == 256 ? 9 : 6, c->ring_cols == 256 ? 9 : 12);
         else
             oz_tiles(ks, ozt, (c->oz_cfg & 8) ? 256 : 128, 32);
         oz_atom_tiles(c, ks, ozat);
@@ -917,7 +918,7 @@ int enqueue_setup(exs_ctx *c, const std::vector<KDesc> &ks, const Uploaded &u, b
         EXS_CUDA(split(1));
         const int q = c->oz_cfg;
         if (mod)
-            EXS_CUDA(exs::launch_ring_ho(&c->ring_mapHO, p, u.d_k, u.d_oztiles, u.noztiles, c->oz_ring, c->kp8,
+            EXS_CUDA(exs::launch_ring_ho(c->ring_cols, &c->ring_mapHO1, &c->ring_mapHO2, p, u.d_k, u.d_oztiles, u.noztiles, c->oz_ring, c->kp8,
                                          c->d_res, c->d_pace, s));
         else
             EXS_CUDA(exs::launch_oz_mma(q, &c->oz_mapA[q], (q & 8) ? &c->oz_mapB2[q] : &c->oz_mapB[q], p, u.d_k,

@@ -83,14 +83,19 @@ struct OzRing {
     int n, b, bx;
     long long wait;                    // limit of the pipeline waits in cycles (0: OZ_WAIT_CYCLES)
     int p[OZ_RING_MAX];
-    int mg[OZ_RING_MAX];               // round(2^32 / p): quotient estimate by a multiply-high
+    // quotient estimates by a multiply-high: round and floor of 2^32 / p; the multiple of p above 2^27
+    int mg[OZ_RING_MAX];
+    unsigned mf[OZ_RING_MAX];
+    int up[OZ_RING_MAX];
     float inv[OZ_RING_MAX];            // 1 / p
     // the split: symmetric residues of 2^(8k) (clo, chi: k = 0..3, 4..6) and of i_m 2^(8k) (ilo, ihi) as
     // packed signed bytes; the sums' start values
     int clo[OZ_RING_MAX], chi[OZ_RING_MAX], ilo[OZ_RING_MAX], ihi[OZ_RING_MAX];
     int base[OZ_RING_MAX], icorr[OZ_RING_MAX];
-    // the recombination (two moduli at a time): weights of the real and imaginary parts, round(2^96 / (p p'))
-    unsigned fre[OZ_RING_MAX], fim[OZ_RING_MAX], d96[3][OZ_RING_MAX / 2];
+    // the recombination (two moduli p, p' at a time): weights of the residues in the real and imaginary parts
+    // as packed signed bytes, their offset (a multiple of p p'), round(2^96 / (p p')) in 32-bit words
+    int wlo[2][OZ_RING_MAX / 2], whi[2][OZ_RING_MAX / 2], woff[OZ_RING_MAX / 2];
+    unsigned d96[3][OZ_RING_MAX / 2];
     int sh, shx;                       // 64-bit window below the top of the 96-bit sum: H/O, per-atom products
     double fin, finx;                  // value of its unit: M 2^-(64+sh) 2^-2b, M 2^-(64+shx) 2^-(b+bx)
 };
@@ -314,7 +319,8 @@ struct exs_ctx {
     CUtensorMap oz_mapB2[exs::OZ_NCFG];                            // half-B views (two-SM tiles)
     // moduli: rings, TMA views (H/O operands, A by atom windows, h_a and loa), residues, pacing
     exs::OzRing oz_ring{};
-    CUtensorMap ring_mapHO, ring_mapA, ring_mapX;
+    CUtensorMap ring_mapHO1, ring_mapHO2, ring_mapA, ring_mapX;
+    int ring_cols = 128;                                           // H/O tile columns
     int ring_nb = 0, ring_nrows = 0;                               // row blocks of the per-atom tiles
     uint8_t *d_res = nullptr;                                      // residues of the products of one launch
     int *d_pace = nullptr;                                         // pacing of the product kernel
@@ -396,18 +402,20 @@ int oz_mod_plan(int n, int K, int kx, OzScheme *sch);
 int oz_ring_plan(int b, int bx, OzRing *out);
 int ring_kpad(int K);
 size_t ring_slot_bytes(const OzRing &rg, int npad, int kp8, int relativity);
-size_t ring_ho_tile_bytes(const OzRing &rg);
+int ring_ho_cols(int K);
+size_t ring_ho_tile_bytes(const OzRing &rg, int cols);
 size_t ring_atom_tile_bytes(const OzRing &rg, int nb);
 size_t ring_pace_bytes();
 void ring_row_blocks(int rows, int *nb, int *nrows);
 bool make_ring_maps(void *base, size_t nsp, int npad, int kp8, int narr, void *xbase, size_t xgroups, int nrows,
-                    int nb, int lw, CUtensorMap *ho, CUtensorMap *arow, CUtensorMap *x);
+                    int nb, int lw, CUtensorMap *ho1, CUtensorMap *ho2, CUtensorMap *arow, CUtensorMap *x);
 cudaError_t launch_oz_norm(const DevParams &p, const KDesc *d_k, int nk, int which, cudaStream_t s);
 cudaError_t launch_ring_split(const DevParams &p, const KDesc *d_k, int nk, const OzRing &rg, int kp8, int which,
                               cudaStream_t s);
 cudaError_t launch_ring_x(const DevParams &p, const OzAtomArgs &xa, const OzRing &rg, cudaStream_t s);
-cudaError_t launch_ring_ho(const CUtensorMap *map, const DevParams &p, const KDesc *d_k, const void *d_tiles,
-                           int ntiles, const OzRing &rg, int kp8, uint8_t *res, int *pace, cudaStream_t s);
+cudaError_t launch_ring_ho(int cols, const CUtensorMap *map1, const CUtensorMap *map2, const DevParams &p,
+                           const KDesc *d_k, const void *d_tiles, int ntiles, const OzRing &rg, int kp8, uint8_t *res,
+                           int *pace, cudaStream_t s);
 cudaError_t launch_ring_atom(const CUtensorMap *mapA, const CUtensorMap *mapX, const DevParams &p, const KDesc *d_k,
                              const void *d_tiles, int ntiles, const OzRing &rg, const OzAtomArgs &xa, uint8_t *res,
                              size_t res_bytes, cudaStream_t s);

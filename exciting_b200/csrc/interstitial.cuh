@@ -5,11 +5,11 @@
 
 namespace exs {
 
-// Interstitial term of element (i, j), i <= j < ngp (hmlistln.f90:61-86,
-// olpistln.f90:53-82).  Returns false when nothing is added.  The tables are
-// read-only during every kernel that calls this (read-only data path).
-__device__ __forceinline__ bool interstitial(const DevParams &p, int kind, const int *ivi, const int *ivj,
-                                             const double *vi, const double *vj, double &zr, double &zi)
+// Index (1-based) of G_i - G_j in the G list, 0 when nothing is added there
+// (outside ngvec); a difference outside the box raises the device flag.  The
+// tables are read-only during every kernel that calls this (read-only data
+// path).
+__device__ __forceinline__ int interstitial_index(const DevParams &p, const int *ivi, const int *ivj)
 {
     const int d0 = ivi[0] - ivj[0] - p.intgv_lo[0];
     const int d1 = ivi[1] - ivj[1] - p.intgv_lo[1];
@@ -17,10 +17,17 @@ __device__ __forceinline__ bool interstitial(const DevParams &p, int kind, const
     if ((unsigned)d0 >= (unsigned)p.intgv_n[0] || (unsigned)d1 >= (unsigned)p.intgv_n[1] ||
         (unsigned)d2 >= (unsigned)p.intgv_n[2]) {
         atomicOr(p.err, DEV_ERR_INDEX);
-        return false;
+        return 0;
     }
     const int ig = __ldg(p.ivgig + d0 + p.intgv_n[0] * (d1 + p.intgv_n[1] * d2));
-    if (ig <= 0 || ig > p.ngvec) return false;
+    return ig > p.ngvec ? 0 : max(ig, 0);
+}
+
+// Interstitial H or O term at G index ig > 0 (hmlistln.f90:61-86,
+// olpistln.f90:53-82).
+__device__ __forceinline__ void interstitial_value(const DevParams &p, int kind, int ig, const double *vi,
+                                                   const double *vj, double &zr, double &zi)
+{
     const double dp = vi[0] * vj[0] + vi[1] * vj[1] + vi[2] * vj[2];
     if (kind == EPI_HAM) {
         const double t1 = 0.5 * dp;
@@ -44,6 +51,16 @@ __device__ __forceinline__ bool interstitial(const DevParams &p, int kind, const
             zi = c.im;
         }
     }
+}
+
+// Interstitial term of element (i, j), i <= j < ngp.  Returns false when
+// nothing is added.
+__device__ __forceinline__ bool interstitial(const DevParams &p, int kind, const int *ivi, const int *ivj,
+                                             const double *vi, const double *vj, double &zr, double &zi)
+{
+    const int ig = interstitial_index(p, ivi, ivj);
+    if (ig <= 0) return false;
+    interstitial_value(p, kind, ig, vi, vj, zr, zi);
     return true;
 }
 

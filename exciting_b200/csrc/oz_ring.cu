@@ -52,12 +52,9 @@ namespace exs {
 
 constexpr int RG_CHUNK = 128;                    // bytes of K in one swizzle row
 constexpr int RG_BOX = 128 * RG_CHUNK;           // 16 KB: one K chunk of 128 operand rows
-constexpr int RG_KCH = 2;                        // K chunks per stage
-constexpr int RG_STAGE = 2 * RG_KCH * RG_BOX;    // 64 KB: this CTA's A rows, then its half of B
-constexpr int RG_NST = 3;
-constexpr int RG_SMEM = RG_NST * RG_STAGE + 1024;
-constexpr int RG_THREADS = 384;                  // 12 warps: see the roles below
-constexpr int RG_BM = 256, RG_BJ = 128;          // H/O tile of a CTA pair: 256 G_i x 128 G_j
+constexpr int RG_EPI = 16;                       // epilogue warps of a CTA
+constexpr int RG_THREADS = 128 + 32 * RG_EPI;    // see the roles below
+constexpr int RG_BM = 256;                       // tile rows of a CTA pair
 constexpr int RG_ACC = 256;                      // tensor-memory columns of one accumulator
 
 // ------------------------------------------------------------ residues
@@ -290,48 +287,64 @@ __global__ void __launch_bounds__(256) oz_ring_x_kernel(DevParams p, OzAtomArgs 
 // ------------------------------------------------------------ the products
 // A cluster of two CTAs forms tiles of 256 rows with tcgen05.mma.cta_group::2
 // (M = 256): each CTA holds its own 128 rows of the A operand and half of the
-// B operand's N rows.
-//   RG_HO    tiles {k, ib, jb}: 256 G_i x 128 G_j, N = 256: CTA 0 holds B_P,
-//            CTA 1 A_(P^1) (C_P with iora*) of the G_j; columns 0..127 of the
-//            sums are H, 128..255 O
+// N rows of each B operand.
+//   RG_HO    tiles {k, ib, jb}: 256 G_i x 128 G_j, one MMA of N = 256: CTA 0
+//            holds B_P, CTA 1 A_(P^1) (C_P with iora*) of the G_j; columns
+//            0..127 of the sums are H, 128..255 O
+//   RG_WIDE  tiles {k, ib, jb}: 256 G_i x 256 G_j, two MMAs of N = 256 on the
+//            same A operand, one for H and one for O
 //   RG_ATOM  tiles {k, atom, ib, xb}: 256 G x nb rows of h_a and loa of one
 //            atom (N = nb, a multiple of 32), over the atom's K window
 // The work list is flat in (tile, plane): while full rounds of one tile per
 // cluster last, a cluster takes a tile and walks its 2n planes; the (tile,
-// plane) pairs of the remaining tiles are dealt out one by one, so that a
+// plane) pairs of the remaining tiles are dealt out in equal runs, so that a
 // handful of tiles (two for a k-point of the two-atom cell) still occupies
 // every SM pair and the last round is never short of more than one product.
-// Two accumulators in tensor memory: the MMAs of one product run while the
-// epilogue reduces the previous one.
+// Two accumulators in tensor memory.  RG_HO, RG_ATOM: products take them in
+// turn, the MMAs of one run while the epilogue reduces the previous one.
+// RG_WIDE: every product fills both, and the epilogue frees H while O waits.
 //
-// Roles (384 threads): warp 0 / 1 TMA producers of the A / B operand, warp 3
-// MMA issuer (CTA 0) and tensor-memory owner, warps 4-11 epilogue: two per
-// tensor-memory lane quadrant, half the columns each; residues of 16 columns
-// leave as 16 bytes per row, 512 contiguous bytes per warp.
+// Roles (640 threads): warps 0, 1 (and 2) TMA producers of the A and B (O)
+// operands, warp 3 MMA issuer (CTA 0) and tensor-memory owner, warps 4-19
+// epilogue: four per tensor-memory lane quadrant, every fourth chunk of 16
+// columns each, whose residues leave as 16 bytes per row, 512 contiguous
+// bytes per warp.  (Eight warps: 4 % slower on the per-atom products,
+// where the reduction of a short product is a chain of latencies.)
 // CTA 0's full barriers count the bytes of both CTAs' copies; MMA completion
 // is committed to both CTAs; both epilogues report to CTA 0's barrier.
 // Every wait is bounded and gives up when another role of the CTA gave up;
 // the kernel then lets its copies and MMAs drain, records DEV_ERR_TIMEOUT,
 // frees tensor memory and returns.
 //
-// What bounds it: the L2 -> SM operand stream (32 KB per K chunk and CTA
-// against 512 cycles of MMAs) while K is long.  Measured, H/O: 64 atoms (N =
-// 8075, K = 10,368) 14.4 ms, 27 k-points of the eight-atom cell 1.50 ms; the
-// real-and-imaginary form with 13 moduli, 256 x 64 tiles and one accumulator
-// set took 23.1 and 2.65 ms.  Per-atom products with their recombination: 3.6
-// and 2.5 ms, against 4.07 and 2.21 ms for 128 x 64 tiles with 64-bit sums in
-// tensor memory (L2 -> SM stream of 25.8 GB in the eight-atom batch).
-enum : int { RG_HO = 0, RG_ATOM = 1 };
+// What bounds it: the power cap while K is long (64 atoms, N = 8075, K =
+// 10,368: 13.9 - 14.6 ms from box to box, 2.8 POP/s, the SM clock down to
+// 1.5 GHz; the form with real and imaginary planes, 13 moduli and 256 x 64
+// tiles took 23.1 ms); HBM for the per-atom products (64 atoms 1.25 ms, the 27
+// k-points of the eight-atom cell 0.95 ms at about 4.5 TB/s of residues out
+// and operands in).  H/O of the 27 k-points 1.46 - 1.57 ms (was 2.65).
+enum : int { RG_HO = 0, RG_ATOM = 1, RG_WIDE = 2 };
+
+template <int MODE>
+struct RingCfg {
+    static constexpr bool WIDE = MODE == RG_WIDE;
+    static constexpr int KCH = WIDE ? 1 : 2;             // K chunks per stage
+    static constexpr int NB = WIDE ? 2 : 1;              // B operands (accumulators per product)
+    static constexpr int OPER = KCH * RG_BOX;            // one operand of a stage
+    static constexpr int STAGE = (1 + NB) * OPER;        // this CTA's A rows, then its half of each B
+    static constexpr int NST = WIDE ? 4 : 3;             // 192 KB in all
+    static constexpr int SMEM = NST * STAGE + 1024;
+    static constexpr int BJ = WIDE ? 256 : 128;          // H/O tile columns
+};
 
 // Pacing of large H/O launches (pace != null): every cluster publishes, every
-// RG_PACE_STAGES stages it issues, its step count in pace[cluster] and waits
+// RG_PACE_CHUNKS K chunks it issues, its step count in pace[cluster] and waits
 // until the slowest cluster is at most RG_PACE_LAG steps behind, so that the
 // tiles running at one time read the same row and column blocks within a few
 // MB of each other's position and the L2 serves the repeats.  The wait is a
 // hint, not a dependency: it gives up after RG_PACE_CYCLES (a cluster that is
 // not resident, or a slow one, delays the others by that much per step at
 // most) and never raises an error.  A finished cluster publishes INT_MAX.
-constexpr int RG_PACE_STAGES = 16;                // 32 K chunks
+constexpr int RG_PACE_CHUNKS = 32;
 constexpr int RG_PACE_LAG = 1;
 constexpr long long RG_PACE_CYCLES = 40000;
 constexpr int RG_PACE_MAX = 1024;                 // clusters (ints of the pace array)
@@ -359,6 +372,15 @@ __device__ __forceinline__ void ring_pace(int *pace, int me, int ncl, int step)
     st_relaxed_gpu(pace + me, step);
 }
 
+// An arrival that orders nothing but the tensor-memory reads before it, which
+// tcgen05.wait::ld has completed: a release here would make the warp wait
+// until its residue stores are performed (per-atom products of 64 atoms: 2.19 ms
+// with release, 1.36 ms without).
+__device__ __forceinline__ void mbar_arrive_relaxed(uint32_t cluster_addr)
+{
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
+}
+
 __device__ __forceinline__ void tma_load_4d_2sm(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, int c3,
                                                 uint32_t bar)
 {
@@ -369,31 +391,60 @@ __device__ __forceinline__ void tma_load_4d_2sm(uint32_t dst, const CUtensorMap 
         : "memory");
 }
 
-// The flat work list of cluster c: count() products, at(i) the i-th.
+// The flat work list of cluster c, walked by every role: np products of each
+// of its full-round tiles, then its run of the (tile, plane) pairs of the
+// remaining tiles.
 struct RingUnits {
-    int ncl, np, full, rest;         // full rounds of one tile per cluster, remaining tiles
-    __device__ RingUnits(int ntiles, int ncl_, int np_) : ncl(ncl_), np(np_), full(ntiles / ncl_), rest(ntiles % ncl_) {}
-    __device__ int count(int c) const { return full * np + (rest * np - c + ncl - 1) / ncl; }
-    __device__ void at(int i, int c, int &tile, int &P) const
+    int ncl, np, count, tile, P, full_end, rest_tile, rest_P;
+    __device__ RingUnits(int ntiles, int ncl_, int np_, int c) : ncl(ncl_), np(np_)
     {
-        if (i < full * np) {
-            tile = (i / np) * ncl + c;
-            P = i % np;
-        } else {
-            const int v = (i - full * np) * ncl + c;
-            tile = full * ncl + v % rest;
-            P = v / rest;
+        const int full = ntiles / ncl;
+        const long long pairs = (long long)(ntiles - full * ncl) * np;
+        const int first = (int)(pairs * c / ncl);
+        count = full * np + (int)(pairs * (c + 1) / ncl) - first;
+        full_end = full * ncl;
+        rest_tile = full_end + first / np;
+        rest_P = first % np;
+        tile = full > 0 ? c : rest_tile;
+        P = full > 0 ? 0 : rest_P;
+    }
+    __device__ void next()
+    {
+        if (++P < np) return;
+        P = 0;
+        if (tile >= full_end) {          // in the run of the remaining tiles
+            tile++;
+            return;
+        }
+        tile += ncl;
+        if (tile >= full_end) {
+            tile = rest_tile;
+            P = rest_P;
         }
     }
 };
 
-// Residue of an int32 sum in [0, p): q = floor(v mg / 2^32), mg = round(2^32 / p),
-// leaves v - q p in [-p/4, 5p/4]; the unsigned minima add or take p.
+// Residue bytes of an int32 sum |v| < 2^30: q = floor(v mg / 2^32), mg =
+// round(2^32 / p), leaves v - q p in [-p/4, 5p/4]; the unsigned minima add or
+// take p.
 __device__ __forceinline__ uint32_t ring_mod(int v, int p, int mg)
 {
     uint32_t x = (uint32_t)(v - __mulhi(v, mg) * p);
     x = min(x, x + (uint32_t)p);
     return min(x, x - (uint32_t)p);
+}
+
+// The same for |v| < 2^27 (K <= RG_SHORT_K, |residue| <= 123) in half the
+// instructions: with x = v + up, up = the multiple of p just above 2^27, and
+// mf = floor(2^32 / p), q = floor(x mf / 2^32) is at most floor(x / p), and
+// x - q p <= p + p f / 16, f = frac(2^32 / p): at most 246 for every modulus
+// of the table, a byte, though not always below p (the recombination takes
+// any representative below 2 p).
+constexpr int RG_SHORT_K = 8192;
+__device__ __forceinline__ uint32_t ring_mod_short(int v, int p, uint32_t mf, int up)
+{
+    const uint32_t x = (uint32_t)(v + up);
+    return x - __umulhi(x, mf) * (uint32_t)p;
 }
 
 template <int MODE>
@@ -402,8 +453,10 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                 const KDesc *ks, const int *tiles, int ntiles, const __grid_constant__ OzRing rg, OzAtomArgs xa,
                 uint8_t *res, int *pace)
 {
+    using C = RingCfg<MODE>;
+    constexpr int NST = C::NST, KCH = C::KCH;
     extern __shared__ __align__(1024) uint8_t rg_smem[];
-    __shared__ uint64_t full[RG_NST], empty[RG_NST], accf[2], acce[2];
+    __shared__ uint64_t full[NST], empty[NST], accf[2], acce[2];
     __shared__ uint32_t tmem_sh;
     __shared__ int abort_sh;
     volatile int *abort = &abort_sh;
@@ -412,10 +465,9 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     const uint32_t rank = cluster_ctarank();
     const uint32_t sbase = (smem_u32(rg_smem) + 1023u) & ~1023u;
     const int cl = (int)(blockIdx.x >> 1), NP = 2 * rg.n;
-    const RingUnits units(ntiles, (int)(gridDim.x >> 1), NP);
-    const int nu = units.count(cl);
-    const int N = MODE == RG_HO ? 2 * RG_BJ : xa.nb;
-    const int b_rows = N / 2;                            // operand rows of B in this CTA
+    RingUnits units(ntiles, (int)(gridDim.x >> 1), NP, cl);
+    const int N = MODE == RG_ATOM ? xa.nb : 256;         // MMA N
+    const int b_rows = N / 2;                            // operand rows of a B operand in this CTA
 
     if (warp == 3) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_sh)),
@@ -423,13 +475,13 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::);
     }
     if (tid == 0) {
-        for (int q = 0; q < RG_NST; q++) {
+        for (int q = 0; q < NST; q++) {
             mbar_init(&full[q], 1);      // CTA 0: one arrive (with the bytes of both CTAs)
             mbar_init(&empty[q], 1);
         }
         for (int a = 0; a < 2; a++) {
             mbar_init(&accf[a], 1);
-            mbar_init(&acce[a], 16);     // CTA 0: eight epilogue warps in each CTA
+            mbar_init(&acce[a], 2 * RG_EPI);     // CTA 0: the epilogue warps of both CTAs
         }
         abort_sh = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -440,79 +492,76 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     tc_fence_after();
     const uint32_t tbase = tmem_sh;
 
-    if (warp < 2) {
+    if (warp < 1 + C::NB) {
         // ------------------------------------------------ TMA producers (both CTAs)
         if (lane == 0) {
-            const int role = warp;       // 0: this CTA's A rows, 1: this CTA's half of B
-            uint32_t fills[RG_NST];
+            const int role = warp;       // 0: this CTA's A rows, 1 (2): this CTA's half of B (of O's operand)
+            uint32_t fills[NST];
 #pragma unroll
-            for (int q = 0; q < RG_NST; q++) fills[q] = 0;
-            int st = 0, issued = 0;
+            for (int q = 0; q < NST; q++) fills[q] = 0;
+            int st = 0, chunks = 0, last = -1;
             bool bad = false;
             const bool pacer = pace != nullptr && rank == 0 && role == 0;
-            for (int u = 0; u < nu && !bad; u++) {
-                int tile, P;
-                units.at(u, cl, tile, P);
-                int slot, row, arr, plane, x0 = 0, nch;
-                if (MODE == RG_HO) {
-                    slot = ks[tiles[3 * tile]].oz_slot;
-                    nch = (p.K + RG_CHUNK - 1) / RG_CHUNK;
-                    if (role == 0) {
-                        row = tiles[3 * tile + 1] * RG_BM + (int)rank * 128;
-                        arr = 1;
-                        plane = P;
-                    } else {             // H: B_P; O: A_(P^1), or C_P with iora*
-                        row = tiles[3 * tile + 2] * RG_BJ;
-                        arr = rank == 0 ? 0 : (p.relativity == EXS_REL_IORA ? 2 : 1);
-                        plane = (rank == 0 || arr == 2) ? P : (P ^ 1);
-                    }
-                } else {
-                    const int ias = tiles[4 * tile + 1];
-                    const AtomDesc &at = p.atoms[ias];
-                    nch = at.oz_nch;
-                    if (role == 0) {
-                        slot = ks[tiles[4 * tile]].oz_slot;
-                        row = tiles[4 * tile + 2] * RG_BM + (int)rank * 128;
-                        x0 = at.oz_x0;
+            int slot = 0, row = 0, arr = 1, flip = 0, x0 = 0, nch = (p.K + RG_CHUNK - 1) / RG_CHUNK;
+            if (MODE != RG_ATOM && role > 0) {           // H: B_P; O: A_(P^1), or C_P with iora*
+                const bool o = C::WIDE ? role == 2 : rank == 1;
+                arr = !o ? 0 : (p.relativity == EXS_REL_IORA ? 2 : 1);
+                flip = o && arr == 1 ? 1 : 0;
+            }
+            for (int u = 0; u < units.count && !bad; u++, units.next()) {
+                const int tile = units.tile, P = units.P;
+                if (tile != last) {      // what depends on the tile: dependent loads, once per tile
+                    last = tile;
+                    if (MODE == RG_ATOM) {
+                        const int ias = tiles[4 * tile + 1];
+                        const AtomDesc &at = p.atoms[ias];
+                        nch = at.oz_nch;
+                        if (role == 0) {
+                            slot = ks[tiles[4 * tile]].oz_slot;
+                            row = tiles[4 * tile + 2] * RG_BM + (int)rank * 128;
+                            x0 = at.oz_x0;
+                        } else {
+                            slot = ias;
+                            row = tiles[4 * tile + 3] * N + (int)rank * b_rows;
+                        }
                     } else {
-                        slot = ias;
-                        row = tiles[4 * tile + 3] * xa.nb + (int)rank * b_rows;
+                        slot = ks[tiles[3 * tile]].oz_slot;
+                        row = role == 0 ? tiles[3 * tile + 1] * RG_BM + (int)rank * 128
+                                        : tiles[3 * tile + 2] * C::BJ + (C::WIDE ? (int)rank * 128 : 0);
                     }
-                    arr = 1;
-                    plane = P;
                 }
-                for (int kb = 0; kb < nch; kb += RG_KCH, issued++) {
-                    if (pacer && issued % RG_PACE_STAGES == 0) ring_pace(pace, cl, units.ncl, issued / RG_PACE_STAGES);
+                const int plane = slot * NP + (P ^ flip);
+                for (int kb = 0; kb < nch; kb += KCH, chunks += KCH) {
+                    if (pacer && chunks % RG_PACE_CHUNKS == 0) ring_pace(pace, cl, units.ncl, chunks / RG_PACE_CHUNKS);
                     if (fills[st] > 0 && !mbar_wait_ab(&empty[st], (fills[st] - 1) & 1, abort, rg.wait)) {
                         bad = true;
                         break;
                     }
-                    const int nc = min(RG_KCH, nch - kb);
+                    const int nc = min(KCH, nch - kb);
                     const uint32_t bar = smem_u32(&full[st]);
-                    const uint32_t dst = sbase + st * RG_STAGE + role * RG_KCH * RG_BOX;
-                    if (MODE == RG_HO) {                 // one box of two K chunks (zeros past the last one)
-                        if (rank == 0 && role == 0) mbar_expect_tx(&full[st], 2 * RG_STAGE);
-                        tma_load_5d_2sm(dst, &mapA, 0, row, arr, kb, slot * NP + plane, bar);
+                    const uint32_t dst = sbase + st * C::STAGE + role * C::OPER;
+                    if (MODE != RG_ATOM) {               // one box of KCH chunks (zeros past the last one)
+                        if (rank == 0 && role == 0) mbar_expect_tx(&full[st], 2 * C::STAGE);
+                        tma_load_5d_2sm(dst, &mapA, 0, row, arr, kb, plane, bar);
                     } else {
                         if (rank == 0 && role == 0)
                             mbar_expect_tx(&full[st], 2 * nc * (RG_BOX + b_rows * RG_CHUNK));
                         for (int c = 0; c < nc; c++) {
                             if (role == 0)
-                                tma_load_4d_2sm(dst + c * RG_BOX, &mapA, x0 + (kb + c) * RG_CHUNK, row, arr,
-                                                slot * NP + plane, bar);
+                                tma_load_4d_2sm(dst + c * RG_BOX, &mapA, x0 + (kb + c) * RG_CHUNK, row, 1, plane, bar);
                             else
-                                tma_load_4d_2sm(dst + c * RG_BOX, &mapB, 0, row, slot * NP + plane, kb + c, bar);
+                                tma_load_4d_2sm(dst + c * RG_BOX, &mapB, 0, row, plane, kb + c, bar);
                         }
                     }
                     fills[st]++;
-                    st = (st + 1 == RG_NST) ? 0 : st + 1;
+                    st = (st + 1 == NST) ? 0 : st + 1;
                 }
             }
             if (pacer) st_relaxed_gpu(pace + cl, 0x7fffffff);     // done: nobody waits for this cluster
             // copies already issued (both CTAs') must land before the pair goes away: CTA 0 waits on its full
             // barriers, CTA 1, whose copies signal CTA 0's barriers, lets far more than their time pass
             if (bad && rank == 0)
-                for (int q = 0; q < RG_NST; q++)
+                for (int q = 0; q < NST; q++)
                     if (fills[q] > 0) mbar_drain(&full[q], (fills[q] - 1) & 1);
             if (bad && rank == 1)
                 for (const long long t0 = clock64(); clock64() - t0 < 1000000;) {
@@ -522,84 +571,109 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         // ------------------------------------------------ MMA issuer (CTA 0)
         if (lane == 0 && rank == 0) {
             const uint32_t idesc = umma_idesc_i8(256, N);
-            uint32_t uses[RG_NST];
+            uint32_t uses[NST];
 #pragma unroll
-            for (int q = 0; q < RG_NST; q++) uses[q] = 0;
-            int st = 0;
+            for (int q = 0; q < NST; q++) uses[q] = 0;
+            int st = 0, last = -1;
+            int steps = (p.K + 31) / 32;                  // K steps of 32 bytes
             bool bad = false;
-            for (int u = 0; u < nu && !bad; u++) {
-                const int buf = u & 1, use = u >> 1;
-                int steps;                                // K steps of 32 bytes
-                if (MODE == RG_HO) {
-                    steps = (p.K + 31) / 32;
-                } else {
-                    int tile, P;
-                    units.at(u, cl, tile, P);
-                    const AtomDesc &at = p.atoms[tiles[4 * tile + 1]];
-                    steps = (at.apw_off - at.oz_x0 + at.napw + 31) / 32;
+            for (int u = 0; u < units.count && !bad; u++, units.next()) {
+                const int buf = C::WIDE ? 0 : u & 1, use = C::WIDE ? u : u >> 1;
+                if (MODE == RG_ATOM) {
+                    const int tile = units.tile;
+                    if (tile != last) {
+                        last = tile;
+                        const AtomDesc &at = p.atoms[tiles[4 * tile + 1]];
+                        steps = (at.apw_off - at.oz_x0 + at.napw + 31) / 32;
+                    }
                 }
-                // the epilogues of both CTAs must have read this accumulator's previous product
-                if (use > 0 && !mbar_wait_ab(&acce[buf], (use - 1) & 1, abort, rg.wait)) {
-                    bad = true;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t tacc = tbase + (uint32_t)(buf * RG_ACC);
-                for (int k0 = 0; k0 < steps; k0 += RG_KCH * 4) {
+                for (int k0 = 0; k0 < steps; k0 += KCH * 4) {
                     if (!mbar_wait_ab(&full[st], uses[st] & 1, abort, rg.wait)) {
                         bad = true;
                         break;
                     }
-                    tc_fence_after();
-                    const uint32_t sa = sbase + st * RG_STAGE, sb = sa + RG_KCH * RG_BOX;
 #pragma unroll
-                    for (int q = 0; q < RG_KCH * 4; q++)
-                        if (k0 + q < steps) {
-                            const uint32_t o = (q >> 2) * RG_BOX + (q & 3) * 32;
-                            umma_i8_2sm(tacc, umma_desc_sw128(sa + o), umma_desc_sw128(sb + o), idesc,
-                                        k0 + q > 0 ? 1u : 0u);
+                    for (int o = 0; o < C::NB; o++) {
+                        // the epilogues of both CTAs must have read this accumulator's previous product
+                        if (k0 == 0 && use > 0 && !mbar_wait_ab(&acce[buf + o], (use - 1) & 1, abort, rg.wait)) {
+                            bad = true;
+                            break;
                         }
+                        tc_fence_after();
+                        const uint32_t sa = sbase + st * C::STAGE, sb = sa + (1 + o) * C::OPER;
+#pragma unroll
+                        for (int q = 0; q < KCH * 4; q++)
+                            if (k0 + q < steps) {
+                                const uint32_t off = (q >> 2) * RG_BOX + (q & 3) * 32;
+                                umma_i8_2sm(tbase + (uint32_t)((buf + o) * RG_ACC), umma_desc_sw128(sa + off),
+                                            umma_desc_sw128(sb + off), idesc, k0 + q > 0 ? 1u : 0u);
+                            }
+                        if (C::WIDE && k0 + KCH * 4 >= steps) umma_commit_2sm(&accf[o]);   // H first, then O
+                    }
+                    if (bad) break;
                     umma_commit_2sm(&empty[st]);
                     uses[st]++;
-                    st = (st + 1 == RG_NST) ? 0 : st + 1;
+                    st = (st + 1 == NST) ? 0 : st + 1;
                 }
-                if (!bad) umma_commit_2sm(&accf[buf]);
+                if (!C::WIDE && !bad) umma_commit_2sm(&accf[buf]);
             }
             if (bad)
-                for (int q = 0; q < RG_NST; q++)
+                for (int q = 0; q < NST; q++)
                     if (uses[q] > 0) mbar_drain(&empty[q], (uses[q] - 1) & 1);
         }
     } else if (warp >= 4) {
-        // ------------------------------------------------ epilogue (both CTAs, warps 4..11)
-        const int qd = warp & 3, half = (warp - 4) >> 2;
+        // ------------------------------------------------ epilogue (both CTAs, warps 4..19)
+        const int qd = warp & 3, part = (warp - 4) >> 2;
         const int row = qd * 32 + lane;
-        const int nq = b_rows / 16;                                 // 16-column chunks of this half
+        const int nq = N / 16;                                      // 16-column chunks of an accumulator
         const uint32_t acce0[2] = {mapa_shared(smem_u32(&acce[0]), 0), mapa_shared(smem_u32(&acce[1]), 0)};
-        const size_t plane_bytes = (size_t)N * 128;                 // residues of one product, this CTA's 128 rows
-        for (int u = 0; u < nu; u++) {
-            const int buf = u & 1, use = u >> 1;
-            int tile, P;
-            units.at(u, cl, tile, P);
-            if (!__all_sync(0xffffffffu, mbar_wait_ab(&accf[buf], use & 1, abort, rg.wait))) break;
-            tc_fence_after();
-            const int pm = rg.p[P >> 1], mg = rg.mg[P >> 1];
-            const uint32_t tacc = tbase + ((uint32_t)(qd * 32) << 16) + (uint32_t)(buf * RG_ACC + half * b_rows);
-            uint8_t *out = res + ((size_t)(2 * tile + (int)rank) * NP + P) * plane_bytes +
-                           ((size_t)half * nq * 128 + row) * 16;
-            for (int c = 0; c < nq; c++) {
-                uint32_t v[16];
-                tm_ld16(tacc + c * 16, v);
-                tm_wait_ld();
-                uint32_t w[4];
+        const size_t plane_bytes = (size_t)C::NB * N * 128;         // residues of one product, this CTA's 128 rows
+        bool bad = false;
+        for (int u = 0; u < units.count && !bad; u++, units.next()) {
+            const int P = units.P, m = P >> 1;
+            const int pm = rg.p[m], mg = rg.mg[m], up = rg.up[m];
+            const uint32_t mf = rg.mf[m];
+            uint8_t *out = res + ((size_t)(2 * units.tile + (int)rank) * NP + P) * plane_bytes + (size_t)row * 16;
 #pragma unroll
-                for (int q = 0; q < 4; q++)
-                    w[q] = pack4(ring_mod((int)v[4 * q], pm, mg), ring_mod((int)v[4 * q + 1], pm, mg),
-                                 ring_mod((int)v[4 * q + 2], pm, mg), ring_mod((int)v[4 * q + 3], pm, mg));
-                *reinterpret_cast<uint4 *>(out + (size_t)c * 128 * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+            for (int o = 0; o < C::NB; o++) {
+                const int buf = C::WIDE ? o : u & 1, use = C::WIDE ? u : u >> 1;
+                if (!__all_sync(0xffffffffu, mbar_wait_ab(&accf[buf], use & 1, abort, rg.wait))) {
+                    bad = true;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t tacc = tbase + ((uint32_t)(qd * 32) << 16) + (uint32_t)(buf * RG_ACC);
+                uint8_t *po = out + (size_t)o * N * 128;
+                // 16 columns at a time, the next 16 on their way while these are reduced
+                auto put = [&](const uint32_t (&v)[16], int c) {
+                    uint32_t w[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        uint32_t x[4];
+#pragma unroll
+                        for (int e = 0; e < 4; e++)
+                            x[e] = C::WIDE ? ring_mod((int)v[4 * q + e], pm, mg)
+                                           : ring_mod_short((int)v[4 * q + e], pm, mf, up);
+                        w[q] = pack4(x[0], x[1], x[2], x[3]);
+                    }
+                    *reinterpret_cast<uint4 *>(po + (size_t)c * 128 * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+                };
+                uint32_t v0[16], v1[16];
+                if (part < nq) tm_ld16(tacc + part * 16, v0);
+                for (int c = part; c < nq; c += 8) {
+                    tm_wait_ld();
+                    if (c + 4 < nq) tm_ld16(tacc + (c + 4) * 16, v1);
+                    put(v0, c);
+                    if (c + 4 < nq) {
+                        tm_wait_ld();
+                        if (c + 8 < nq) tm_ld16(tacc + (c + 8) * 16, v0);
+                        put(v1, c + 4);
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_relaxed(acce0[buf]);     // CTA 0's barrier (also from CTA 0)
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_remote(acce0[buf]);          // CTA 0's barrier (also from CTA 0)
         }
     }
     if (tid == 0 && *abort) atomicOr(p.err, DEV_ERR_TIMEOUT);
@@ -613,183 +687,246 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
 }
 
 // ------------------------------------------------------------ recombination
-// Eight real or imaginary parts from the residues of both images (wp[m] of
-// z+, wm[m] of z-: 8 bytes each).  With s_m = z+ + z- (real parts) or
-// z+ - z- + p_m (imaginary parts), s_m < 2 p_m, X / M = sum_m s_m e_m / p_m
-// (mod 1), e_m = y_m / 2 or y_m / (2 i_m) mod p_m, y_m = (M / p_m)^-1.  Two
-// moduli at a time: w = s_m (e_m p_m') + s_m' (e_m' p_m) < 2^26, and
-// t += w D (mod 2^96), D = round(2^96 / (p_m p_m')), three 32 x 32 -> 64-bit
-// multiply-adds per PAIR of moduli, carries propagated once at the end.  The
-// signed 64-bit window sh bits below the top of t is 2^(64+sh) X / M up to
-// the rounding of D (below 2^29 units of 2^-96).
-__device__ __forceinline__ void ring_crt8(const OzRing &rg, const uint2 (&wp)[OZ_RING_MAX],
-                                          const uint2 (&wm)[OZ_RING_MAX], bool im, int sh, double fin, double (&v)[8])
-{
-    unsigned long long a[8][3];
-#pragma unroll
-    for (int e = 0; e < 8; e++) a[e][0] = a[e][1] = a[e][2] = 0ull;
-#pragma unroll
-    for (int q = 0; q < OZ_RING_MAX / 2; q++) {
-        if (2 * q >= rg.n) break;
-        uint32_t w[8];
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const int m = 2 * q + j;
-            // an odd count leaves the last pair half empty: weight 0
-            const uint32_t f = im ? rg.fim[m] : rg.fre[m], pp = (uint32_t)rg.p[m] * 0x10001u;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const uint32_t zp = h ? wp[m].y : wp[m].x, zm = h ? wm[m].y : wm[m].x;
-                uint32_t s[2];                          // 16-bit lanes: bytes 0, 2 and 1, 3
-                const uint32_t p0 = zp & 0xff00ffu, p1 = (zp >> 8) & 0xff00ffu;
-                const uint32_t m0 = zm & 0xff00ffu, m1 = (zm >> 8) & 0xff00ffu;
-                s[0] = im ? p0 + pp - m0 : p0 + m0;
-                s[1] = im ? p1 + pp - m1 : p1 + m1;
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const uint32_t x = (e & 2) ? s[e & 1] >> 16 : s[e & 1] & 0xffffu;
-                    w[4 * h + e] = (j ? w[4 * h + e] : 0u) + x * f;
-                }
-            }
-        }
-        const unsigned long long d0 = rg.d96[0][q], d1 = rg.d96[1][q], d2 = rg.d96[2][q];
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-            a[e][0] += w[e] * d0;
-            a[e][1] += w[e] * d1;
-            a[e][2] += w[e] * d2;
-        }
-    }
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-        const unsigned long long a1 = a[e][1] + (a[e][0] >> 32);
-        const unsigned long long a2 = a[e][2] + (a1 >> 32);
-        const unsigned long long top = (((a2 << 32) | (a1 & 0xffffffffull)) << sh) |
-                                       ((a[e][0] & 0xffffffffull) >> (32 - sh));
-        v[e] = (double)(long long)top * fin;
-    }
-}
+// The residue words of four columns of one row: z+ of modulus m in plane
+// 2m + first, z- in the other.
+struct RingWords {
+    uint32_t p[OZ_RING_MAX], m[OZ_RING_MAX];
+};
 
-// The residue bytes of 8 columns of one row: z+ of modulus m in plane 2m + first.
-__device__ __forceinline__ void ring_load8(const uint8_t *tres, size_t plane, int n, int first,
-                                           uint2 (&wp)[OZ_RING_MAX], uint2 (&wm)[OZ_RING_MAX])
+__device__ __forceinline__ void ring_load4(const uint8_t *tres, size_t plane, int n, int first, RingWords &w)
 {
 #pragma unroll
     for (int m = 0; m < OZ_RING_MAX; m++) {
-        wp[m] = wm[m] = make_uint2(0u, 0u);
+        w.p[m] = w.m[m] = 0u;
         if (m < n) {
-            wp[m] = *reinterpret_cast<const uint2 *>(tres + (size_t)(2 * m + first) * plane);
-            wm[m] = *reinterpret_cast<const uint2 *>(tres + (size_t)(2 * m + 1 - first) * plane);
+            w.p[m] = *reinterpret_cast<const uint32_t *>(tres + (size_t)(2 * m + first) * plane);
+            w.m[m] = *reinterpret_cast<const uint32_t *>(tres + (size_t)(2 * m + 1 - first) * plane);
         }
     }
 }
 
-// Recombination, scaling, interstitial term and store of the H/O tiles: one
-// thread per (row of a 128-row tile, 8-column group, matrix: 0 = H, 1 = O):
-// blocks of 128 threads (the rows), blockIdx.y = (matrix, column group).
-// Every thread first issues the loads of its residue bytes, then recombines:
-// the loads of a warp cover 32 rows of 16 bytes of which the group uses half.
+// Real and imaginary parts of four values from their residues z+, z- (any
+// representatives in [0, 255]).  X / M = sum_m s_m e_m / p_m (mod 1) with
+// s_m = z+ + z-, e_m = y_m / 2 mod p_m for the real parts, s_m = z+ - z-,
+// e_m = y_m / (2 i_m) mod p_m for the imaginary parts, y_m = (M / p_m)^-1.
+// Two moduli p, p' at a time: w = s_m (e_m p') + s_m' (e_m' p) with both
+// weights reduced to symmetric residues mod p p' (|.| < 2^15), in two signed
+// bytes: two dot products with the bytes z+, z-, z+', z-' of the value, the
+// low one started at a multiple of p p' that keeps 0 <= w < 2^27.  Then
+// t += w D (mod 2^96), D = round(2^96 / (p p')): three 32 x 32-bit
+// multiply-adds (the top one needs 32 bits only) per PAIR of moduli, carries
+// propagated once at the end.  The signed 64-bit window sh bits below the top
+// of t is 2^(64+sh) X / M up to the rounding of D (below 2^29 units of 2^-96).
+__device__ __forceinline__ void ring_crt4(const OzRing &rg, const RingWords &z, int sh, double fin, double (&re)[4],
+                                          double (&im)[4])
+{
+    unsigned long long a0[8], a1[8];                    // re 0..3, im 0..3
+    uint32_t a2[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+        a0[e] = a1[e] = 0ull;
+        a2[e] = 0u;
+    }
+#pragma unroll
+    for (int q = 0; q < OZ_RING_MAX / 2; q++) {
+        if (2 * q >= rg.n) break;
+        // bytes (z+, z-, z+', z-') of each value: a 4 x 4 byte transpose
+        const uint32_t t0 = __byte_perm(z.p[2 * q], z.m[2 * q], 0x5140), t1 = __byte_perm(z.p[2 * q], z.m[2 * q], 0x7362);
+        const uint32_t u0 = __byte_perm(z.p[2 * q + 1], z.m[2 * q + 1], 0x5140),
+                       u1 = __byte_perm(z.p[2 * q + 1], z.m[2 * q + 1], 0x7362);
+        const uint32_t b[4] = {__byte_perm(t0, u0, 0x5410), __byte_perm(t0, u0, 0x7632), __byte_perm(t1, u1, 0x5410),
+                               __byte_perm(t1, u1, 0x7632)};
+        const uint32_t d0 = rg.d96[0][q], d1 = rg.d96[1][q], d2 = rg.d96[2][q];
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            const int c = e >> 2;                       // 0: real part, 1: imaginary part
+            const uint32_t w = (uint32_t)(dp4a_us(b[e & 3], rg.wlo[c][q], rg.woff[q]) +
+                                          256 * dp4a_us(b[e & 3], rg.whi[c][q], 0));
+            a0[e] += (unsigned long long)w * d0;
+            a1[e] += (unsigned long long)w * d1;
+            a2[e] += w * d2;
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+        const unsigned long long c1 = a1[e] + (a0[e] >> 32);
+        const unsigned long long hi = ((unsigned long long)(a2[e] + (uint32_t)(c1 >> 32)) << 32) | (uint32_t)c1;
+        const unsigned long long top = (hi << sh) | ((a0[e] & 0xffffffffull) >> (32 - sh));
+        const double v = (double)(long long)top * fin;
+        if (e < 4)
+            re[e] = v;
+        else
+            im[e - 4] = v;
+    }
+}
+
+// Recombination, scaling, interstitial term and store of the H/O tiles: a
+// block of four warps takes 32 rows x 16 columns of both matrices.  Lane l
+// of a warp recombines row l / 4 of its eight, columns 4 (l % 4) .. + 3, so a
+// warp reads 128 contiguous residue bytes per plane; the index of G_i - G_j
+// is looked up once for H and O.  The values are staged in shared memory and
+// leave as whole column segments: 512 bytes of the upper triangle, 256 bytes
+// of the mirror.  Bound by the residue reads and the H/O writes (HBM) and
+// by the integer multiply-adds.  27 k-points of the eight-atom cell 0.54 ms, 64
+// atoms 1.36 ms; one thread per row and eight columns, the mirror stored from
+// registers, took 0.88 and 2.18 ms.
+constexpr int RC_R = 32, RC_C = 16;
+
+template <int BJ>
 __global__ void __launch_bounds__(128) oz_crt_kernel(DevParams p, const KDesc *ks, const int *tiles,
                                                      const __grid_constant__ OzRing rg, const uint8_t *res)
 {
-    constexpr int NG = RG_BJ / 8;                                // 8-column groups
-    const int tile = blockIdx.x >> 1, row = threadIdx.x;
-    const int cg = blockIdx.y % NG, half = blockIdx.y / NG;
+    __shared__ exs_complex T[2][RC_R][RC_C + 1];
+    __shared__ double sv[RC_R + RC_C][3], ssig[RC_R + 2 * RC_C];
+    __shared__ int siv[RC_R + RC_C][3];
+    constexpr int NR = RG_BM / RC_R;                             // row groups of a tile
+    const int tile = blockIdx.x / NR, rgrp = blockIdx.x % NR;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const KDesc kd = ks[tiles[3 * tile]];
-    const int i = tiles[3 * tile + 1] * RG_BM + (blockIdx.x & 1) * 128 + row;
-    const int jb = tiles[3 * tile + 2] * RG_BJ + cg * 8;
-    if (i >= kd.ngp || jb >= kd.ngp || jb + 7 < i) return;     // no element i <= j < ngp here
-    constexpr size_t plane = 2 * RG_BJ * 128;
-    const uint8_t *tres = res + (size_t)blockIdx.x * 2 * rg.n * plane +
-                          ((size_t)(half * (RG_BJ / 16) + (cg >> 1)) * 128 + row) * 16 + (cg & 1) * 8;
-    uint2 wp[OZ_RING_MAX], wm[OZ_RING_MAX];
-    ring_load8(tres, plane, rg.n, 0, wp, wm);
-    // row data
-    int gi = kd.igpig[i] - 1;
-    if (gi < 0 || gi >= p.ngrtot) {
-        atomicOr(p.err, DEV_ERR_INDEX);
-        gi = 0;
+    const int i0 = tiles[3 * tile + 1] * RG_BM + rgrp * RC_R;
+    const int j0 = tiles[3 * tile + 2] * BJ + blockIdx.y * RC_C;
+    if (i0 >= kd.ngp || j0 >= kd.ngp || j0 + RC_C - 1 < i0) return;    // no element i <= j < ngp here
+    constexpr size_t plane = 2 * BJ * 128;
+    const int r = warp * 8 + (lane >> 2), cq = lane & 3;
+    const int row = (rgrp * RC_R & 127) + r;                     // of the 128-row tile
+    const uint8_t *tres = res + (size_t)(2 * tile + rgrp * RC_R / 128) * 2 * rg.n * plane +
+                          ((size_t)blockIdx.y * 128 + row) * 16 + cq * 4;
+    RingWords z;
+    ring_load4(tres, plane, rg.n, 0, z);                         // H
+    if (tid < RC_R + RC_C) {                                     // G vectors and scales of the rows and columns
+        const int g = tid < RC_R ? i0 + tid : j0 + tid - RC_R;
+        if (g < kd.ngp) {
+            int ig = kd.igpig[g] - 1;
+            if (ig < 0 || ig >= p.ngrtot) {
+                atomicOr(p.err, DEV_ERR_INDEX);
+                ig = 0;
+            }
+            for (int x = 0; x < 3; x++) {
+                siv[tid][x] = p.ivg[3 * ig + x];
+                sv[tid][x] = kd.vgpc[3 * g + x];
+            }
+            if (tid < RC_R) {
+                ssig[tid] = oz_sigma(kd.oz_scale[g]);
+            } else {   // H: sigma_B(j); O: sigma_A(j), or sigma_C(j) with iora* (O = A^H C)
+                ssig[tid] = oz_sigma(kd.oz_scale[p.npad + g]);
+                ssig[tid + RC_C] = oz_sigma(kd.oz_scale[(p.relativity == EXS_REL_IORA ? 2 * p.npad : 0) + g]);
+            }
+        }
     }
-    const int ivi[3] = {p.ivg[3 * gi], p.ivg[3 * gi + 1], p.ivg[3 * gi + 2]};
-    const double vi[3] = {kd.vgpc[3 * i], kd.vgpc[3 * i + 1], kd.vgpc[3 * i + 2]};
-    const double sai = oz_sigma(kd.oz_scale[i]);
-    // H: sigma_B(j); O: sigma_A(j), or sigma_C(j) with iora* (O = A^H C)
-    const double *scol = kd.oz_scale + (half == 0 ? p.npad : (p.relativity == EXS_REL_IORA ? 2 * p.npad : 0));
-    const int kind = half == 0 ? EPI_HAM : EPI_OVL;
-    exs_complex *out = half == 0 ? kd.h : kd.o;
-    double vre[8], vim[8];
-    ring_crt8(rg, wp, wm, false, rg.sh, rg.fin, vre);
-    ring_crt8(rg, wp, wm, true, rg.sh, rg.fin, vim);
+    __syncthreads();
+    int ig[4];
 #pragma unroll
-    for (int e = 0; e < 8; e++) {
-        const int j = jb + e;
-        if (j >= kd.ngp || j < i) continue;
-        int gj = kd.igpig[j] - 1;
-        if (gj < 0 || gj >= p.ngrtot) {
-            atomicOr(p.err, DEV_ERR_INDEX);
-            gj = 0;
+    for (int e = 0; e < 4; e++) {
+        const int c = RC_R + cq * 4 + e, j = j0 + cq * 4 + e;
+        ig[e] = (i0 + r <= j && j < kd.ngp) ? interstitial_index(p, siv[r], siv[c]) : 0;
+    }
+#pragma unroll
+    for (int w = 0; w < 2; w++) {
+        double re[4], im[4];
+        ring_crt4(rg, z, rg.sh, rg.fin, re, im);
+        if (w == 0) ring_load4(tres + (size_t)BJ * 128, plane, rg.n, 0, z);      // O
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const int c = RC_R + cq * 4 + e;
+            const double sc = ssig[r] * ssig[c + w * RC_C];
+            exs_complex v;
+            v.re = re[e] * sc;
+            v.im = im[e] * sc;
+            if (ig[e] > 0) {
+                double ar, ai;
+                interstitial_value(p, w == 0 ? EPI_HAM : EPI_OVL, ig[e], sv[r], sv[c], ar, ai);
+                v.re += ar;
+                v.im += ai;
+            }
+            T[w][r][cq * 4 + e] = v;
         }
-        const int ivj[3] = {p.ivg[3 * gj], p.ivg[3 * gj + 1], p.ivg[3 * gj + 2]};
-        const double vj[3] = {kd.vgpc[3 * j], kd.vgpc[3 * j + 1], kd.vgpc[3 * j + 2]};
-        const double sc = sai * oz_sigma(scol[j]);
-        double re = vre[e] * sc, im = vim[e] * sc;
-        double ar, ai;
-        if (interstitial(p, kind, ivi, ivj, vi, vj, ar, ai)) {
-            re += ar;
-            im += ai;
+    }
+    __syncthreads();
+    const size_t nm = (size_t)kd.nmat;
+#pragma unroll
+    for (int w = 0; w < 2; w++) {
+        exs_complex *out = w == 0 ? kd.h : kd.o;
+#pragma unroll
+        for (int q = 0; q < RC_C / 4; q++) {                     // upper: lane = row
+            const int c = warp + 4 * q, i = i0 + lane, j = j0 + c;
+            if (j < kd.ngp && i <= j) out[(size_t)i + nm * j] = T[w][lane][c];
         }
-        exs_complex v;
-        v.re = re;
-        v.im = im;
-        out[(size_t)i + (size_t)kd.nmat * j] = v;
-        if (i < j) {
-            v.im = -im;
-            out[(size_t)j + (size_t)kd.nmat * i] = v;
+#pragma unroll
+        for (int q = 0; q < RC_R / 8; q++) {                     // mirror: lanes = two rows of 16 columns
+            const int rr = warp * 8 + 2 * q + (lane >> 4), i = i0 + rr, j = j0 + (lane & 15);
+            if (j < kd.ngp && i < j) {
+                exs_complex v = T[w][rr][lane & 15];
+                v.im = -v.im;
+                out[(size_t)j + nm * i] = v;
+            }
         }
     }
 }
 
-// Recombination of the per-atom tiles: the B planes and the APW-lo rows of H
-// with their mirror.  One thread per (G of a 128-row tile, 8 rows of X),
-// blockIdx.y = the 8-row group: a warp writes 32 consecutive G of one plane row.
+// Recombination of the per-atom tiles, organised like oz_crt_kernel (32 G x
+// 16 rows of X per block): the B planes, 256 contiguous bytes per row, and the
+// APW-lo rows of H with their mirror.  64 atoms 1.07 ms (one thread per G and
+// eight rows: 1.36 ms).
 __global__ void __launch_bounds__(128) oz_bcrt_kernel(DevParams p, const KDesc *ks, const int *tiles,
                                                       const __grid_constant__ OzRing rg, OzAtomArgs xa,
                                                       const uint8_t *res)
 {
-    const int tile = blockIdx.x >> 1, row = threadIdx.x, cg = blockIdx.y;
+    __shared__ double T[2][RC_R][RC_C + 1];
+    constexpr int NR = RG_BM / RC_R;
+    const int tile = blockIdx.x / NR, rgrp = blockIdx.x % NR;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const KDesc kd = ks[tiles[4 * tile]];
     const int ias = tiles[4 * tile + 1];
-    const int g = tiles[4 * tile + 2] * RG_BM + (blockIdx.x & 1) * 128 + row;
-    const int n0 = tiles[4 * tile + 3] * xa.nb + cg * 8;
-    const AtomDesc at = p.atoms[ias];
-    if (g >= kd.ngp || n0 >= at.napw + at.losize) return;
+    const int g0 = tiles[4 * tile + 2] * RG_BM + rgrp * RC_R;
+    const int n0 = tiles[4 * tile + 3] * xa.nb + blockIdx.y * RC_C;
+    const AtomDesc &at = p.atoms[ias];
+    const int napw = at.napw, nrow = at.napw + at.losize;
+    if (g0 >= kd.ngp || n0 >= nrow) return;
     const size_t plane = (size_t)xa.nb * 128;
-    const uint8_t *tres = res + (size_t)blockIdx.x * 2 * rg.n * plane + ((size_t)(cg >> 1) * 128 + row) * 16 + (cg & 1) * 8;
-    uint2 wp[OZ_RING_MAX], wm[OZ_RING_MAX];
-    ring_load8(tres, plane, rg.n, 1, wp, wm);
-    const double sa = oz_sigma(kd.oz_scale[g]);
-    const double *sig = xa.xsig + (size_t)ias * xa.nrows + n0;
-    double vre[8], vim[8];
-    ring_crt8(rg, wp, wm, false, rg.shx, rg.finx, vre);
-    ring_crt8(rg, wp, wm, true, rg.shx, rg.finx, vim);
-    const size_t row0 = (size_t)kd.ngp + at.lo_off;
+    const int r = warp * 8 + (lane >> 2), cq = lane & 3;
+    const int row = (rgrp * RC_R & 127) + r;
+    RingWords z;
+    ring_load4(res + (size_t)(2 * tile + rgrp * RC_R / 128) * 2 * rg.n * plane + ((size_t)blockIdx.y * 128 + row) * 16 +
+                   cq * 4,
+               plane, rg.n, 1, z);
+    const double sa = g0 + r < kd.ngp ? oz_sigma(kd.oz_scale[g0 + r]) : 0.0;
+    const double *sig = xa.xsig + (size_t)ias * xa.nrows + n0 + cq * 4;
+    double re[4], im[4];
+    ring_crt4(rg, z, rg.shx, rg.finx, re, im);
 #pragma unroll
-    for (int e = 0; e < 8; e++) {
-        const int n = n0 + e;
+    for (int e = 0; e < 4; e++) {
         const double sc = sa * sig[e];
-        const double re = vre[e] * sc, im = vim[e] * sc;
-        if (n < at.napw) {
+        T[0][r][cq * 4 + e] = re[e] * sc;
+        T[1][r][cq * 4 + e] = im[e] * sc;
+    }
+    __syncthreads();
+    const int g = g0 + lane;
+    const size_t row0 = (size_t)kd.ngp + at.lo_off, nm = (size_t)kd.nmat;
+#pragma unroll
+    for (int q = 0; q < RC_C / 4; q++) {                         // lane = G
+        const int c = warp + 4 * q, n = n0 + c;
+        if (g >= kd.ngp) continue;
+        if (n < napw) {
             const size_t off = (size_t)(at.apw_off + n) * p.npad + g;
-            kd.br[off] = re;
-            kd.bi[off] = im;
-        } else if (n < at.napw + at.losize) {
-            const int r = n - at.napw;
+            kd.br[off] = T[0][lane][c];
+            kd.bi[off] = T[1][lane][c];
+        } else if (n < nrow) {
             exs_complex v;
-            v.re = re;
-            v.im = im;
-            kd.h[(row0 + r) + (size_t)kd.nmat * g] = v;
-            v.im = -im;
-            kd.h[(size_t)g + (size_t)kd.nmat * (row0 + r)] = v;
+            v.re = T[0][lane][c];
+            v.im = -T[1][lane][c];
+            kd.h[(size_t)g + nm * (row0 + n - napw)] = v;
+        }
+    }
+    if (n0 + RC_C > napw) {                                      // lo rows: lanes = two G of 16 rows
+#pragma unroll
+        for (int q = 0; q < RC_R / 8; q++) {
+            const int rr = warp * 8 + 2 * q + (lane >> 4), n = n0 + (lane & 15), gg = g0 + rr;
+            if (gg < kd.ngp && n >= napw && n < nrow) {
+                exs_complex v;
+                v.re = T[0][rr][lane & 15];
+                v.im = T[1][rr][lane & 15];
+                kd.h[(row0 + n - napw) + nm * gg] = v;
+            }
         }
     }
 }
@@ -923,19 +1060,38 @@ int oz_ring_plan(int b, int bx, OzRing *out)
         const int start = 12582912 / p * p;
         r.base[m] = 0x4B000000 - (1 << 23) + start + sym(-((1LL << 55) % p));
         r.icorr[m] = sym(-((1LL << 55) % p) * im);
-        // recombination: e_m times the other modulus of the pair (2q, 2q + 1)
-        const int other = (m ^ 1) < r.n ? OZ_RINGS[m ^ 1] : 1;
-        r.fre[m] = (unsigned)((long long)y * half % p) * (unsigned)other;
-        r.fim[m] = (unsigned)((long long)y * half % p * iinv % p) * (unsigned)other;
+        r.mf[m] = (unsigned)((1LL << 32) / p);
+        r.up[m] = ((1 << 27) / p + 1) * p;
+        // recombination: e_m times the other modulus of the pair (2q, 2q + 1), symmetric mod their product,
+        // as signed bytes 256 h + l for z+ (and, negated for the imaginary parts, z-)
+        const int other = (m ^ 1) < r.n ? OZ_RINGS[m ^ 1] : 1, pq = p * other, q = m / 2, sft = 16 * (m & 1);
+        for (int c = 0; c < 2; c++) {
+            long long f = (long long)y * half % p * (c ? iinv : 1) % p * other;
+            if (f > pq / 2) f -= pq;
+            for (int w = 0; w < 2; w++) {                // z+, z-
+                const int v = (int)(c && w ? -f : f);
+                const int l = (int)(int8_t)(uint8_t)(v & 255), h = (v - l) / 256;
+                if (h < -128 || h > 127) return -1;
+                r.wlo[c][q] |= (int)((unsigned)(uint8_t)(int8_t)l << (sft + 8 * w));
+                r.whi[c][q] |= (int)((unsigned)(uint8_t)(int8_t)h << (sft + 8 * w));
+            }
+        }
         if ((m & 1) == 0) {
-            const unsigned pq = (unsigned)(p * other);
+            r.woff[q] = (((1 << 26) + pq - 1) / pq) * pq;   // |w| <= 4 * 255 * 2^15 < 2^26 before the offset
             const unsigned __int128 d = (((unsigned __int128)1 << 96) + pq / 2) / pq;
-            for (int w = 0; w < 3; w++) r.d96[w][m / 2] = (unsigned)(d >> (32 * w));
+            for (int w = 0; w < 3; w++) r.d96[w][q] = (unsigned)(d >> (32 * w));
         }
     }
     *out = r;
     return 0;
 }
+
+// Columns of the H/O tiles.  256-column tiles read three quarters of the
+// operand bytes per product, but their epilogue stops the MMAs once per
+// product: 0.85 against 0.81 ms at K = 2592 (16 atoms, 3 k), 1.68 against
+// 1.49 ms at K = 1936, 13.9 against 14.3 ms at K = 10,368.  Up to RG_SHORT_K
+// the 128-column tiles also have the short residue reduction.
+int ring_ho_cols(int K) { return K > RG_SHORT_K ? 256 : 128; }
 
 int ring_kpad(int K) { return (K + RG_CHUNK - 1) / RG_CHUNK * RG_CHUNK; }
 
@@ -944,7 +1100,7 @@ size_t ring_slot_bytes(const OzRing &rg, int npad, int kp8, int relativity)
     return (size_t)2 * rg.n * ring_narr(relativity) * npad * (size_t)kp8;
 }
 
-size_t ring_ho_tile_bytes(const OzRing &rg) { return (size_t)2 * rg.n * RG_BM * 2 * RG_BJ; }
+size_t ring_ho_tile_bytes(const OzRing &rg, int cols) { return (size_t)2 * rg.n * RG_BM * 2 * cols; }
 
 size_t ring_atom_tile_bytes(const OzRing &rg, int nb) { return (size_t)2 * rg.n * RG_BM * nb; }
 
@@ -991,7 +1147,7 @@ static cudaError_t plane_grid(int ntiles, int np, cudaStream_t s, int *ncl)
 {
     static std::atomic<unsigned long long> attr{0};
     cudaError_t e = once_per_device(attr, [] {
-        return cudaFuncSetAttribute(oz_plane_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, RG_SMEM);
+        return cudaFuncSetAttribute(oz_plane_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, RingCfg<MODE>::SMEM);
     });
     if (e != cudaSuccess) return e;
     static std::atomic<int> resident{0};         // the same for every device of this build's architecture
@@ -1000,7 +1156,7 @@ static cudaError_t plane_grid(int ntiles, int np, cudaStream_t s, int *ncl)
         cudaLaunchConfig_t lc = {};
         lc.gridDim = dim3(2 * RG_PACE_MAX);
         lc.blockDim = dim3(RG_THREADS);
-        lc.dynamicSmemBytes = RG_SMEM;
+        lc.dynamicSmemBytes = RingCfg<MODE>::SMEM;
         lc.stream = s;
         if (cudaOccupancyMaxActiveClusters(&act, (void *)oz_plane_kernel<MODE>, &lc) != cudaSuccess || act < 1) {
             (void)cudaGetLastError();
@@ -1021,24 +1177,35 @@ static cudaError_t plane_grid(int ntiles, int np, cudaStream_t s, int *ncl)
 // HBM again and again.
 constexpr size_t RG_PACE_BYTES = (size_t)100 << 20;
 
-cudaError_t launch_ring_ho(const CUtensorMap *map, const DevParams &p, const KDesc *d_k, const void *d_tiles,
-                           int ntiles, const OzRing &rg, int kp8, uint8_t *res, int *pace, cudaStream_t s)
+template <int MODE>
+static cudaError_t launch_ho(const CUtensorMap *map, const DevParams &p, const KDesc *d_k, const int *d_tiles,
+                             int ntiles, const OzRing &rg, int kp8, uint8_t *res, int *pace, cudaStream_t s)
 {
-    if (ntiles <= 0) return cudaSuccess;
+    using C = RingCfg<MODE>;
     int ncl = 0;
-    cudaError_t e = plane_grid<RG_HO>(ntiles, 2 * rg.n, s, &ncl);
+    cudaError_t e = plane_grid<MODE>(ntiles, 2 * rg.n, s, &ncl);
     if (e != cudaSuccess) return e;
     const bool paced = (size_t)3 * p.npad * kp8 > RG_PACE_BYTES;
     if (paced) {
         e = cudaMemsetAsync(pace, 0, sizeof(int) * ncl, s);
         if (e != cudaSuccess) return e;
     }
-    oz_plane_kernel<RG_HO><<<2 * ncl, RG_THREADS, RG_SMEM, s>>>(*map, *map, p, d_k, (const int *)d_tiles, ntiles, rg,
-                                                                OzAtomArgs{}, res, paced ? pace : nullptr);
+    oz_plane_kernel<MODE><<<2 * ncl, RG_THREADS, C::SMEM, s>>>(*map, *map, p, d_k, d_tiles, ntiles, rg, OzAtomArgs{},
+                                                               res, paced ? pace : nullptr);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    oz_crt_kernel<<<dim3(2 * ntiles, 2 * (RG_BJ / 8)), 128, 0, s>>>(p, d_k, (const int *)d_tiles, rg, res);
+    oz_crt_kernel<C::BJ><<<dim3(ntiles * (RG_BM / RC_R), C::BJ / RC_C), 128, 0, s>>>(p, d_k, d_tiles, rg, res);
     return cudaGetLastError();
+}
+
+cudaError_t launch_ring_ho(int cols, const CUtensorMap *map1, const CUtensorMap *map2, const DevParams &p,
+                           const KDesc *d_k, const void *d_tiles, int ntiles, const OzRing &rg, int kp8, uint8_t *res,
+                           int *pace, cudaStream_t s)
+{
+    if (ntiles <= 0) return cudaSuccess;
+    const int *t = (const int *)d_tiles;
+    return cols == 256 ? launch_ho<RG_WIDE>(map1, p, d_k, t, ntiles, rg, kp8, res, pace, s)
+                       : launch_ho<RG_HO>(map2, p, d_k, t, ntiles, rg, kp8, res, pace, s);
 }
 
 // Per-atom products in chunks of tiles whose residues fit the residue buffer.
@@ -1054,11 +1221,11 @@ cudaError_t launch_ring_atom(const CUtensorMap *mapA, const CUtensorMap *mapX, c
         int ncl = 0;
         cudaError_t e = plane_grid<RG_ATOM>(nt, 2 * rg.n, s, &ncl);
         if (e != cudaSuccess) return e;
-        oz_plane_kernel<RG_ATOM><<<2 * ncl, RG_THREADS, RG_SMEM, s>>>(*mapA, *mapX, p, d_k, tiles, nt, rg, xa, res,
+        oz_plane_kernel<RG_ATOM><<<2 * ncl, RG_THREADS, RingCfg<RG_ATOM>::SMEM, s>>>(*mapA, *mapX, p, d_k, tiles, nt, rg, xa, res,
                                                                       nullptr);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
-        oz_bcrt_kernel<<<dim3(2 * nt, xa.nb / 8), 128, 0, s>>>(p, d_k, tiles, rg, xa, res);
+        oz_bcrt_kernel<<<dim3(nt * (RG_BM / RC_R), xa.nb / RC_C), 128, 0, s>>>(p, d_k, tiles, rg, xa, res);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
@@ -1066,9 +1233,9 @@ cudaError_t launch_ring_atom(const CUtensorMap *mapA, const CUtensorMap *mapX, c
 }
 
 // TMA views (int8):
-//   ho    the planes of all slots as 5D (K byte in a 128-byte chunk, G,
-//         array, K chunk, slot x plane), box {128, 128, 1, 2, 1}: 128 G rows of
-//         one array, two K chunks, each chunk contiguous in shared memory
+//   ho1, ho2  the planes of all slots as 5D (K byte in a 128-byte chunk, G,
+//         array, K chunk, slot x plane), boxes {128, 128, 1, 1 or 2, 1}: 128 G
+//         rows of one array, one or two K chunks, each contiguous in shared memory
 //   arow  the same bytes as 4D (K byte, G, array, slot x plane), box {128,
 //         128, 1, 1}: a K chunk starting at any multiple of 16 bytes (the atom
 //         windows are not chunk aligned)
@@ -1076,7 +1243,7 @@ cudaError_t launch_ring_atom(const CUtensorMap *mapA, const CUtensorMap *mapX, c
 //         K chunk), box {128, nb / 2, 1, 1}
 // Rows past npad (or past the rows of X) and K chunks past kp8 arrive as zeros.
 bool make_ring_maps(void *base, size_t nsp, int npad, int kp8, int narr, void *xbase, size_t xgroups, int nrows,
-                    int nb, int lw, CUtensorMap *ho, CUtensorMap *arow, CUtensorMap *x)
+                    int nb, int lw, CUtensorMap *ho1, CUtensorMap *ho2, CUtensorMap *arow, CUtensorMap *x)
 {
     typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
@@ -1096,13 +1263,14 @@ bool make_ring_maps(void *base, size_t nsp, int npad, int kp8, int narr, void *x
     };
     const cuuint64_t K = kp8, G = npad, A = narr;
     const cuuint64_t dho[5] = {RG_CHUNK, G, A, K / RG_CHUNK, nsp}, sho[4] = {K, G * K, RG_CHUNK, A * G * K};
-    const cuuint32_t bho[5] = {RG_CHUNK, 128, 1, RG_KCH, 1};
+    const cuuint32_t bho1[5] = {RG_CHUNK, 128, 1, 1, 1}, bho2[5] = {RG_CHUNK, 128, 1, 2, 1};
     const cuuint64_t dar[4] = {K, G, A, nsp}, sar[3] = {K, G * K, A * G * K};
     const cuuint32_t bar[4] = {RG_CHUNK, 128, 1, 1};
     const cuuint64_t L = lw, R = nrows;
     const cuuint64_t dx[4] = {RG_CHUNK, R, xgroups, L / RG_CHUNK}, sx[3] = {L, R * L, RG_CHUNK};
     const cuuint32_t bx[4] = {RG_CHUNK, (cuuint32_t)(nb / 2), 1, 1};
-    return make(ho, 5, base, dho, sho, bho) && make(arow, 4, base, dar, sar, bar) && make(x, 4, xbase, dx, sx, bx);
+    return make(ho1, 5, base, dho, sho, bho1) && make(ho2, 5, base, dho, sho, bho2) &&
+           make(arow, 4, base, dar, sar, bar) && make(x, 4, xbase, dx, sx, bx);
 }
 
 }  // namespace exs

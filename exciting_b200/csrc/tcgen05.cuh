@@ -30,6 +30,21 @@ __device__ __forceinline__ bool mbar_try(uint64_t *bar, uint32_t parity)
     return ok != 0;
 }
 
+// The same, the thread suspended in hardware for up to 10 us meanwhile: a
+// warp that polls burns issue slots and power that the tensor cores then lack.
+__device__ __forceinline__ bool mbar_try_suspend(uint64_t *bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(10000)
+        : "memory");
+    return ok != 0;
+}
+
 // Bounded wait (limit cycles; 0: OZ_WAIT_CYCLES) that also gives up as soon
 // as another role raised `abort`.
 __device__ __forceinline__ bool mbar_wait_ab(uint64_t *bar, uint32_t parity, volatile int *abort, long long limit)
@@ -37,7 +52,7 @@ __device__ __forceinline__ bool mbar_wait_ab(uint64_t *bar, uint32_t parity, vol
     const long long t0 = clock64();
     const long long lim = limit > 0 ? limit : OZ_WAIT_CYCLES;
     while (true) {
-        if (mbar_try(bar, parity)) return true;
+        if (limit > 0 ? mbar_try(bar, parity) : mbar_try_suspend(bar, parity)) return true;
         if (*abort) return false;
         if (clock64() - t0 > lim) {
             *abort = 1;

@@ -89,6 +89,23 @@ def test_split_residues(p):
     assert all((int(a) - im * int(c) - int(r)) % p == 0 for a, c, r in zip(x, y, d))
 
 
+def reduce(v, p):
+    """The byte the short product kernel stores for the int32 sums v, |v| < 2^27."""
+    x = v + ((1 << 27) // p + 1) * p
+    r = x - ((x * ((1 << 32) // p)) >> 32) * p
+    assert r.min() >= 0 and r.max() <= 246
+    return r
+
+
+@pytest.mark.parametrize("p", RINGS)
+def test_short_reduction(p):
+    """Bytes congruent to the sums over the whole range of the short kernel."""
+    v = np.concatenate([np.random.default_rng(p).integers(-2 ** 27 + 1, 2 ** 27, 20000),
+                        np.array([0, -1, 1, p, -p, p - 1, -p - 1, 2 ** 27 - 1, -2 ** 27 + 1])])
+    assert np.array_equal(reduce(v, p) % p, v % p)
+    assert 8192 * 123 ** 2 < 2 ** 27
+
+
 @pytest.mark.parametrize("n", [6, 13, 14, 16])
 def test_products_recombine(n):
     """conj(A)^T B of integer columns of norm 2^b, through the rings."""
@@ -106,18 +123,22 @@ def test_products_recombine(n):
     t = np.zeros((2, 4, 4), dtype=object)
     bound = 0
     for q in range(0, len(ps), 2):
-        w = np.zeros((2, 4, 4), dtype=object)
-        for j, p in enumerate(ps[q:q + 2]):
-            other = ps[q + 1 - j] if q + 1 < len(ps) else 1
+        pair = ps[q:q + 2]
+        pq = math.prod(pair)
+        w = np.full((2, 4, 4), -(-(1 << 26) // pq) * pq, dtype=object)
+        for j, p in enumerate(pair):
             (ap, am), (bp, bm) = split(ar, ai, p), split(br, bi, p)
-            zp, zm = (am.T @ bp) % p, (ap.T @ bm) % p                   # exact: K 127^2 < 2^31
-            y, half = pow(M // p, -1, p), pow(2, -1, p)
-            w[0] += (zp + zm).astype(object) * (y * half % p * other)
-            w[1] += (zp - zm + p).astype(object) * (y * half % p * pow(root(p), -1, p) % p * other)
-        assert w.max() < 2 ** 26
-        pq = math.prod(ps[q:q + 2])
+            zp, zm = reduce(am.T @ bp, p), reduce(ap.T @ bm, p)         # exact: K 127^2 < 2^27
+            y, half, other = pow(M // p, -1, p), pow(2, -1, p), pq // p
+            for c, f in ((0, y * half % p * other), (1, y * half % p * pow(root(p), -1, p) % p * other)):
+                f -= pq if f > pq // 2 else 0
+                for sgn in (1, -1):                                     # two signed bytes hold +-f
+                    lo = sym(sgn * f, 256) if sym(sgn * f, 256) < 128 else -128
+                    assert -128 <= (sgn * f - lo) // 256 <= 127
+                w[c] += f * (zp + (-1) ** c * zm).astype(object)
+        assert w.min() >= 0 and w.max() < 2 ** 27
         t += w * (((1 << 96) + pq // 2) // pq)
-        bound += 2 ** 26 / 2
+        bound += 2 ** 27 / 2
     for part, exact in ((0, lambda i, j: ar[:, i].astype(object) @ br[:, j] + ai[:, i].astype(object) @ bi[:, j]),
                         (1, lambda i, j: ar[:, i].astype(object) @ bi[:, j] - ai[:, i].astype(object) @ br[:, j])):
         for i in range(4):
@@ -131,17 +152,25 @@ def test_products_recombine(n):
 @pytest.mark.parametrize("ntiles,ncl,planes", [(1, 28, 28), (2, 56, 28), (3, 74, 28), (74, 74, 28), (75, 74, 28),
                                                (147, 74, 30), (540, 74, 28)])
 def test_work_list_covers_every_product_once(ntiles, ncl, planes):
-    full, rest = divmod(ntiles, ncl)
+    full = ntiles // ncl
+    pairs, full_end = (ntiles - full * ncl) * planes, full * ncl
     seen, most, least = set(), 0, 1 << 30
     for c in range(ncl):
-        count = full * planes + (rest * planes - c + ncl - 1) // ncl
+        first = pairs * c // ncl
+        count = full * planes + pairs * (c + 1) // ncl - first
         most, least = max(most, count), min(least, count)
-        for i in range(count):
-            if i < full * planes:
-                u = ((i // planes) * ncl + c, i % planes)
-            else:
-                v = (i - full * planes) * ncl + c
-                u = (full * ncl + v % rest, v // rest)
-            assert u not in seen and u[0] < ntiles and u[1] < planes
-            seen.add(u)
+        rest = (full_end + first // planes, first % planes)
+        tile, P = (c, 0) if full else rest
+        for _ in range(count):
+            assert (tile, P) not in seen and tile < ntiles
+            seen.add((tile, P))
+            P += 1
+            if P == planes:
+                P = 0
+                if tile >= full_end:
+                    tile += 1
+                else:
+                    tile += ncl
+                    if tile >= full_end:
+                        tile, P = rest
     assert len(seen) == ntiles * planes and most - least <= 1
