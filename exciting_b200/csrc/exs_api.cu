@@ -159,6 +159,7 @@ int exs_ctx_destroy(exs_ctx *c)
     if (c->d_res) cudaFree(c->d_res);
     if (c->d_pace) cudaFree(c->d_pace);
     if (c->d_ozscale) cudaFree(c->d_ozscale);
+    if (c->d_ozpart) cudaFree(c->d_ozpart);
     if (c->d_xs) cudaFree(c->d_xs);
     if (c->d_xsig) cudaFree(c->d_xsig);
     if (c->fk_dev) cudaFree(c->fk_dev);
@@ -407,6 +408,7 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
     if (c->d_res) { cudaFree(c->d_res); c->d_res = nullptr; c->res_bytes = 0; }
     if (c->d_pace) { cudaFree(c->d_pace); c->d_pace = nullptr; }
     if (c->d_ozscale) { cudaFree(c->d_ozscale); c->d_ozscale = nullptr; }
+    if (c->d_ozpart) { cudaFree(c->d_ozpart); c->d_ozpart = nullptr; }
     if (c->d_xs) { cudaFree(c->d_xs); c->d_xs = nullptr; }
     if (c->d_xsig) { cudaFree(c->d_xsig); c->d_xsig = nullptr; }
     // per-atom operands: windows of 128-byte chunks; slices: 64-row blocks of h_a and lo rows, moduli:
@@ -446,6 +448,8 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
         if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_pace, exs::ring_pace_bytes());
     }
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_ozscale, sizeof(double) * 3 * c->npad * c->max_batch);
+    if (e == cudaSuccess && mod)
+        e = cudaMalloc((void **)&c->d_ozpart, sizeof(double) * c->natmtot * c->npad * c->max_batch);
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_xs, xs_bytes);
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_xsig, sizeof(double) * nxsig);
     if (e != cudaSuccess || c->oz_xseg < 1) {
@@ -657,7 +661,7 @@ int exs_match(exs_ctx *c, int ngp, const double *gpc, const double *tpgpc, const
                                sizeof(exs_complex) * ngp, c->natmtot, cudaMemcpyHostToDevice, s));
     (void)cudaGetLastError();
     EXS_CUDA(cudaEventRecord(c->ev[0], s));
-    EXS_CUDA(exs::launch_match_ref(c->params(), ngp, c->ngkmax, c->d_match_in, c->d_match_in + c->ngkmax,
+    EXS_CUDA(exs::launch_match_ref(c->params(), ngp, c->d_match_in, c->d_match_in + c->ngkmax,
                                    c->d_match_sf, c->d_apwalm, s));
     for (int i = 1; i <= 4; i++) EXS_CUDA(cudaEventRecord(c->ev[i], s));
     c->timed = true;
@@ -878,7 +882,7 @@ int enqueue_setup(exs_ctx *c, const std::vector<KDesc> &ks, const Uploaded &u, b
     if (timed) EXS_CUDA(cudaEventRecord(c->ev[i], s))
     EXS_EV(0);
     if (!have_planes) EXS_CUDA(oz_reset_maxima(c, ks, s));
-    if (!have_planes) EXS_CUDA(exs::launch_match_planes(p, u.d_k, (int)ks.size(), ngp_max, s));
+    if (!have_planes) EXS_CUDA(exs::launch_match_planes(p, u.d_k, (int)ks.size(), !c->oz_sch.mod, s));
     if (c->relativity == EXS_REL_IORA) EXS_CUDA(exs::launch_iora_planes(p, u.d_k, (int)ks.size(), ngp_max, s));
     EXS_EV(1);
     const bool oz = c->oz_on(), mod = oz && c->oz_sch.mod;
@@ -974,6 +978,7 @@ KDesc slot_desc(exs_ctx *c, int slot, int ngp, const int *d_igpig, const double 
     k.oz_slices = c->d_oz ? c->d_oz + (size_t)slot * c->oz_slot_bytes : nullptr;
     const bool oz = c->oz_on() && c->d_ozscale;
     k.oz_scale = oz ? c->d_ozscale + (size_t)slot * 3 * c->npad : nullptr;
+    k.oz_part = oz && c->oz_sch.mod ? c->d_ozpart + (size_t)slot * c->natmtot * c->npad : nullptr;
     k.oz_slot = slot;
     return k;
 }
@@ -1764,7 +1769,8 @@ int exs_hamiltonandoverlapsetup(exs_ctx *c, int ngp, const exs_complex *apwalm, 
     std::vector<KDesc> ks;
     ks.push_back(slot_desc(c, 0, ngp, c->d_igpig, c->d_vgpc, c->d_ho, c->d_ho + (size_t)c->nmatmax * c->nmatmax));
     EXS_CUDA(oz_reset_maxima(c, ks, s));
-    EXS_CUDA(exs::launch_apwalm_to_planes(c->params(), ngp, c->d_apwalm, ks[0].ar, ks[0].ai, ks[0].oz_scale, s));
+    EXS_CUDA(exs::launch_apwalm_to_planes(c->params(), ngp, c->d_apwalm, ks[0].ar, ks[0].ai,
+                                          c->oz_sch.mod ? nullptr : ks[0].oz_scale, ks[0].oz_part, s));
     int rc = run_setup(c, ks, true);
     if (rc < 0) return rc;
     const size_t bytes = sizeof(exs_complex) * (size_t)ks[0].nmat * ks[0].nmat;

@@ -136,6 +136,7 @@ struct KDesc {
     int8_t *oz_slices;       // split-precision path: int8 slices of this slot [S][4 arrays][npad][kp8]
     double *oz_scale;        // split-precision path: column bounds of A and B [2][npad] (maxima with slices,
                              // 2-norms with moduli; the scale is the power of two above; null: FP64 path)
+    double *oz_part;         // moduli: sums of squares of the A columns per atom [natmtot][npad], else null
     int oz_slot;             // split-precision path: slot index in the slice tensor maps
 };
 
@@ -314,6 +315,7 @@ struct exs_ctx {
     int oz_seg = 0;              // slice pairs per exact int32 segment
     int8_t *d_oz = nullptr;      // int8 slices of all slots
     double *d_ozscale = nullptr; // column scales of all slots
+    double *d_ozpart = nullptr;  // moduli: sums of squares of the A columns per atom, all slots
     size_t oz_slot_bytes = 0;
     CUtensorMap oz_mapA[exs::OZ_NCFG], oz_mapB[exs::OZ_NCFG];   // TMA views of d_oz per pipeline configuration
     CUtensorMap oz_mapB2[exs::OZ_NCFG];                            // half-B views (two-SM tiles)
@@ -352,12 +354,13 @@ struct exs_ctx {
 
 // Launch helpers implemented in the .cu files.
 namespace exs {
-cudaError_t launch_match_planes(const DevParams &p, const KDesc *d_k, int nk, int ngp_max, cudaStream_t s);
+// maxima: split precision by slices (column maxima raised in oz_scale); else sums of squares into oz_part
+cudaError_t launch_match_planes(const DevParams &p, const KDesc *d_k, int nk, int maxima, cudaStream_t s);
 cudaError_t launch_match_dlu(const DevParams &p, double *dlu, cudaStream_t s);
-cudaError_t launch_match_ref(const DevParams &p, int ngp, int ngkmax, const double *gpc, const double *tpgpc,
+cudaError_t launch_match_ref(const DevParams &p, int ngp, const double *gpc, const double *tpgpc,
                              const exs_complex *sfacgp, exs_complex *apwalm, cudaStream_t s);
 cudaError_t launch_apwalm_to_planes(const DevParams &p, int ngp, const exs_complex *apwalm, double *ar,
-                                    double *ai, double *amax, cudaStream_t s);
+                                    double *ai, double *amax, double *part, cudaStream_t s);
 cudaError_t launch_iora_planes(const DevParams &p, const KDesc *d_k, int nk, int ngp_max, cudaStream_t s);
 cudaError_t launch_lolo_blocks(const DevParams &p, const KDesc *d_k, int nk, cudaStream_t s);
 cudaError_t launch_olp_apwlo(const DevParams &p, const KDesc *d_k, int nk, int ngp_max, cudaStream_t s);

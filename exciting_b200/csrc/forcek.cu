@@ -575,7 +575,7 @@ int run_adjoint(exs_ctx *c, int ngp, const int *igpig, const double *vgpc, int n
     // ---- launches
     (void)cudaGetLastError();   // launch checks below read the last error: start clean
     const exs::DevParams p = c->params();
-    FK_CUDA(exs::launch_match_planes(p, d_k, 1, ngp, s));
+    FK_CUDA(exs::launch_match_planes(p, d_k, 1, 0, s));
     {
         dim3 blk(32, 8), grd((ngp + 31) / 32, (c->K + 31) / 32);
         exs::fk_transpose_a<<<grd, blk, 0, s>>>(c->K, ngp, npad, Kp, kd.ar, kd.ai, fw.atr, fw.ati);

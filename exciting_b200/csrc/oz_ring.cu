@@ -98,7 +98,7 @@ __device__ __forceinline__ uint2 ring_digits(double x, double sc)
     return make_uint2((uint32_t)u, (uint32_t)(u >> 32));
 }
 
-// Column 2-norms of the A, B or C planes (which = 0, 1, 2) into oz_scale
+// Column 2-norms of the B or C planes (which = 1, 2) into oz_scale
 // block `which`.  One column per thread column of a 32 x 32 block, the rows
 // of threads covering interleaved rows f (stride 32), the partial sums
 // combined in a fixed order, so that the scales, and every result, are the
@@ -131,6 +131,18 @@ __global__ void __launch_bounds__(1024) oz_norm_kernel(DevParams p, const KDesc 
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     const int gc = blockIdx.x * 32 + ty;
     if (tx == 0 && gc < p.npad) k.oz_scale[(size_t)which * p.npad + gc] = sqrt(t) * (1.0 + 0x1p-30);
+}
+
+// The same for A from the sums of squares that its producer left per atom,
+// added in the order of the atoms.
+__global__ void __launch_bounds__(64) oz_norm_parts_kernel(DevParams p, const KDesc *ks)
+{
+    const KDesc k = ks[blockIdx.y];
+    const int g = blockIdx.x * 64 + threadIdx.x;
+    double t = 0.0;
+#pragma unroll 8
+    for (int a = 0; a < p.natmtot; a++) t += k.oz_part[(size_t)a * p.npad + g];
+    k.oz_scale[g] = sqrt(t) * (1.0 + 0x1p-30);
 }
 
 // The 2n residue planes of one operand (which = 0: A, 1: B, 2: C).  A
@@ -1117,7 +1129,10 @@ void ring_row_blocks(int rows, int *nb, int *nrows)
 
 cudaError_t launch_oz_norm(const DevParams &p, const KDesc *d_k, int nk, int which, cudaStream_t s)
 {
-    oz_norm_kernel<<<dim3(p.npad / 32, nk), dim3(32, 32), 0, s>>>(p, d_k, which);
+    if (which == 0)
+        oz_norm_parts_kernel<<<dim3(p.npad / 64, nk), 64, 0, s>>>(p, d_k);      // npad: a multiple of 64
+    else
+        oz_norm_kernel<<<dim3(p.npad / 32, nk), dim3(32, 32), 0, s>>>(p, d_k, which);
     return cudaGetLastError();
 }
 

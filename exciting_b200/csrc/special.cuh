@@ -2,11 +2,11 @@
 //
 // Each routine follows the reference routine named beside it step by step, so
 // that the device values agree with the reference to rounding:
-//   exs_sbessel    -- src/src_lib/sbessel.f90:48-147
-//   exs_sbesseldm  -- src/src_lib/sbesseldm.f90:40-130
-//   exs_ylm_l      -- one l of src/src_lib/genylm.f90:50-92
-//   exs_polynom    -- src/src_lib/polynom.f90 (m >= 0 branches)
-//   exs_sphcrd     -- src/src_lib/sphcrd.f90:30-56
+//   sbessel    -- src/src_lib/sbessel.f90:48-147
+//   sbesseldm_*    -- src/src_lib/sbesseldm.f90:40-130
+//   ylm_l      -- one l of src/src_lib/genylm.f90:50-92
+//   polynom    -- src/src_lib/polynom.f90 (m >= 0 branches)
+//   sphcrd     -- src/src_lib/sphcrd.f90:30-56
 // sin, cos, sqrt, acos and atan2 are CUDA's own functions.
 #pragma once
 #include <cuda_runtime.h>
@@ -54,8 +54,15 @@ __device__ inline double factr(int n, int d)
     return r;
 }
 
-// j_l(x), l = 0..lmax.  Caller guarantees 0 <= lmax <= EXS_LMAX_APW+1.
-__device__ inline void sbessel(int lmax, double x, double *jl)
+// One value per l at a stride (the lanes of a warp side by side in shared memory).
+struct Strided {
+    double *p;
+    int ld;
+    __device__ double &operator[](int l) const { return p[l * ld]; }
+};
+
+// j_l(x), l = 0..lmax.
+__device__ inline void sbessel(int lmax, double x, Strided jl)
 {
     const int lst = 25;
     const double rsc = 1e150, rsci = 1.0 / 1e150;
@@ -109,66 +116,69 @@ __device__ inline void sbessel(int lmax, double x, double *jl)
     }
 }
 
-// m-th derivative of j_l(x), l = 0..lmax (m <= 6).
-__device__ inline void sbesseldm(int m, int lmax, double x, double *djl)
+// m-th derivative (1 <= m <= 6) of j_l(x), l = 0..lmax, for x > 1 from
+// jl = j_0..j_{lmax+1}(x) (sbesseldm.f90:65-99): for m = 1 the recurrence's
+// a = (0, l), a1 = (-1) give -j_{l+1} + l j_l / x.
+__device__ inline void sbesseldm_large(int m, int lmax, double x, Strided jl, Strided djl)
 {
-    if (m == 0) { sbessel(lmax, x, djl); return; }
-    const int maxns = 20;
-    if (x > 1.0) {
-        double jl[EXS_LMAX_APW + 3];
-        int a[8], a1[8], b[8], b1[8];
-        sbessel(lmax + 1, x, jl);
-        for (int l = 0; l <= lmax; l++) {
-            for (int i = 1; i <= m + 1; i++) a[i] = 0;
-            a[0] = 1;
-            for (int i = 0; i <= m + 1; i++) a1[i] = 0;
-            for (int i = 1; i <= m; i++) {
-                b[0] = 0;
-                b1[0] = 0;
-                for (int j = 0; j <= i; j++) {
-                    b[j + 1] = a[j] * (l - j);
-                    b1[j + 1] = -a1[j] * (j + l + 2);
-                }
-                for (int j = 0; j <= i; j++) {
-                    b1[j] = b1[j] - a[j];
-                    b[j] = b[j] + a1[j];
-                }
-                for (int j = 0; j <= i + 1; j++) { a[j] = b[j]; a1[j] = b1[j]; }
-            }
-            double t1 = 1.0;
-            double sum = (double)a[0] * jl[l] + (double)a1[0] * jl[l + 1];
-            for (int i = 1; i <= m + 1; i++) {
-                t1 = t1 * x;
-                sum = sum + ((double)a[i] * jl[l] + (double)a1[i] * jl[l + 1]) / t1;
-            }
-            djl[l] = sum;
-        }
-    } else {
-        const double x2 = x * x;
-        for (int l = 0; l <= lmax; l++) {
-            int i0 = (m - l + 1) / 2;
-            if (i0 < 0) i0 = 0;
-            int j = 2 * i0 + l - m;
-            double t1 = (j == 0) ? 1.0 : powi(x, j);
-            const double p2 = powi(-2.0, i0);
-            t1 = factr(j + m, j) * t1 / (factnm(i0, 1) * factnm(j + l + m + 1, 2) * p2);
-            double sum = t1;
-            for (int i = i0 + 1; i <= maxns; i++) {
-                j = 2 * i + l;
-                t1 = -t1 * (double)((j - 1) * j) * x2
-                     / (double)((j - l) * (j - m - 1) * (j - m) * (j + l + 1));
-                if (fabs(t1) <= 1e-40) break;
-                sum = sum + t1;
-            }
-            djl[l] = sum;
-        }
+    if (m == 1) {
+        for (int l = 0; l <= lmax; l++) djl[l] = -jl[l + 1] + (double)l * jl[l] / x;
+        return;
     }
+    int a[8], a1[8], b[8], b1[8];
+    for (int l = 0; l <= lmax; l++) {
+        for (int i = 1; i <= m + 1; i++) a[i] = 0;
+        a[0] = 1;
+        for (int i = 0; i <= m + 1; i++) a1[i] = 0;
+        for (int i = 1; i <= m; i++) {
+            b[0] = 0;
+            b1[0] = 0;
+            for (int j = 0; j <= i; j++) {
+                b[j + 1] = a[j] * (l - j);
+                b1[j + 1] = -a1[j] * (j + l + 2);
+            }
+            for (int j = 0; j <= i; j++) {
+                b1[j] = b1[j] - a[j];
+                b[j] = b[j] + a1[j];
+            }
+            for (int j = 0; j <= i + 1; j++) { a[j] = b[j]; a1[j] = b1[j]; }
+        }
+        double t1 = 1.0;
+        double sum = (double)a[0] * jl[l] + (double)a1[0] * jl[l + 1];
+        for (int i = 1; i <= m + 1; i++) {
+            t1 = t1 * x;
+            sum = sum + ((double)a[i] * jl[l] + (double)a1[i] * jl[l + 1]) / t1;
+        }
+        djl[l] = sum;
+    }
+}
+
+// The same for x <= 1 and one l: the power series (sbesseldm.f90:100-125).
+__device__ inline double sbesseldm_small(int m, int l, double x)
+{
+    const int maxns = 20;
+    const double x2 = x * x;
+    int i0 = (m - l + 1) / 2;
+    if (i0 < 0) i0 = 0;
+    int j = 2 * i0 + l - m;
+    double t1 = (j == 0) ? 1.0 : powi(x, j);
+    const double p2 = powi(-2.0, i0);
+    t1 = factr(j + m, j) * t1 / (factnm(i0, 1) * factnm(j + l + m + 1, 2) * p2);
+    double sum = t1;
+    for (int i = i0 + 1; i <= maxns; i++) {
+        j = 2 * i + l;
+        t1 = -t1 * (double)((j - 1) * j) * x2
+             / (double)((j - l) * (j - m - 1) * (j - m) * (j + l + 1));
+        if (fabs(t1) <= 1e-40) break;
+        sum = sum + t1;
+    }
+    return sum;
 }
 
 // Real Masters & Richards-Dinger values of one l: x(m), m = 0..l, already
 // multiplied by sin(theta)^m and normalised, i.e. Y_lm = xm[m] * e^{i m phi}
 // for m >= 0 (genylm.f90:58-83).  Y_00 = 0.28209479177387814347.
-__device__ inline void ylm_l(int l, double sn, double cs, double *xm)
+__device__ inline void ylm_l(int l, double sn, double cs, Strided xm)
 {
     const double fourpi = 12.566370614359172954;
     if (l == 0) { xm[0] = 0.28209479177387814347; return; }
@@ -280,21 +290,29 @@ __device__ inline int lu_factor(int n, double *d, int *ipiv)
     return 0;
 }
 
-// zgetrs steps for one complex right-hand side (re, im held separately).
-__device__ inline void lu_solve(int n, const double *d, const int *ipiv, double *br, double *bi)
+// zgetrs steps for one real right-hand side; d and the pivots in memory, b
+// indexed statically (it stays in registers).
+template <int N>
+__device__ inline void lu_solve(const double *d, const double *ipiv, double (&b)[N])
 {
-    for (int k = 0; k < n; k++)
-        if (ipiv[k] != k) {
-            const int p = ipiv[k];
-            double t = br[k]; br[k] = br[p]; br[p] = t;
-            t = bi[k]; bi[k] = bi[p]; bi[p] = t;
-        }
-    for (int k = 0; k < n; k++)
-        for (int i = k + 1; i < n; i++) { br[i] -= br[k] * d[i + k * n]; bi[i] -= bi[k] * d[i + k * n]; }
-    for (int k = n - 1; k >= 0; k--) {
-        br[k] = br[k] / d[k + k * n];
-        bi[k] = bi[k] / d[k + k * n];
-        for (int i = 0; i < k; i++) { br[i] -= br[k] * d[i + k * n]; bi[i] -= bi[k] * d[i + k * n]; }
+#pragma unroll
+    for (int k = 0; k < N; k++)
+#pragma unroll
+        for (int i = k + 1; i < N; i++)
+            if ((int)ipiv[k] == i) {
+                const double t = b[k];
+                b[k] = b[i];
+                b[i] = t;
+            }
+#pragma unroll
+    for (int k = 0; k < N; k++)
+#pragma unroll
+        for (int i = k + 1; i < N; i++) b[i] -= b[k] * d[i + k * N];
+#pragma unroll
+    for (int k = N - 1; k >= 0; k--) {
+        b[k] = b[k] / d[k + k * N];
+#pragma unroll
+        for (int i = 0; i < k; i++) b[i] -= b[k] * d[i + k * N];
     }
 }
 
