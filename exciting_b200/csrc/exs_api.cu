@@ -680,9 +680,9 @@ namespace {
 // buffer, upload them with one copy and return the device addresses.
 struct Uploaded {
     const KDesc *d_k;
-    const void *d_probs[4];
-    const void *d_work[4];
-    int nwork[4];
+    const void *d_probs;
+    const void *d_work[3];
+    int nwork[3], edge[3];
     const void *d_oztiles;
     int noztiles;
     const void *d_ozatiles;   // per-atom tiles of the split-precision path
@@ -744,8 +744,8 @@ void oz_atom_tiles(const exs_ctx *c, const std::vector<KDesc> &ks, std::vector<i
 
 // Layout of the packed tables (byte offsets from the start of the buffer).
 struct TableLayout {
-    size_t k, probs[4], work[4], oz, oza, total;
-    int nwork[4], noz, noza;
+    size_t k, probs, work[3], oz, oza, total;
+    int nwork[3], edge[3], noz, noza;
 };
 
 void pack_tables(exs_ctx *c, const std::vector<KDesc> &ks, std::vector<int> &ozt, TableLayout &L)
@@ -767,12 +767,13 @@ void pack_tables(exs_ctx *c, const std::vector<KDesc> &ks, std::vector<int> &ozt
     size_t off = 0;
     L.k = off;
     off += al(ks.size() * sizeof(KDesc));
-    for (int q = 0; q < 4; q++) {
-        L.probs[q] = off;
-        off += al(c->gt.probs[q].size() * sizeof(exs::GemmProb));
+    L.probs = off;
+    off += al(c->gt.probs.size() * sizeof(exs::GemmProb));
+    for (int q = 0; q < 3; q++) {
         L.work[q] = off;
         off += al(c->gt.work[q].size() * sizeof(exs::TileWork));
         L.nwork[q] = (int)c->gt.work[q].size();
+        L.edge[q] = c->gt.edge[q];
     }
     L.oz = off;
     L.oza = off + sizeof(int) * 3 * (size_t)L.noz;
@@ -784,12 +785,10 @@ void write_tables(const exs_ctx *c, const std::vector<KDesc> &ks, const std::vec
                   char *h)
 {
     std::memcpy(h + L.k, ks.data(), ks.size() * sizeof(KDesc));
-    for (int q = 0; q < 4; q++) {
-        if (!c->gt.probs[q].empty())
-            std::memcpy(h + L.probs[q], c->gt.probs[q].data(), c->gt.probs[q].size() * sizeof(exs::GemmProb));
+    std::memcpy(h + L.probs, c->gt.probs.data(), c->gt.probs.size() * sizeof(exs::GemmProb));
+    for (int q = 0; q < 3; q++)
         if (!c->gt.work[q].empty())
             std::memcpy(h + L.work[q], c->gt.work[q].data(), c->gt.work[q].size() * sizeof(exs::TileWork));
-    }
     if (!ozt.empty()) std::memcpy(h + L.oz, ozt.data(), ozt.size() * sizeof(int));
 }
 
@@ -797,10 +796,11 @@ Uploaded device_view(const TableLayout &L, char *d)
 {
     Uploaded u{};
     u.d_k = (const KDesc *)(d + L.k);
-    for (int q = 0; q < 4; q++) {
-        u.d_probs[q] = d + L.probs[q];
+    u.d_probs = d + L.probs;
+    for (int q = 0; q < 3; q++) {
         u.d_work[q] = d + L.work[q];
         u.nwork[q] = L.nwork[q];
+        u.edge[q] = L.edge[q];
     }
     u.d_oztiles = d + L.oz;
     u.noztiles = L.noz;
@@ -913,9 +913,12 @@ int enqueue_setup(exs_ctx *c, const std::vector<KDesc> &ks, const Uploaded &u, b
             EXS_CUDA(exs::launch_oz_atom(c->oz_cfg, &c->oz_mapArow, &c->oz_mapX, p, u.d_k, u.d_ozatiles,
                                          u.nozatiles, c->oz_sch, c->kp8, c->oz_atom_args(), s));
     }
-    if (b64) {
-        EXS_CUDA(exs::launch_gemm_kind(exs::EPI_PLANAR, p, u.d_probs[exs::EPI_PLANAR], u.d_work[exs::EPI_PLANAR],
-                                       u.nwork[exs::EPI_PLANAR], u.d_k, s));
+    auto gemm = [&](int group, int q) {
+        return exs::launch_gemm(group, u.edge[q], p, u.d_probs, u.d_work[q], u.nwork[q], u.d_k, s);
+    };
+    if (b64) {   // h_a A and the APW-lo rows of H
+        EXS_CUDA(gemm(0, 0));
+        EXS_CUDA(gemm(0, 1));
     }
     EXS_EV(2);
     if (oz) {
@@ -928,15 +931,9 @@ int enqueue_setup(exs_ctx *c, const std::vector<KDesc> &ks, const Uploaded &u, b
             EXS_CUDA(exs::launch_oz_mma(q, &c->oz_mapA[q], (q & 8) ? &c->oz_mapB2[q] : &c->oz_mapB[q], p, u.d_k,
                                         u.d_oztiles, u.noztiles, c->oz_sch, c->kp8, s));
     } else {
-        EXS_CUDA(exs::launch_gemm_kind(exs::EPI_HAM, p, u.d_probs[exs::EPI_HAM], u.d_work[exs::EPI_HAM],
-                                       u.nwork[exs::EPI_HAM], u.d_k, s));
-        EXS_CUDA(exs::launch_gemm_kind(exs::EPI_OVL, p, u.d_probs[exs::EPI_OVL], u.d_work[exs::EPI_OVL],
-                                       u.nwork[exs::EPI_OVL], u.d_k, s));
+        EXS_CUDA(gemm(1, 2));
     }
     EXS_EV(3);
-    if (b64)
-        EXS_CUDA(exs::launch_gemm_kind(exs::EPI_LOROWS, p, u.d_probs[exs::EPI_LOROWS], u.d_work[exs::EPI_LOROWS],
-                                       u.nwork[exs::EPI_LOROWS], u.d_k, s));
     EXS_CUDA(exs::launch_olp_apwlo(p, u.d_k, (int)ks.size(), ngp_max, s));
     EXS_CUDA(exs::launch_lolo_blocks(p, u.d_k, (int)ks.size(), s));
     EXS_EV(4);

@@ -206,14 +206,15 @@ struct GemmProb {
     const double *yr, *yi;
     long ldy;
     int M, N, K;
-    int conjx;
+    short conjx;
+    short kind;            // EpiKind
     double *outr, *outi;   // EPI_PLANAR output [m][n]
     long ldo;
     exs_complex *z;        // EPI_HAM / EPI_OVL / EPI_LOROWS: za(ldz, *)
     long ldz;
     int row0;              // EPI_LOROWS: za row of m = 0
     int kidx;              // k-point of this problem (interstitial tables)
-    double *colmax;        // EPI_PLANAR: column maxima of |out| raised atomically (split precision), or null
+    double *colmax;        // EPI_PLANAR: column maxima of |out| raised atomically (slices), or null
 };
 
 struct TileWork {
@@ -221,8 +222,10 @@ struct TileWork {
 };
 
 struct GemmTables {
-    std::vector<GemmProb> probs[4];
-    std::vector<TileWork> work[4];
+    std::vector<GemmProb> probs;
+    int first_lo = 0, first_ho = 0;      // probs: h_a A, from first_lo the APW-lo rows, from first_ho H and O
+    std::vector<TileWork> work[3];       // tiles of the three
+    int edge[3] = {64, 64, 64};          // and their edges
 };
 
 }  // namespace exs
@@ -366,8 +369,10 @@ cudaError_t launch_lolo_blocks(const DevParams &p, const KDesc *d_k, int nk, cud
 cudaError_t launch_olp_apwlo(const DevParams &p, const KDesc *d_k, int nk, int ngp_max, cudaStream_t s);
 // Grouped FP64 GEMM stages (setup_f64.cu)
 void build_gemm_tables(const exs_ctx *c, const std::vector<KDesc> &ks, GemmTables &t);
-cudaError_t launch_gemm_kind(int kind, const DevParams &p, const void *d_probs, const void *d_work, int nwork,
-                             const KDesc *d_k, cudaStream_t s);
+int gemm_edge_of(const std::vector<GemmProb> &probs, int first, int last);
+void gemm_tiles(const std::vector<GemmProb> &probs, int first, int last, int edge, std::vector<TileWork> &w);
+cudaError_t launch_gemm(int group, int edge, const DevParams &p, const void *d_probs, const void *d_work, int nwork,
+                        const KDesc *d_k, cudaStream_t s);
 // Device eigen-solve (solve.cu)
 void solver_release(exs_ctx *c);
 // Muffin-tin integral generation (mtint.cu)

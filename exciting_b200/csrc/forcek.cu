@@ -422,13 +422,6 @@ cudaError_t grow(void **p, size_t *cap, size_t need, bool pinned)
     return e;
 }
 
-void add_tiles(std::vector<TileWork> &w, int pi, int M, int N, bool upper)
-{
-    const int tm = (M + 63) / 64, tn = (N + 63) / 64;
-    for (int a = 0; a < tm; a++)
-        for (int b = upper ? a : 0; b < tn; b++) w.push_back({pi, a, b});
-}
-
 // The whole adjoint of one k-point.  Fills c->fk_force (device, 3*natmtot),
 // the scatter sums and U; returns an EXS_ code.
 int run_adjoint(exs_ctx *c, int ngp, const int *igpig, const double *vgpc, int nst, const exs_complex *evec, int ldv,
@@ -524,11 +517,12 @@ int run_adjoint(exs_ctx *c, int ngp, const int *igpig, const double *vgpc, int n
         P.yr = fw.ct[0][0]; P.yi = fw.ct[0][1]; P.ldy = ldu;
         P.M = c->K; P.N = ldu; P.K = ngp; P.conjx = 0;
         P.outr = fw.u[0][0]; P.outi = fw.u[0][1]; P.ldo = ldu;
-        add_tiles(w1, (int)probs.size(), P.M, P.N, false);
         probs.push_back(P);
     }
+    const int e_u = exs::gemm_edge_of(probs, 0, 1);
+    exs::gemm_tiles(probs, 0, 1, e_u, w1);
     for (int i0 = 0; i0 < ngp; i0 += band) {   // P^T = conj(C)^T (w C), Q^T = conj(C)^T (w eps C): rows i0..,
-        wb_off.push_back(wb.size());             // columns j >= i0 (the scatter takes the upper triangle)
+                                               // columns j >= i0 (the scatter takes the upper triangle)
         for (int which = 0; which < 2; which++) {
             GemmProb P{};
             P.xr = fw.cn[0] + i0; P.xi = fw.cn[1] + i0; P.ldx = npad;
@@ -536,9 +530,13 @@ int run_adjoint(exs_ctx *c, int ngp, const int *igpig, const double *vgpc, int n
             P.ldy = npad;
             P.M = std::min(band, ngp - i0); P.N = ngp - i0; P.K = nst; P.conjx = 1;
             P.outr = which == 0 ? fw.pt[0] : fw.qt[0]; P.outi = which == 0 ? fw.pt[1] : fw.qt[1]; P.ldo = npad;
-            add_tiles(wb, (int)probs.size(), P.M, P.N, false);
             probs.push_back(P);
         }
+    }
+    const int nb = (int)probs.size(), e_b = exs::gemm_edge_of(probs, 1, std::min(nb, 3));
+    for (int i = 1; i < nb; i += 2) {          // tiles of one band
+        wb_off.push_back(wb.size());
+        exs::gemm_tiles(probs, i, i + 2, e_b, wb);
     }
     wb_off.push_back(wb.size());
     for (int ias = 0; ias < c->natmtot; ias++) {   // h_a [U_0 .. U_3] per atom, N = 4 nstp
@@ -550,9 +548,10 @@ int run_adjoint(exs_ctx *c, int ngp, const int *igpig, const double *vgpc, int n
         P.M = a.napw; P.N = ldu; P.K = a.napw; P.conjx = 0;
         P.outr = fw.hu[0][0] + (size_t)a.apw_off * ldu; P.outi = fw.hu[0][1] + (size_t)a.apw_off * ldu;
         P.ldo = ldu;
-        add_tiles(w2, (int)probs.size(), P.M, P.N, false);
         probs.push_back(P);
     }
+    const int e_h = exs::gemm_edge_of(probs, nb, (int)probs.size());
+    exs::gemm_tiles(probs, nb, (int)probs.size(), e_h, w2);
     const size_t kb = al256(sizeof(KDesc)), pb = al256(sizeof(GemmProb) * probs.size());
     const size_t wbytes = sizeof(TileWork) * (w1.size() + w2.size() + wb.size());
     const size_t tb = kb + pb + wbytes;
@@ -582,8 +581,8 @@ int run_adjoint(exs_ctx *c, int ngp, const int *igpig, const double *vgpc, int n
         exs::fk_pack_evec<<<dim3((ngp + 127) / 128, nstp), 128, 0, s>>>(fw, npad, c->d_vgpc, nmat);
         FK_CUDA(cudaGetLastError());
     }
-    FK_CUDA(exs::launch_gemm_kind(exs::EPI_PLANAR, p, d_p, d_w1, (int)w1.size(), d_k, s));
-    FK_CUDA(exs::launch_gemm_kind(exs::EPI_PLANAR, p, d_p, d_w2, (int)w2.size(), d_k, s));
+    FK_CUDA(exs::launch_gemm(0, e_u, p, d_p, d_w1, (int)w1.size(), d_k, s));
+    FK_CUDA(exs::launch_gemm(0, e_h, p, d_p, d_w2, (int)w2.size(), d_k, s));
     if (iora) exs::fk_iora_u<<<dim3((nstp + 63) / 64, c->natmtot, 4), 64, 0, s>>>(p, fw);
     const unsigned fch = (unsigned)((c->maxaa + exs::FK_FROWS - 1) / exs::FK_FROWS);
     exs::fk_terms_mt<<<dim3(c->natmtot, 3, fch), 64, 0, s>>>(p, fw);
@@ -591,8 +590,7 @@ int run_adjoint(exs_ctx *c, int ngp, const int *igpig, const double *vgpc, int n
         exs::fk_terms_lo<<<dim3(c->natmtot, 3, fch), 256, 0, s>>>(p, fw, c->d_loa_r, c->d_loa_i, c->ldlo, c->maxaa);
     for (size_t b = 0; b + 1 < wb_off.size(); b++) {   // one band of P^T, Q^T, then its scatter
         const int i0 = (int)b * band, i1 = std::min(ngp, i0 + band);
-        FK_CUDA(exs::launch_gemm_kind(exs::EPI_PLANAR, p, d_p, d_wb + wb_off[b], (int)(wb_off[b + 1] - wb_off[b]),
-                                      d_k, s));
+        FK_CUDA(exs::launch_gemm(0, e_b, p, d_p, d_wb + wb_off[b], (int)(wb_off[b + 1] - wb_off[b]), d_k, s));
         exs::fk_scatter<<<dim3((i1 - i0 + 127) / 128, ngp - i0), 128, 0, s>>>(p, fw, d_k, i0, i1);
         FK_CUDA(cudaGetLastError());
     }

@@ -295,9 +295,9 @@ extern "C" int exs_mt_contract_noalloc(int natmtot, int maxaa, const int *napw, 
     na_pack_h<<<dim3((ldh + 63) / 64, ldh, natmtot), 64, 0, s>>>(natmtot, maxaa, ldh, aa, hr, hi);
     if ((e = cudaGetLastError()) != cudaSuccess) return EXS_ERR_CUDA;
     const DevParams none{};
-    e = launch_gemm_kind(EPI_PLANAR, none, d_probs, d_work, (int)nwork_ha, nullptr, s);
+    e = launch_gemm(0, 64, none, d_probs, d_work, (int)nwork_ha, nullptr, s);
     if (e == cudaSuccess)
-        e = launch_gemm_kind(EPI_PLANAR, none, d_probs, d_work + nwork_ha, (int)nwork_main, nullptr, s);
+        e = launch_gemm(0, 64, none, d_probs, d_work + nwork_ha, (int)nwork_main, nullptr, s);
     if (e != cudaSuccess) return EXS_ERR_CUDA;
     na_store_hermitian<<<dim3((ngp + 127) / 128, ngp), 128, 0, s>>>(ngp, np, Hr, Hi, h, ld);
     na_store_hermitian<<<dim3((ngp + 127) / 128, ngp), 128, 0, s>>>(ngp, np, Or, Oi, o, ld);

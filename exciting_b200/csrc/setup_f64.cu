@@ -25,10 +25,27 @@
 
 namespace exs {
 
-constexpr int GB_M = 64, GB_N = 64, GB_K = 16, GB_LDS = GB_M + 8, GB_STAGES = 3, GB_THREADS = 128;
-constexpr int GB_PLANE = GB_K * GB_LDS;                 // doubles per plane per stage
-constexpr int GB_STAGE = 4 * GB_PLANE;                  // xr, xi, yr, yi
-constexpr size_t GB_SMEM = (size_t)GB_STAGES * GB_STAGE * sizeof(double);
+// Tiles are EDGE x EDGE, 128 threads, K slabs of 16 in a three-stage cp.async
+// ring.  EDGE 64 and 32: 2 x 2 warps of EDGE/2 x EDGE/2.  EDGE 16: the four
+// warps share one 16 x 16 tile, each taking every fourth K step, and add their
+// sums in a fixed order at the end: a 64 x 64 tile of K = 316 keeps one SM's
+// FP64 pipe busy for 42 us, so a single k-point of the two-atom cell (six
+// tiles) left 142 SMs idle.  gemm_edge picks the edge.  Rows are padded to
+// 4 (mod 16) doubles: the four K rows and four columns that half a warp reads
+// fall into different banks.
+constexpr int GB_K = 16, GB_STAGES = 3, GB_THREADS = 128;
+template <int EDGE>
+struct GemmCfg {
+    static constexpr int KS = EDGE == 16 ? 4 : 1;               // warps sharing a tile's K
+    static constexpr int WT = EDGE == 16 ? 16 : EDGE / 2;       // edge of a warp's sub-tile
+    static constexpr int MT = WT / 8;                           // 8 x 8 MMA tiles per warp and direction
+    static constexpr int LDS = EDGE + 4;
+    static constexpr int PLANE = GB_K * LDS;                    // doubles per plane per stage
+    static constexpr int STAGE = 4 * PLANE;                     // xr, xi, yr, yi
+    static constexpr int RING = GB_STAGES * STAGE;
+    static constexpr int SUMS = KS > 1 ? (KS - 1) * 32 * MT * MT * 4 : 0;       // the other warps' sums
+    static constexpr size_t SMEM = (size_t)(RING > SUMS ? RING : SUMS) * sizeof(double);
+};
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool valid)
 {
@@ -47,54 +64,63 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
                  : "d"(a), "d"(b));
 }
 
-// Load one K-slab (GB_K rows) of the four operand planes into stage buffer s.
+// Load one K-slab (GB_K rows) of the four operand planes into stage buffer st.
+template <int EDGE>
 __device__ __forceinline__ void load_stage(double *st, const GemmProb &P, int m0, int n0, int k0)
 {
+    using C = GemmCfg<EDGE>;
     const int tid = threadIdx.x;
 #pragma unroll
-    for (int it = 0; it < (GB_K * GB_M / 2) / GB_THREADS; it++) {
+    for (int it = 0; it < (GB_K * EDGE / 2) / GB_THREADS; it++) {
         const int c = tid + it * GB_THREADS;
-        const int row = c / (GB_M / 2);
-        const int col = (c % (GB_M / 2)) * 2;
+        const int row = c / (EDGE / 2);
+        const int col = (c % (EDGE / 2)) * 2;
         const int gk = k0 + row;
         {
             const int gm = m0 + col;
             const bool v = gk < P.K && gm < P.M;
             const size_t off = v ? (size_t)gk * P.ldx + gm : 0;
-            cp_async16(st + 0 * GB_PLANE + row * GB_LDS + col, P.xr + off, v);
-            cp_async16(st + 1 * GB_PLANE + row * GB_LDS + col, P.xi + off, v);
+            cp_async16(st + 0 * C::PLANE + row * C::LDS + col, P.xr + off, v);
+            cp_async16(st + 1 * C::PLANE + row * C::LDS + col, P.xi + off, v);
         }
         {
             const int gn = n0 + col;
             const bool v = gk < P.K && gn < P.N;
             const size_t off = v ? (size_t)gk * P.ldy + gn : 0;
-            cp_async16(st + 2 * GB_PLANE + row * GB_LDS + col, P.yr + off, v);
-            cp_async16(st + 3 * GB_PLANE + row * GB_LDS + col, P.yi + off, v);
+            cp_async16(st + 2 * C::PLANE + row * C::LDS + col, P.yr + off, v);
+            cp_async16(st + 3 * C::PLANE + row * C::LDS + col, P.yi + off, v);
         }
     }
 }
 
-template <int KIND>
+// GROUP 0: EPI_PLANAR and EPI_LOROWS problems, GROUP 1: EPI_HAM and EPI_OVL
+// (the problem's kind); one launch takes a group's problems together.
+template <int GROUP, int EDGE>
 __global__ void __launch_bounds__(GB_THREADS, 2)
 zgemm_dmma_kernel(DevParams p, const GemmProb *probs, const TileWork *work, const KDesc *ks)
 {
+    using C = GemmCfg<EDGE>;
+    constexpr int MT = C::MT;
     extern __shared__ __align__(16) double smem[];
     const TileWork tw = work[blockIdx.x];
     const GemmProb P = probs[tw.prob];
-    const int m0 = tw.tm * GB_M, n0 = tw.tn * GB_N;
+    const int m0 = tw.tm * EDGE, n0 = tw.tn * EDGE;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wm = warp >> 1, wn = warp & 1;
+    const int wm = C::KS > 1 ? 0 : warp >> 1, wn = C::KS > 1 ? 0 : warp & 1;
+    const int mw = wm * C::WT, nw = wn * C::WT;            // this warp's sub-tile
+    // upper tiles: sub-tiles below the diagonal are not formed
+    const bool idle = GROUP == 1 && m0 + mw > n0 + nw + C::WT - 1;
 
-    double cre[4][4][2], cim[4][4][2];
+    double cre[MT][MT][2], cim[MT][MT][2];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < MT; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) { cre[i][j][0] = cre[i][j][1] = cim[i][j][0] = cim[i][j][1] = 0.0; }
+        for (int j = 0; j < MT; j++) { cre[i][j][0] = cre[i][j][1] = cim[i][j][0] = cim[i][j][1] = 0.0; }
 
     const int nkt = (P.K + GB_K - 1) / GB_K;
 #pragma unroll
     for (int s = 0; s < GB_STAGES - 1; s++) {
-        if (s < nkt) load_stage(smem + s * GB_STAGE, P, m0, n0, s * GB_K);
+        if (s < nkt) load_stage<EDGE>(smem + s * C::STAGE, P, m0, n0, s * GB_K);
         cp_async_commit();
     }
     const double sgn = P.conjx ? 1.0 : -1.0;
@@ -103,95 +129,129 @@ zgemm_dmma_kernel(DevParams p, const GemmProb *probs, const TileWork *work, cons
         __syncthreads();
         {
             const int nt = kt + GB_STAGES - 1;
-            if (nt < nkt) load_stage(smem + (nt % GB_STAGES) * GB_STAGE, P, m0, n0, nt * GB_K);
+            if (nt < nkt) load_stage<EDGE>(smem + (nt % GB_STAGES) * C::STAGE, P, m0, n0, nt * GB_K);
             cp_async_commit();
         }
-        const double *st = smem + (kt % GB_STAGES) * GB_STAGE;
+        const double *st = smem + (kt % GB_STAGES) * C::STAGE;
+        if (idle) continue;
 #pragma unroll
-        for (int kk = 0; kk < GB_K / 4; kk++) {
-            const int kr = kk * 4 + (lane & 3);
-            double ar[4], aim[4], naim[4], br[4], bi[4];
+        for (int kq = 0; kq < GB_K / 4 / C::KS; kq++) {
+            const int kr = (C::KS > 1 ? warp : kq) * 4 + (lane & 3);
+            double ar[MT], aim[MT], naim[MT], br[MT], bi[MT];
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int mm = wm * 32 + i * 8 + (lane >> 2);
-                ar[i] = st[0 * GB_PLANE + kr * GB_LDS + mm];
-                aim[i] = sgn * st[1 * GB_PLANE + kr * GB_LDS + mm];   // conj: +ai, plain: -ai
+            for (int i = 0; i < MT; i++) {
+                const int mm = mw + i * 8 + (lane >> 2);
+                ar[i] = st[0 * C::PLANE + kr * C::LDS + mm];
+                aim[i] = sgn * st[1 * C::PLANE + kr * C::LDS + mm];   // conj: +ai, plain: -ai
                 naim[i] = -aim[i];
             }
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int nn = wn * 32 + j * 8 + (lane >> 2);
-                br[j] = st[2 * GB_PLANE + kr * GB_LDS + nn];
-                bi[j] = st[3 * GB_PLANE + kr * GB_LDS + nn];
+            for (int j = 0; j < MT; j++) {
+                const int nn = nw + j * 8 + (lane >> 2);
+                br[j] = st[2 * C::PLANE + kr * C::LDS + nn];
+                bi[j] = st[3 * C::PLANE + kr * C::LDS + nn];
             }
-            // four passes over the 4x4 sub-tiles so that the two products
-            // accumulated into one register pair are 16 DMMAs apart
+            // four passes over the MT x MT sub-tiles so that the two products
+            // accumulated into one register pair are MT^2 DMMAs apart
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < MT; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) dmma(cre[i][j][0], cre[i][j][1], ar[i], br[j]);
+                for (int j = 0; j < MT; j++) dmma(cre[i][j][0], cre[i][j][1], ar[i], br[j]);
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < MT; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) dmma(cim[i][j][0], cim[i][j][1], ar[i], bi[j]);
+                for (int j = 0; j < MT; j++) dmma(cim[i][j][0], cim[i][j][1], ar[i], bi[j]);
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < MT; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) dmma(cre[i][j][0], cre[i][j][1], aim[i], bi[j]);
+                for (int j = 0; j < MT; j++) dmma(cre[i][j][0], cre[i][j][1], aim[i], bi[j]);
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < MT; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) dmma(cim[i][j][0], cim[i][j][1], naim[i], br[j]);
+                for (int j = 0; j < MT; j++) dmma(cim[i][j][0], cim[i][j][1], naim[i], br[j]);
         }
     }
     cp_async_wait<0>();
     __syncthreads();
 
-    if (KIND == EPI_PLANAR) {
-        // split-precision path: column maxima of |B| (rows m of this tile),
-        // reduced over the 8 row groups of a warp, then one atomic per column
-        double *bmax = P.colmax;
-        if (bmax) {
+    if constexpr (C::KS > 1) {      // warps 1.. hand their sums to warp 0, which adds them in order
+        if (warp > 0) {
+            double *o = smem + (warp - 1) * 32 * MT * MT * 4 + lane;
 #pragma unroll
-            for (int j = 0; j < 4; j++)
+            for (int i = 0; i < MT; i++)
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    double mx = 0.0;
+                for (int j = 0; j < MT; j++)
 #pragma unroll
-                    for (int i = 0; i < 4; i++) mx = fmax(mx, fmax(fabs(cre[i][j][h]), fabs(cim[i][j][h])));
-                    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-                    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-                    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-                    const int n = n0 + wn * 32 + j * 8 + 2 * (lane & 3) + h;
-                    if (lane < 4 && n < P.N) atomic_max_nonneg(bmax + n, mx);
-                }
+                    for (int h = 0; h < 2; h++) {
+                        o[((i * MT + j) * 4 + h) * 32] = cre[i][j][h];
+                        o[((i * MT + j) * 4 + 2 + h) * 32] = cim[i][j][h];
+                    }
         }
+        __syncthreads();
+        if (warp == 0)
+            for (int w = 0; w < C::KS - 1; w++) {
+                const double *o = smem + w * 32 * MT * MT * 4 + lane;
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+                for (int i = 0; i < MT; i++)
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int m = m0 + wm * 32 + i * 8 + (lane >> 2);
-                const int n = n0 + wn * 32 + j * 8 + 2 * (lane & 3);
-                if (m >= P.M) continue;
-                if (n + 1 < P.N) {
-                    *reinterpret_cast<double2 *>(P.outr + (size_t)m * P.ldo + n) = make_double2(cre[i][j][0], cre[i][j][1]);
-                    *reinterpret_cast<double2 *>(P.outi + (size_t)m * P.ldo + n) = make_double2(cim[i][j][0], cim[i][j][1]);
-                } else if (n < P.N) {
-                    P.outr[(size_t)m * P.ldo + n] = cre[i][j][0];
-                    P.outi[(size_t)m * P.ldo + n] = cim[i][j][0];
-                }
+                    for (int j = 0; j < MT; j++)
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            cre[i][j][h] += o[((i * MT + j) * 4 + h) * 32];
+                            cim[i][j][h] += o[((i * MT + j) * 4 + 2 + h) * 32];
+                        }
             }
-        return;
+        __syncthreads();
     }
-    if (KIND == EPI_LOROWS) {
+    const bool out = C::KS == 1 || warp == 0;       // warps that hold results
+
+    if (GROUP == 0) {
+        if (!out) return;
+        if (P.kind == EPI_PLANAR) {
+            // split-precision path: column maxima of |B| (rows m of this tile),
+            // reduced over the 8 row groups of a warp, then one atomic per column
+            double *bmax = P.colmax;
+            if (bmax) {
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+                for (int j = 0; j < MT; j++)
 #pragma unroll
-            for (int j = 0; j < 4; j++)
+                    for (int h = 0; h < 2; h++) {
+                        double mx = 0.0;
+#pragma unroll
+                        for (int i = 0; i < MT; i++) mx = fmax(mx, fmax(fabs(cre[i][j][h]), fabs(cim[i][j][h])));
+                        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+                        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+                        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+                        const int n = n0 + nw + j * 8 + 2 * (lane & 3) + h;
+                        if (lane < 4 && n < P.N) atomic_max_nonneg(bmax + n, mx);
+                    }
+            }
+#pragma unroll
+            for (int i = 0; i < MT; i++)
+#pragma unroll
+                for (int j = 0; j < MT; j++) {
+                    const int m = m0 + mw + i * 8 + (lane >> 2);
+                    const int n = n0 + nw + j * 8 + 2 * (lane & 3);
+                    if (m >= P.M) continue;
+                    if (n + 1 < P.N) {
+                        *reinterpret_cast<double2 *>(P.outr + (size_t)m * P.ldo + n) = make_double2(cre[i][j][0], cre[i][j][1]);
+                        *reinterpret_cast<double2 *>(P.outi + (size_t)m * P.ldo + n) = make_double2(cim[i][j][0], cim[i][j][1]);
+                    } else if (n < P.N) {
+                        P.outr[(size_t)m * P.ldo + n] = cre[i][j][0];
+                        P.outi[(size_t)m * P.ldo + n] = cim[i][j][0];
+                    }
+                }
+            return;
+        }
+        // EPI_LOROWS
+#pragma unroll
+        for (int i = 0; i < MT; i++)
+#pragma unroll
+            for (int j = 0; j < MT; j++)
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    const int r = m0 + wm * 32 + i * 8 + (lane >> 2);
-                    const int g = n0 + wn * 32 + j * 8 + 2 * (lane & 3) + h;
+                    const int r = m0 + mw + i * 8 + (lane >> 2);
+                    const int g = n0 + nw + j * 8 + 2 * (lane & 3) + h;
                     if (r >= P.M || g >= P.N) continue;
                     exs_complex v; v.re = cre[i][j][h]; v.im = cim[i][j][h];
                     exs_complex vc; vc.re = v.re; vc.im = -v.im;
@@ -201,13 +261,13 @@ zgemm_dmma_kernel(DevParams p, const GemmProb *probs, const TileWork *work, cons
         return;
     }
     // EPI_HAM / EPI_OVL: APW-APW block, upper tiles, interstitial + mirror.
-    int *s_iv = reinterpret_cast<int *>(smem);                 // [128][3]
-    double *s_v = smem + 2 * 128;                              // [128][3] (after 1536 bytes)
+    int *s_iv = reinterpret_cast<int *>(smem);                 // [2 EDGE][3]
+    double *s_v = smem + 3 * EDGE;                             // [2 EDGE][3], after 24 EDGE bytes
     const KDesc kd = ks[P.kidx];
     {
-        const int t = threadIdx.x;                             // 0..63 rows, 64..127 cols
-        const int idx = (t < 64) ? (m0 + t) : (n0 + t - 64);
-        if (idx < kd.ngp) {
+        const int t = threadIdx.x;                             // rows, then columns
+        const int idx = (t < EDGE) ? (m0 + t) : (n0 + t - EDGE);
+        if (t < 2 * EDGE && idx < kd.ngp) {
             int g = kd.igpig[idx] - 1;
             if (g < 0 || g >= p.ngrtot) {      // caller's index table out of range
                 atomicOr(p.err, DEV_ERR_INDEX);
@@ -222,20 +282,22 @@ zgemm_dmma_kernel(DevParams p, const GemmProb *probs, const TileWork *work, cons
         }
     }
     __syncthreads();
+    if (!out || idle) return;
     const int ngp = kd.ngp;
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < MT; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++)
+        for (int j = 0; j < MT; j++)
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                const int li = wm * 32 + i * 8 + (lane >> 2);
-                const int lj = wn * 32 + j * 8 + 2 * (lane & 3) + h;
+                const int li = mw + i * 8 + (lane >> 2);
+                const int lj = nw + j * 8 + 2 * (lane & 3) + h;
                 const int gi = m0 + li, gj = n0 + lj;
                 if (gi >= ngp || gj >= ngp || gi > gj) continue;
                 double zr = cre[i][j][h], zi = cim[i][j][h];
                 double ar, ai;
-                if (interstitial(p, KIND, s_iv + 3 * li, s_iv + 3 * (64 + lj), s_v + 3 * li, s_v + 3 * (64 + lj), ar, ai)) {
+                if (interstitial(p, P.kind, s_iv + 3 * li, s_iv + 3 * (EDGE + lj), s_v + 3 * li, s_v + 3 * (EDGE + lj),
+                                 ar, ai)) {
                     zr += ar;
                     zi += ai;
                 }
@@ -249,104 +311,154 @@ zgemm_dmma_kernel(DevParams p, const GemmProb *probs, const TileWork *work, cons
 }
 
 // ---------------------------------------------------------------- host side
-template <int KIND>
-static cudaError_t launch_kind(const DevParams &p, const GemmProb *d_probs, const TileWork *d_work, int nwork,
+// Tile edge for a set of problems.  A tile's time is its area over the FP64
+// pipe of one SM, so a launch of n tiles takes edge^2 max(1, n / 148) units;
+// the smaller tiles re-read more of their operands (0.9 and 0.7 of the rate).
+// One k-point of the two-atom cell: H and O 156 us in two launches of 64-tiles
+// -> 18 us (16), h_a A and the lo rows 62 -> 8 us; APW-lo rows of 27 k-points
+// (27 rows) 926 -> 498 us (32); A C of the eight-atom adjoint 178 -> 124 us (32).
+int gemm_edge(const long long n[3])
+{
+    const int edge[3] = {64, 32, 16};
+    const double rate[3] = {1.0, 0.9, 0.7};
+    int best = 0;
+    double tb = 0.0;
+    for (int q = 0; q < 3; q++) {
+        const double t = (double)edge[q] * edge[q] * std::max(1.0, (double)n[q] / 148.0) / rate[q];
+        if (q == 0 || t < tb) {
+            tb = t;
+            best = q;
+        }
+    }
+    return edge[best];
+}
+
+static long long tile_count(const GemmProb &P, int edge)
+{
+    const long long tm = (P.M + edge - 1) / edge, tn = (P.N + edge - 1) / edge;
+    return (P.kind == EPI_HAM || P.kind == EPI_OVL) ? tm * (tm + 1) / 2 : tm * tn;
+}
+
+void gemm_tiles(const std::vector<GemmProb> &probs, int first, int last, int edge, std::vector<TileWork> &w)
+{
+    for (int i = first; i < last; i++) {
+        const GemmProb &P = probs[i];
+        const bool upper = P.kind == EPI_HAM || P.kind == EPI_OVL;
+        for (int tm = 0; tm < (P.M + edge - 1) / edge; tm++)
+            for (int tn = upper ? tm : 0; tn < (P.N + edge - 1) / edge; tn++) w.push_back({i, tm, tn});
+    }
+}
+
+int gemm_edge_of(const std::vector<GemmProb> &probs, int first, int last)
+{
+    long long n[3] = {0, 0, 0};
+    const int edge[3] = {64, 32, 16};
+    for (int q = 0; q < 3; q++)
+        for (int i = first; i < last; i++) n[q] += tile_count(probs[i], edge[q]);
+    return gemm_edge(n);
+}
+
+template <int GROUP, int EDGE>
+static cudaError_t launch_edge(const DevParams &p, const GemmProb *d_probs, const TileWork *d_work, int nwork,
                                const KDesc *d_k, cudaStream_t s)
 {
-    if (nwork <= 0) return cudaSuccess;
     static std::atomic<unsigned long long> attr{0};
     cudaError_t e = once_per_device(attr, [] {
-        return cudaFuncSetAttribute(zgemm_dmma_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GB_SMEM);
+        return cudaFuncSetAttribute(zgemm_dmma_kernel<GROUP, EDGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)GemmCfg<EDGE>::SMEM);
     });
     if (e != cudaSuccess) return e;
-    zgemm_dmma_kernel<KIND><<<(unsigned)nwork, GB_THREADS, GB_SMEM, s>>>(p, d_probs, d_work, d_k);
+    zgemm_dmma_kernel<GROUP, EDGE><<<(unsigned)nwork, GB_THREADS, GemmCfg<EDGE>::SMEM, s>>>(p, d_probs, d_work, d_k);
     return cudaGetLastError();
 }
 
-// Problem and tile tables of the three GEMM stages of one batched call.
+template <int GROUP>
+static cudaError_t launch_group(int edge, const DevParams &p, const GemmProb *d_probs, const TileWork *d_work,
+                                int nwork, const KDesc *d_k, cudaStream_t s)
+{
+    if (nwork <= 0) return cudaSuccess;
+    if (edge == 16) return launch_edge<GROUP, 16>(p, d_probs, d_work, nwork, d_k, s);
+    if (edge == 32) return launch_edge<GROUP, 32>(p, d_probs, d_work, nwork, d_k, s);
+    return launch_edge<GROUP, 64>(p, d_probs, d_work, nwork, d_k, s);
+}
+
+// Problem and tile tables of the GEMM launches of one batched call: work[0]
+// h_a A and work[1] the APW-lo rows of H (in work[0] too when they take the
+// same tile edge), work[2] H and O.
 void build_gemm_tables(const exs_ctx *c, const std::vector<KDesc> &ks, GemmTables &t)
 {
-    for (int q = 0; q < 4; q++) { t.probs[q].clear(); t.work[q].clear(); }
-    for (size_t k = 0; k < ks.size(); k++) {
-        const int ncols = std::min(c->npad, (ks[k].ngp + GB_N - 1) / GB_N * GB_N);
-        for (int ias = 0; ias < c->natmtot; ias++) {
-            const AtomDesc &a = c->atoms[ias];
-            // stage 1: B_a = h_a A_a  (planar output, all padded columns)
-            {
+    t.probs.clear();
+    for (auto &w : t.work) w.clear();
+    for (int kind : {EPI_PLANAR, EPI_LOROWS})
+        for (size_t k = 0; k < ks.size(); k++) {
+            const int ncols = std::min(c->npad, (ks[k].ngp + 63) / 64 * 64);
+            for (int ias = 0; ias < c->natmtot; ias++) {
+                const AtomDesc &a = c->atoms[ias];
                 GemmProb P{};
-                P.xr = c->d_haa_r + (size_t)ias * c->ldh * c->ldh;
-                P.xi = c->d_haa_i + (size_t)ias * c->ldh * c->ldh;
-                P.ldx = c->ldh;
+                P.kind = (short)kind;
                 P.yr = ks[k].ar + (size_t)a.apw_off * c->npad;
                 P.yi = ks[k].ai + (size_t)a.apw_off * c->npad;
                 P.ldy = c->npad;
-                P.M = a.napw; P.N = ncols; P.K = a.napw;
+                P.K = a.napw;
                 P.conjx = 0;
-                P.outr = ks[k].br + (size_t)a.apw_off * c->npad;
-                P.outi = ks[k].bi + (size_t)a.apw_off * c->npad;
-                P.ldo = c->npad;
                 P.kidx = (int)k;
-                P.colmax = ks[k].oz_scale ? ks[k].oz_scale + c->npad : nullptr;
-                const int pi = (int)t.probs[EPI_PLANAR].size();
-                t.probs[EPI_PLANAR].push_back(P);
-                for (int tm = 0; tm < (P.M + GB_M - 1) / GB_M; tm++)
-                    for (int tn = 0; tn < (P.N + GB_N - 1) / GB_N; tn++) t.work[EPI_PLANAR].push_back({pi, tm, tn});
+                if (kind == EPI_PLANAR) {      // B_a = h_a A_a (planar output, all padded columns)
+                    P.xr = c->d_haa_r + (size_t)ias * c->ldh * c->ldh;
+                    P.xi = c->d_haa_i + (size_t)ias * c->ldh * c->ldh;
+                    P.ldx = c->ldh;
+                    P.M = a.napw;
+                    P.N = ncols;
+                    P.outr = ks[k].br + (size_t)a.apw_off * c->npad;
+                    P.outi = ks[k].bi + (size_t)a.apw_off * c->npad;
+                    P.ldo = c->npad;
+                    P.colmax = ks[k].oz_scale && !ks[k].oz_part ? ks[k].oz_scale + c->npad : nullptr;
+                } else {                       // APW-lo rows of H
+                    if (a.losize == 0) continue;
+                    P.xr = c->d_loa_r + (size_t)ias * c->ldlo * c->maxaa;
+                    P.xi = c->d_loa_i + (size_t)ias * c->ldlo * c->maxaa;
+                    P.ldx = c->ldlo;
+                    P.M = a.losize;
+                    P.N = ks[k].ngp;
+                    P.z = ks[k].h;
+                    P.ldz = ks[k].nmat;
+                    P.row0 = ks[k].ngp + a.lo_off;
+                }
+                t.probs.push_back(P);
             }
-            // stage 3: APW-lo rows of H
-            if (a.losize > 0) {
-                GemmProb P{};
-                P.xr = c->d_loa_r + (size_t)ias * c->ldlo * c->maxaa;
-                P.xi = c->d_loa_i + (size_t)ias * c->ldlo * c->maxaa;
-                P.ldx = c->ldlo;
-                P.yr = ks[k].ar + (size_t)a.apw_off * c->npad;
-                P.yi = ks[k].ai + (size_t)a.apw_off * c->npad;
-                P.ldy = c->npad;
-                P.M = a.losize; P.N = ks[k].ngp; P.K = a.napw;
-                P.conjx = 0;
-                P.z = ks[k].h;
-                P.ldz = ks[k].nmat;
-                P.row0 = ks[k].ngp + a.lo_off;
-                P.kidx = (int)k;
-                const int pi = (int)t.probs[EPI_LOROWS].size();
-                t.probs[EPI_LOROWS].push_back(P);
-                for (int tm = 0; tm < (P.M + GB_M - 1) / GB_M; tm++)
-                    for (int tn = 0; tn < (P.N + GB_N - 1) / GB_N; tn++) t.work[EPI_LOROWS].push_back({pi, tm, tn});
-            }
+            if (kind == EPI_PLANAR && k + 1 == ks.size()) t.first_lo = (int)t.probs.size();
         }
-        // stage 2: H = A^H B and O = A^H A (A^H C for iora*), upper tiles
-        for (int which = 0; which < 2; which++) {
-            const int kind = which == 0 ? EPI_HAM : EPI_OVL;
+    t.first_ho = (int)t.probs.size();
+    // H = A^H B and O = A^H A (A^H C for iora*), upper tiles
+    for (size_t k = 0; k < ks.size(); k++)
+        for (int kind : {EPI_HAM, EPI_OVL}) {
             GemmProb P{};
+            P.kind = (short)kind;
             P.xr = ks[k].ar; P.xi = ks[k].ai; P.ldx = c->npad;
-            if (which == 0) { P.yr = ks[k].br; P.yi = ks[k].bi; }
+            if (kind == EPI_HAM) { P.yr = ks[k].br; P.yi = ks[k].bi; }
             else { P.yr = ks[k].cr; P.yi = ks[k].ci; }
             P.ldy = c->npad;
             P.M = P.N = ks[k].ngp;
             P.K = c->K;
             P.conjx = 1;
-            P.z = which == 0 ? ks[k].h : ks[k].o;
+            P.z = kind == EPI_HAM ? ks[k].h : ks[k].o;
             P.ldz = ks[k].nmat;
             P.kidx = (int)k;
-            const int pi = (int)t.probs[kind].size();
-            t.probs[kind].push_back(P);
-            const int nt = (P.M + GB_M - 1) / GB_M;
-            for (int tm = 0; tm < nt; tm++)
-                for (int tn = tm; tn < nt; tn++) t.work[kind].push_back({pi, tm, tn});
+            t.probs.push_back(P);
         }
-    }
+    t.edge[0] = gemm_edge_of(t.probs, 0, t.first_lo);
+    t.edge[1] = gemm_edge_of(t.probs, t.first_lo, t.first_ho);
+    t.edge[2] = gemm_edge_of(t.probs, t.first_ho, (int)t.probs.size());
+    gemm_tiles(t.probs, 0, t.first_lo, t.edge[0], t.work[0]);
+    gemm_tiles(t.probs, t.first_lo, t.first_ho, t.edge[1], t.work[t.edge[1] == t.edge[0] ? 0 : 1]);
+    gemm_tiles(t.probs, t.first_ho, (int)t.probs.size(), t.edge[2], t.work[2]);
 }
 
-cudaError_t launch_gemm_kind(int kind, const DevParams &p, const void *d_probs, const void *d_work, int nwork,
-                             const KDesc *d_k, cudaStream_t s)
+cudaError_t launch_gemm(int group, int edge, const DevParams &p, const void *d_probs, const void *d_work, int nwork,
+                        const KDesc *d_k, cudaStream_t s)
 {
     const GemmProb *P = (const GemmProb *)d_probs;
     const TileWork *W = (const TileWork *)d_work;
-    switch (kind) {
-    case EPI_PLANAR: return launch_kind<EPI_PLANAR>(p, P, W, nwork, d_k, s);
-    case EPI_HAM: return launch_kind<EPI_HAM>(p, P, W, nwork, d_k, s);
-    case EPI_OVL: return launch_kind<EPI_OVL>(p, P, W, nwork, d_k, s);
-    default: return launch_kind<EPI_LOROWS>(p, P, W, nwork, d_k, s);
-    }
+    return group == 0 ? launch_group<0>(edge, p, P, W, nwork, d_k, s) : launch_group<1>(edge, p, P, W, nwork, d_k, s);
 }
 
 // ------------------------------------------- lo blocks that need no product
