@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(256) oz_ring_x_kernel(DevParams p, OzAtomArgs 
 //            atom (N = nb, a multiple of 32), over the atom's K window
 // The work list is flat in (tile, plane): while full rounds of one tile per
 // cluster last, a cluster takes a tile and walks its 2n planes; the (tile,
-// plane) pairs of the remaining tiles are dealt out in equal runs, so that a
+// plane) pairs of the remaining tiles are dealt out in equal shares, so that a
 // handful of tiles (two for a k-point of the two-atom cell) still occupies
 // every SM pair and the last round is never short of more than one product.
 // Two accumulators in tensor memory.  RG_HO, RG_ATOM: products take them in
@@ -404,30 +404,45 @@ __device__ __forceinline__ void tma_load_4d_2sm(uint32_t dst, const CUtensorMap 
 }
 
 // The flat work list of cluster c, walked by every role: np products of each
-// of its full-round tiles, then its run of the (tile, plane) pairs of the
-// remaining tiles.
+// of its full-round tiles, then its share of the (tile, plane) pairs of the
+// remaining tiles: by planes (H/O), so that the clusters work on the same plane
+// of all these tiles at a time and share its operands in the L2 (dealt out in
+// runs, every cluster on another plane, they read 17 TB/s from HBM: three
+// k-points of 16 atoms REST), or in one run of planes per cluster (per-atom
+// tiles, which share little and whose producers then look a tile up once).
+template <bool RUNS>
 struct RingUnits {
-    int ncl, np, count, tile, P, full_end, rest_tile, rest_P;
+    int ncl, np, count, tile, P, full_end, rest, rest_tile, rest_P;
     __device__ RingUnits(int ntiles, int ncl_, int np_, int c) : ncl(ncl_), np(np_)
     {
         const int full = ntiles / ncl;
-        const long long pairs = (long long)(ntiles - full * ncl) * np;
-        const int first = (int)(pairs * c / ncl);
-        count = full * np + (int)(pairs * (c + 1) / ncl) - first;
         full_end = full * ncl;
-        rest_tile = full_end + first / np;
-        rest_P = first % np;
+        rest = ntiles - full_end;
+        const int pairs = rest * np;                       // rest < ncl
+        const int first = RUNS ? (int)((long long)pairs * c / ncl) : c;
+        const int mine = RUNS ? (int)((long long)pairs * (c + 1) / ncl) - first : (pairs - c + ncl - 1) / ncl;
+        count = full * np + mine;
+        rest_tile = full_end + (RUNS ? first / np : first % max(rest, 1));
+        rest_P = RUNS ? first % np : first / max(rest, 1);
         tile = full > 0 ? c : rest_tile;
         P = full > 0 ? 0 : rest_P;
     }
     __device__ void next()
     {
-        if (++P < np) return;
-        P = 0;
-        if (tile >= full_end) {          // in the run of the remaining tiles
-            tile++;
+        if (tile >= full_end) {                            // among the remaining tiles
+            if (RUNS) {
+                if (++P < np) return;
+                P = 0;
+                tile++;
+            } else {
+                const int v = tile - full_end + ncl;       // ncl pairs on
+                P += v / rest;
+                tile = full_end + v % rest;
+            }
             return;
         }
+        if (++P < np) return;
+        P = 0;
         tile += ncl;
         if (tile >= full_end) {
             tile = rest_tile;
@@ -477,7 +492,7 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     const uint32_t rank = cluster_ctarank();
     const uint32_t sbase = (smem_u32(rg_smem) + 1023u) & ~1023u;
     const int cl = (int)(blockIdx.x >> 1), NP = 2 * rg.n;
-    RingUnits units(ntiles, (int)(gridDim.x >> 1), NP, cl);
+    RingUnits<MODE == RG_ATOM> units(ntiles, (int)(gridDim.x >> 1), NP, cl);
     const int N = MODE == RG_ATOM ? xa.nb : 256;         // MMA N
     const int b_rows = N / 2;                            // operand rows of a B operand in this CTA
 

@@ -149,28 +149,34 @@ def test_products_recombine(n):
                 assert err <= (bound / 2 ** (32 - sh) + 1) * M
 
 
+@pytest.mark.parametrize("runs", [False, True])
 @pytest.mark.parametrize("ntiles,ncl,planes", [(1, 28, 28), (2, 56, 28), (3, 74, 28), (74, 74, 28), (75, 74, 28),
                                                (147, 74, 30), (540, 74, 28)])
-def test_work_list_covers_every_product_once(ntiles, ncl, planes):
+def test_work_list_covers_every_product_once(ntiles, ncl, planes, runs):
     full = ntiles // ncl
-    pairs, full_end = (ntiles - full * ncl) * planes, full * ncl
+    full_end = full * ncl
+    rest = ntiles - full_end
+    pairs = rest * planes
     seen, most, least = set(), 0, 1 << 30
     for c in range(ncl):
-        first = pairs * c // ncl
-        count = full * planes + pairs * (c + 1) // ncl - first
+        first = pairs * c // ncl if runs else c
+        mine = pairs * (c + 1) // ncl - first if runs else (pairs - c + ncl - 1) // ncl
+        count = full * planes + mine
         most, least = max(most, count), min(least, count)
-        rest = (full_end + first // planes, first % planes)
-        tile, P = (c, 0) if full else rest
+        start = (full_end + first // planes, first % planes) if runs else (full_end + first % max(rest, 1),
+                                                                           first // max(rest, 1))
+        tile, P = (c, 0) if full else start
         for _ in range(count):
-            assert (tile, P) not in seen and tile < ntiles
+            assert (tile, P) not in seen and tile < ntiles and P < planes
             seen.add((tile, P))
-            P += 1
-            if P == planes:
-                P = 0
-                if tile >= full_end:
-                    tile += 1
+            if tile >= full_end:
+                if runs:
+                    tile, P = (tile, P + 1) if P + 1 < planes else (tile + 1, 0)
                 else:
-                    tile += ncl
-                    if tile >= full_end:
-                        tile, P = rest
+                    v = tile - full_end + ncl
+                    tile, P = full_end + v % rest, P + v // rest
+            else:
+                tile, P = (tile, P + 1) if P + 1 < planes else (tile + ncl, 0)
+                if tile >= full_end:
+                    tile, P = start
     assert len(seen) == ntiles * planes and most - least <= 1
