@@ -425,6 +425,7 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
     exs::ring_row_blocks(rows, &c->ring_nb, &c->ring_nrows);
     const size_t xgroups = (size_t)c->natmtot * (mod ? 2 * ring.n : slices * c->oz_nxb);
     const size_t xs_bytes = xgroups * (mod ? c->ring_nrows : 128) * c->oz_lw;
+    c->ozpart_rows = exs::ring_part_rows(c->natmtot, c->ring_nrows);
     const size_t nxsig = (size_t)c->natmtot * (mod ? c->ring_nrows : c->oz_nxb * 64);
     // moduli: the residues of the H/O products of a whole batch (the upper tiles of ngkmax G+k per
     // k-point); the per-atom products run before them in the same buffer, in chunks that fit it, of at
@@ -449,7 +450,7 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
     }
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_ozscale, sizeof(double) * 3 * c->npad * c->max_batch);
     if (e == cudaSuccess && mod)
-        e = cudaMalloc((void **)&c->d_ozpart, sizeof(double) * c->natmtot * c->npad * c->max_batch);
+        e = cudaMalloc((void **)&c->d_ozpart, sizeof(double) * c->ozpart_rows * c->npad * c->max_batch);
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_xs, xs_bytes);
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_xsig, sizeof(double) * nxsig);
     if (e != cudaSuccess || c->oz_xseg < 1) {
@@ -484,6 +485,7 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
     c->oz_sch = sch;
     c->oz_ring = ring;
     c->prec_mode = mode;
+    c->x_valid = false;
     if (c->have_inputs) {   // slices of the current h_a and loa
         EXS_CUDA(exs::launch_x(c, c->stream));
         EXS_CUDA(cudaStreamSynchronize(c->stream));
@@ -576,7 +578,8 @@ int exs_set_scf_inputs(exs_ctx *c, const exs_scf_inputs *in)
     // the matching systems D_l depend only on the tails: factorised once here
     if (!c->d_dlu) EXS_CUDA(dalloc(&c->d_dlu, (size_t)nat * (c->lmaxapw + 1) * exs::DLU_STRIDE));
     EXS_CUDA(exs::launch_match_dlu(c->params(), c->d_dlu, s));
-    if (c->oz_on())   // slices of the new h_a and loa, in place
+    if (!keep_mt) c->x_valid = false;
+    if (c->oz_on() && !c->x_valid)   // slices of the new h_a and loa, in place
         EXS_CUDA(exs::launch_x(c, s));
     EXS_CUDA(cudaStreamSynchronize(s));
     c->have_inputs = true;
@@ -887,12 +890,16 @@ int enqueue_setup(exs_ctx *c, const std::vector<KDesc> &ks, const Uploaded &u, b
     EXS_EV(1);
     const bool oz = c->oz_on(), mod = oz && c->oz_sch.mod;
     const int nk = (int)ks.size();
+    // configuration bit 4: B = h_a A and the APW-lo rows in native FP64 even
+    // when the H/O contraction is split
+    const bool b64 = !oz || (c->oz_cfg & 16);
     // column bounds (2-norms with moduli; with slices the producers raised the maxima, but for C), then the
     // slices or residues of operand `which`: 0 A, 1 B, 2 C
     auto split = [&](int which) -> cudaError_t {
         cudaError_t e = cudaSuccess;
         if (mod) {
-            e = exs::launch_oz_norm(p, u.d_k, nk, which, s);
+            const int per = which == 0 ? 1 : (which == 1 && !b64 ? c->ring_nrows / 16 : 0);
+            e = exs::launch_oz_norm(p, u.d_k, nk, which, per, s);
             return e != cudaSuccess ? e : exs::launch_ring_split(p, u.d_k, nk, c->oz_ring, c->kp8, which, s);
         }
         if (which == 2) e = exs::launch_oz_colmax(p, u.d_k, nk, s);
@@ -900,9 +907,6 @@ int enqueue_setup(exs_ctx *c, const std::vector<KDesc> &ks, const Uploaded &u, b
     };
     // C = (I + h1aa) A, the right operand of O
     if (oz && c->relativity == EXS_REL_IORA) EXS_CUDA(split(2));
-    // configuration bit 4: B = h_a A and the APW-lo rows in native FP64 even
-    // when the H/O contraction is split
-    const bool b64 = !oz || (c->oz_cfg & 16);
     if (oz) {
         // A; B = h_a A and the APW-lo rows of H from the split h_a and loa
         EXS_CUDA(split(0));
@@ -934,8 +938,7 @@ int enqueue_setup(exs_ctx *c, const std::vector<KDesc> &ks, const Uploaded &u, b
         EXS_CUDA(gemm(1, 2));
     }
     EXS_EV(3);
-    EXS_CUDA(exs::launch_olp_apwlo(p, u.d_k, (int)ks.size(), ngp_max, s));
-    EXS_CUDA(exs::launch_lolo_blocks(p, u.d_k, (int)ks.size(), s));
+    EXS_CUDA(exs::launch_lo_blocks(p, u.d_k, nk, ngp_max, s));
     EXS_EV(4);
 #undef EXS_EV
     if (timed) c->timed = true;
@@ -975,7 +978,7 @@ KDesc slot_desc(exs_ctx *c, int slot, int ngp, const int *d_igpig, const double 
     k.oz_slices = c->d_oz ? c->d_oz + (size_t)slot * c->oz_slot_bytes : nullptr;
     const bool oz = c->oz_on() && c->d_ozscale;
     k.oz_scale = oz ? c->d_ozscale + (size_t)slot * 3 * c->npad : nullptr;
-    k.oz_part = oz && c->oz_sch.mod ? c->d_ozpart + (size_t)slot * c->natmtot * c->npad : nullptr;
+    k.oz_part = oz && c->oz_sch.mod ? c->d_ozpart + (size_t)slot * c->ozpart_rows * c->npad : nullptr;
     k.oz_slot = slot;
     return k;
 }

@@ -136,7 +136,8 @@ struct KDesc {
     int8_t *oz_slices;       // split-precision path: int8 slices of this slot [S][4 arrays][npad][kp8]
     double *oz_scale;        // split-precision path: column bounds of A and B [2][npad] (maxima with slices,
                              // 2-norms with moduli; the scale is the power of two above; null: FP64 path)
-    double *oz_part;         // moduli: sums of squares of the A columns per atom [natmtot][npad], else null
+    double *oz_part;         // moduli: sums of squares of the A columns per atom, then of the B columns per 16
+                             // rows of an atom [rows][npad]; else null
     int oz_slot;             // split-precision path: slot index in the slice tensor maps
 };
 
@@ -318,7 +319,9 @@ struct exs_ctx {
     int oz_seg = 0;              // slice pairs per exact int32 segment
     int8_t *d_oz = nullptr;      // int8 slices of all slots
     double *d_ozscale = nullptr; // column scales of all slots
-    double *d_ozpart = nullptr;  // moduli: sums of squares of the A columns per atom, all slots
+    double *d_ozpart = nullptr;  // moduli: partial sums of squares of the A and B columns, all slots
+    size_t ozpart_rows = 0;      // rows of npad per slot
+    bool x_valid = false;        // d_xs holds the split of the current h_a and loa
     size_t oz_slot_bytes = 0;
     CUtensorMap oz_mapA[exs::OZ_NCFG], oz_mapB[exs::OZ_NCFG];   // TMA views of d_oz per pipeline configuration
     CUtensorMap oz_mapB2[exs::OZ_NCFG];                            // half-B views (two-SM tiles)
@@ -365,8 +368,7 @@ cudaError_t launch_match_ref(const DevParams &p, int ngp, const double *gpc, con
 cudaError_t launch_apwalm_to_planes(const DevParams &p, int ngp, const exs_complex *apwalm, double *ar,
                                     double *ai, double *amax, double *part, cudaStream_t s);
 cudaError_t launch_iora_planes(const DevParams &p, const KDesc *d_k, int nk, int ngp_max, cudaStream_t s);
-cudaError_t launch_lolo_blocks(const DevParams &p, const KDesc *d_k, int nk, cudaStream_t s);
-cudaError_t launch_olp_apwlo(const DevParams &p, const KDesc *d_k, int nk, int ngp_max, cudaStream_t s);
+cudaError_t launch_lo_blocks(const DevParams &p, const KDesc *d_k, int nk, int ngp_max, cudaStream_t s);
 // Grouped FP64 GEMM stages (setup_f64.cu)
 void build_gemm_tables(const exs_ctx *c, const std::vector<KDesc> &ks, GemmTables &t);
 int gemm_edge_of(const std::vector<GemmProb> &probs, int first, int last);
@@ -417,7 +419,8 @@ size_t ring_pace_bytes();
 void ring_row_blocks(int rows, int *nb, int *nrows);
 bool make_ring_maps(void *base, size_t nsp, int npad, int kp8, int narr, void *xbase, size_t xgroups, int nrows,
                     int nb, int lw, CUtensorMap *ho1, CUtensorMap *ho2, CUtensorMap *arow, CUtensorMap *x);
-cudaError_t launch_oz_norm(const DevParams &p, const KDesc *d_k, int nk, int which, cudaStream_t s);
+size_t ring_part_rows(int natmtot, int nrows);
+cudaError_t launch_oz_norm(const DevParams &p, const KDesc *d_k, int nk, int which, int per, cudaStream_t s);
 cudaError_t launch_ring_split(const DevParams &p, const KDesc *d_k, int nk, const OzRing &rg, int kp8, int which,
                               cudaStream_t s);
 cudaError_t launch_ring_x(const DevParams &p, const OzAtomArgs &xa, const OzRing &rg, cudaStream_t s);
@@ -428,8 +431,9 @@ cudaError_t launch_ring_atom(const CUtensorMap *mapA, const CUtensorMap *mapX, c
                              const void *d_tiles, int ntiles, const OzRing &rg, const OzAtomArgs &xa, uint8_t *res,
                              size_t res_bytes, cudaStream_t s);
 // Operands of h_a and loa for the active split arithmetic.
-inline cudaError_t launch_x(const exs_ctx *c, cudaStream_t s)
+inline cudaError_t launch_x(exs_ctx *c, cudaStream_t s)
 {
+    c->x_valid = true;
     return c->oz_sch.mod ? launch_ring_x(c->params(), c->oz_atom_args(), c->oz_ring, s)
                          : launch_oz_x(c->params(), c->oz_atom_args(), c->oz_sch, s);
 }

@@ -92,35 +92,66 @@ __device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b, uint32_t c, ui
     return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
 }
 
+// The residue bytes of E (8 or 16) elements to os (x + i_m y) and od (x - i_m y).
+template <int E>
+__device__ __forceinline__ void ring_emit(const OzRing &rg, int m, const uint2 (&x)[E], const uint2 (&y)[E], int8_t *os,
+                                          int8_t *od)
+{
+    uint32_t ws[E / 4], wd[E / 4];
+#pragma unroll
+    for (int q = 0; q < E / 4; q++) {
+        uint32_t s[4], d[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) ring_pair(rg, m, x[4 * q + e], y[4 * q + e], s[e], d[e]);
+        ws[q] = pack4(s[0], s[1], s[2], s[3]);
+        wd[q] = pack4(d[0], d[1], d[2], d[3]);
+    }
+    if constexpr (E == 16) {
+        *reinterpret_cast<uint4 *>(os) = make_uint4(ws[0], ws[1], ws[2], ws[3]);
+        *reinterpret_cast<uint4 *>(od) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
+    } else {
+        *reinterpret_cast<uint2 *>(os) = make_uint2(ws[0], ws[1]);
+        *reinterpret_cast<uint2 *>(od) = make_uint2(wd[0], wd[1]);
+    }
+}
+
 __device__ __forceinline__ uint2 ring_digits(double x, double sc)
 {
     const unsigned long long u = (unsigned long long)(__double2ll_rn(x * sc) + (1ll << 55));
     return make_uint2((uint32_t)u, (uint32_t)(u >> 32));
 }
 
-// Column 2-norms of the B or C planes (which = 1, 2) into oz_scale
-// block `which`.  One column per thread column of a 32 x 32 block, the rows
-// of threads covering interleaved rows f (stride 32), the partial sums
-// combined in a fixed order, so that the scales, and every result, are the
-// same from run to run.  The factor 1 + 2^-30 covers the rounding of a sum of
-// squares.  HBM bound (one read of the planes); 32 row threads instead of
-// eight keep enough loads in flight when few columns are left per SM: 64
-// atoms (254 blocks) 555 -> 201 us, 8 k-points of the two-atom cell 21 -> 7 us.
-__global__ void __launch_bounds__(1024) oz_norm_kernel(DevParams p, const KDesc *ks, int which)
+// Column 2-norms of one operand (which = 0: A, 1: B, 2: C) into its oz_scale
+// block.  One column per thread column of a 32 x 32 block, the rows of threads
+// covering interleaved rows (stride 32), the partial sums combined in a fixed
+// order, so that the scales, and every result, are the same from run to run.
+// The factor 1 + 2^-30 covers the rounding of a sum of squares.
+// PARTS: the rows are the sums of squares that the operand's producer left in
+// oz_part (A: one per atom; B: one per 16 rows of an atom, `per` of them);
+// else the planes themselves are read again (C, and B when it comes from the
+// FP64 products): 64 atoms 201 us, from the parts 7 and 16 us.
+template <bool PARTS>
+__global__ void __launch_bounds__(1024) oz_norm_kernel(DevParams p, const KDesc *ks, int which, int per)
 {
     __shared__ double part[32][33];
     const KDesc k = ks[blockIdx.y];
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int g = blockIdx.x * 32 + tx;
-    const double *pr, *pi;
-    oz_operand(k, which, pr, pi);
     double s = 0.0;
     if (g < k.ngp) {
+        if (PARTS) {
 #pragma unroll 4
-        for (int f = ty; f < p.K; f += 32) {
-            const size_t i = (size_t)f * p.npad + g;
-            const double xr = pr[i], xi = pi[i];
-            s = fma(xr, xr, fma(xi, xi, s));
+            for (int r = ty; r < p.natmtot * per; r += 32)
+                if (per == 1 || r % per * 16 < p.atoms[r / per].napw) s += k.oz_part[(size_t)r * p.npad + g];
+        } else {
+            const double *pr, *pi;
+            oz_operand(k, which, pr, pi);
+#pragma unroll 4
+            for (int f = ty; f < p.K; f += 32) {
+                const size_t i = (size_t)f * p.npad + g;
+                const double xr = pr[i], xi = pi[i];
+                s = fma(xr, xr, fma(xi, xi, s));
+            }
         }
     }
     part[ty][tx] = s;
@@ -133,30 +164,23 @@ __global__ void __launch_bounds__(1024) oz_norm_kernel(DevParams p, const KDesc 
     if (tx == 0 && gc < p.npad) k.oz_scale[(size_t)which * p.npad + gc] = sqrt(t) * (1.0 + 0x1p-30);
 }
 
-// The same for A from the sums of squares that its producer left per atom,
-// added in the order of the atoms.
-__global__ void __launch_bounds__(64) oz_norm_parts_kernel(DevParams p, const KDesc *ks)
-{
-    const KDesc k = ks[blockIdx.y];
-    const int g = blockIdx.x * 64 + threadIdx.x;
-    double t = 0.0;
-#pragma unroll 8
-    for (int a = 0; a < p.natmtot; a++) t += k.oz_part[(size_t)a * p.npad + g];
-    k.oz_scale[g] = sqrt(t) * (1.0 + 0x1p-30);
-}
-
 // The 2n residue planes of one operand (which = 0: A, 1: B, 2: C).  A
 // 128(f) x 32(G) tile per block, transposed through shared memory: reads
 // G-contiguous planes (a warp reads 32 consecutive G), writes K-contiguous
 // int8 rows 16 bytes per thread (8 threads cover a whole 128-byte line of one
 // G row).  The padding of two doubles per 16 rows of the tile spreads the
-// transposed reads over the banks.
-constexpr int RS_F = 128;
-constexpr int RS_LD = RS_F * 33 + 2 * (RS_F / 16);
-__device__ __forceinline__ int rs_at(int f, int g) { return f * 33 + 2 * (f >> 4) + g; }
+// transposed reads over the banks.  Bound by HBM and the residue arithmetic
+// (14 moduli: about 230 instructions per complex element): 27 k-points of the
+// eight-atom cell 0.55 ms, 0.40 of it without the arithmetic; eight elements per
+// thread and twice the warps: 0.74 ms.
+constexpr int RS_F = 128, RS_E = 16;             // tile rows f; elements per thread
+constexpr int RS_THREADS = 32 * RS_F / RS_E;
+constexpr int RS_LD = RS_F * 33 + 2 * (RS_F / RS_E);
+__device__ __forceinline__ int rs_at(int f, int g) { return f * 33 + 2 * (f / RS_E) + g; }
 
-__global__ void __launch_bounds__(256, 2) oz_ring_split_kernel(DevParams p, const KDesc *ks,
-                                                               const __grid_constant__ OzRing rg, int kp8, int which)
+__global__ void __launch_bounds__(RS_THREADS, 2) oz_ring_split_kernel(DevParams p, const KDesc *ks,
+                                                                      const __grid_constant__ OzRing rg, int kp8,
+                                                                      int which)
 {
     extern __shared__ __align__(16) double rs_t[];       // [re, im][RS_LD]
     const KDesc k = ks[blockIdx.z];
@@ -166,52 +190,41 @@ __global__ void __launch_bounds__(256, 2) oz_ring_split_kernel(DevParams p, cons
     const double *pr, *pi;
     oz_operand(k, which, pr, pi);
     {
+        constexpr int R = RS_THREADS / 32, NQ = RS_F / R;
         const int g = g0 + tx;
-        double vr[RS_F / 8], vi[RS_F / 8];
+        double vr[NQ], vi[NQ];
 #pragma unroll
-        for (int q = 0; q < RS_F / 8; q++) {
-            const int f = f0 + ty + 8 * q;
+        for (int q = 0; q < NQ; q++) {
+            const int f = f0 + ty + R * q;
             const bool v = f < p.K && g < k.ngp;
             const size_t i = (size_t)f * p.npad + g;
             vr[q] = v ? pr[i] : 0.0;
             vi[q] = v ? pi[i] : 0.0;
         }
 #pragma unroll
-        for (int q = 0; q < RS_F / 8; q++) {
-            rs_t[rs_at(ty + 8 * q, tx)] = vr[q];
-            rs_t[RS_LD + rs_at(ty + 8 * q, tx)] = vi[q];
+        for (int q = 0; q < NQ; q++) {
+            rs_t[rs_at(ty + R * q, tx)] = vr[q];
+            rs_t[RS_LD + rs_at(ty + R * q, tx)] = vi[q];
         }
     }
     __syncthreads();
-    const int gl = threadIdx.x >> 3, fl = (threadIdx.x & 7) * 16;
+    const int gl = threadIdx.x / (RS_F / RS_E), fl = threadIdx.x % (RS_F / RS_E) * RS_E;
     const int g = g0 + gl, f = f0 + fl;
-    if (g >= p.npad) return;
     // 1/sigma is a power of two: the scaling is exact
     const double sc = ldexp(1.0 / oz_sigma(k.oz_scale[(size_t)which * p.npad + g]), rg.b);
-    uint2 x[16], y[16];
+    uint2 x[RS_E], y[RS_E];
 #pragma unroll
-    for (int e = 0; e < 16; e++) {
+    for (int e = 0; e < RS_E; e++) {
         x[e] = ring_digits(rs_t[rs_at(fl + e, gl)], sc);
         y[e] = ring_digits(rs_t[RS_LD + rs_at(fl + e, gl)], sc);
     }
     const int narr = ring_narr(p.relativity), arr = which == 0 ? 1 : (which == 1 ? 0 : 2);
     const size_t plane = (size_t)narr * p.npad * kp8;
-    int8_t *out = k.oz_slices + ((size_t)arr * p.npad + g) * kp8 + f;
+    // plane 2m: A-, B+, C+; plane 2m + 1: A+, B-, C-
+    int8_t *os = k.oz_slices + ((size_t)arr * p.npad + g) * kp8 + f + (which == 0 ? plane : 0);
+    int8_t *od = k.oz_slices + ((size_t)arr * p.npad + g) * kp8 + f + (which == 0 ? 0 : plane);
 #pragma unroll 1
-    for (int m = 0; m < rg.n; m++, out += 2 * plane) {
-        uint32_t ws[4], wd[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            uint32_t s[4], d[4];
-#pragma unroll
-            for (int e = 0; e < 4; e++) ring_pair(rg, m, x[4 * q + e], y[4 * q + e], s[e], d[e]);
-            ws[q] = pack4(s[0], s[1], s[2], s[3]);
-            wd[q] = pack4(d[0], d[1], d[2], d[3]);
-        }
-        // plane 2m: A-, B+, C+; plane 2m + 1: A+, B-, C-
-        *reinterpret_cast<uint4 *>(out + (which == 0 ? plane : 0)) = make_uint4(ws[0], ws[1], ws[2], ws[3]);
-        *reinterpret_cast<uint4 *>(out + (which == 0 ? 0 : plane)) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
-    }
+    for (int m = 0; m < rg.n; m++, os += 2 * plane, od += 2 * plane) ring_emit(rg, m, x, y, os, od);
 }
 
 // ------------------------------------------------------------ per-atom operands
@@ -234,66 +247,48 @@ __device__ __forceinline__ void ring_x_value(const OzAtomArgs &xa, const AtomDes
 }
 
 // Row 2-norms (their powers of two into xsig) and residue planes of 32 rows
-// of one atom's X: the norms first (interleaved f', fixed order), then the
-// window in steps of 64 bytes transposed through shared memory.
+// of one atom's X, 64 window bytes per block (blockIdx.y): every block forms
+// the norms again (interleaved f', fixed order; the operands are in the L2), then
+// transposes its step through shared memory.  Latency: eight atoms 34 us (50
+// with one block walking the whole window).
 __global__ void __launch_bounds__(256) oz_ring_x_kernel(DevParams p, OzAtomArgs xa, const __grid_constant__ OzRing rg)
 {
     __shared__ double t[2][64][33];
     __shared__ double part[8][33];
-    const int ias = blockIdx.y, n0 = blockIdx.x * 32;
-    const AtomDesc at = p.atoms[ias];
+    const int ias = blockIdx.z, n0 = blockIdx.x * 32, k0 = blockIdx.y * 64;
+    const AtomDesc &at = p.atoms[ias];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int napw = at.napw, delta = at.apw_off - at.oz_x0;
     double s = 0.0;
-#pragma unroll 4
-    for (int fp = ty; fp < at.napw; fp += 8) {
+#pragma unroll 8
+    for (int fp = ty; fp < napw; fp += 8) {
         double re, im;
         ring_x_value(xa, at, ias, n0 + tx, fp, re, im);
         s = fma(re, re, fma(im, im, s));
     }
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const int k = ty + 8 * q;
+        ring_x_value(xa, at, ias, n0 + tx, k0 + k - delta, t[0][k][tx], t[1][k][tx]);
+    }
     part[ty][tx] = s;
     __syncthreads();
-    if (ty == 0) {
-        double v = 0.0;
-        for (int q = 0; q < 8; q++) v += part[q][tx];
-        v = oz_sigma(sqrt(v) * (1.0 + 0x1p-30));
-        part[0][tx] = v;
-        xa.xsig[(size_t)ias * xa.nrows + n0 + tx] = v;
-    }
-    __syncthreads();
-    const int delta = at.apw_off - at.oz_x0;
     const int nl = threadIdx.x >> 3, kl = (threadIdx.x & 7) * 8;
-    const double sc = ldexp(1.0 / part[0][nl], rg.bx);
-    for (int k0 = 0; k0 < xa.lw; k0 += 64) {
-        __syncthreads();
+    double v = 0.0;
+    for (int q = 0; q < 8; q++) v += part[q][nl];
+    v = oz_sigma(sqrt(v) * (1.0 + 0x1p-30));
+    if (k0 == 0 && kl == 0) xa.xsig[(size_t)ias * xa.nrows + n0 + nl] = v;
+    const double sc = ldexp(1.0 / v, rg.bx);
+    uint2 x[8], y[8];
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
-            const int k = ty + 8 * q;
-            ring_x_value(xa, at, ias, n0 + tx, k0 + k - delta, t[0][k][tx], t[1][k][tx]);
-        }
-        __syncthreads();
-        uint2 x[8], y[8];
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-            x[e] = ring_digits(t[0][kl + e][nl], sc);
-            y[e] = ring_digits(t[1][kl + e][nl], sc);
-        }
-        int8_t *out = xa.xs + ((size_t)ias * 2 * rg.n * xa.nrows + n0 + nl) * xa.lw + k0 + kl;
-        const size_t plane = (size_t)xa.nrows * xa.lw;
-#pragma unroll 1
-        for (int m = 0; m < rg.n; m++, out += 2 * plane) {
-            uint32_t ws[2], wd[2];
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                uint32_t sr[4], dr[4];
-#pragma unroll
-                for (int e = 0; e < 4; e++) ring_pair(rg, m, x[4 * q + e], y[4 * q + e], sr[e], dr[e]);
-                ws[q] = pack4(sr[0], sr[1], sr[2], sr[3]);
-                wd[q] = pack4(dr[0], dr[1], dr[2], dr[3]);
-            }
-            *reinterpret_cast<uint2 *>(out) = make_uint2(wd[0], wd[1]);              // h-
-            *reinterpret_cast<uint2 *>(out + plane) = make_uint2(ws[0], ws[1]);      // h+
-        }
+    for (int e = 0; e < 8; e++) {
+        x[e] = ring_digits(t[0][kl + e][nl], sc);
+        y[e] = ring_digits(t[1][kl + e][nl], sc);
     }
+    const size_t plane = (size_t)xa.nrows * xa.lw;
+    int8_t *out = xa.xs + ((size_t)ias * 2 * rg.n * xa.nrows + n0 + nl) * xa.lw + k0 + kl;
+#pragma unroll 1
+    for (int m = 0; m < rg.n; m++, out += 2 * plane) ring_emit(rg, m, x, y, out + plane, out);   // h+, h-
 }
 
 // ------------------------------------------------------------ the products
@@ -407,8 +402,8 @@ __device__ __forceinline__ void tma_load_4d_2sm(uint32_t dst, const CUtensorMap 
 // of its full-round tiles, then its share of the (tile, plane) pairs of the
 // remaining tiles: by planes (H/O), so that the clusters work on the same plane
 // of all these tiles at a time and share its operands in the L2 (dealt out in
-// runs, every cluster on another plane, they read 17 TB/s from HBM: three
-// k-points of 16 atoms REST), or in one run of planes per cluster (per-atom
+// runs, every cluster on another plane, each streams its own from HBM:
+// three k-points of 16 atoms 836 us, by planes 766), or in one run of planes per cluster (per-atom
 // tiles, which share little and whose producers then look a tile up once).
 template <bool RUNS>
 struct RingUnits {
@@ -898,7 +893,7 @@ __global__ void __launch_bounds__(128) oz_bcrt_kernel(DevParams p, const KDesc *
                                                       const __grid_constant__ OzRing rg, OzAtomArgs xa,
                                                       const uint8_t *res)
 {
-    __shared__ double T[2][RC_R][RC_C + 1];
+    __shared__ double T[2][RC_R][RC_C + 1], ssq[4][32];
     constexpr int NR = RG_BM / RC_R;
     const int tile = blockIdx.x / NR, rgrp = blockIdx.x % NR;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -943,6 +938,20 @@ __global__ void __launch_bounds__(128) oz_bcrt_kernel(DevParams p, const KDesc *
             v.im = -T[1][lane][c];
             kd.h[(size_t)g + nm * (row0 + n - napw)] = v;
         }
+    }
+    // sums of squares of the B columns over this block's rows: the warps' parts in order
+    if (n0 < napw) {
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < RC_C / 4; q++) {
+            const int c = warp + 4 * q;
+            if (n0 + c < napw) s = fma(T[0][lane][c], T[0][lane][c], fma(T[1][lane][c], T[1][lane][c], s));
+        }
+        ssq[warp][lane] = s;
+        __syncthreads();
+        if (warp == 0 && g < kd.ngp)
+            kd.oz_part[((size_t)ias * (xa.nrows / RC_C) + n0 / RC_C) * p.npad + g] =
+                ((ssq[0][lane] + ssq[1][lane]) + ssq[2][lane]) + ssq[3][lane];
     }
     if (n0 + RC_C > napw) {                                      // lo rows: lanes = two G of 16 rows
 #pragma unroll
@@ -1142,12 +1151,15 @@ void ring_row_blocks(int rows, int *nb, int *nrows)
     *nrows = blocks * *nb;
 }
 
-cudaError_t launch_oz_norm(const DevParams &p, const KDesc *d_k, int nk, int which, cudaStream_t s)
+size_t ring_part_rows(int natmtot, int nrows) { return (size_t)natmtot * (nrows / RC_C); }
+
+cudaError_t launch_oz_norm(const DevParams &p, const KDesc *d_k, int nk, int which, int per, cudaStream_t s)
 {
-    if (which == 0)
-        oz_norm_parts_kernel<<<dim3(p.npad / 64, nk), 64, 0, s>>>(p, d_k);      // npad: a multiple of 64
+    const dim3 grid(p.npad / 32, nk), block(32, 32);
+    if (per > 0)
+        oz_norm_kernel<true><<<grid, block, 0, s>>>(p, d_k, which, per);
     else
-        oz_norm_kernel<<<dim3(p.npad / 32, nk), dim3(32, 32), 0, s>>>(p, d_k, which);
+        oz_norm_kernel<false><<<grid, block, 0, s>>>(p, d_k, which, 0);
     return cudaGetLastError();
 }
 
@@ -1160,13 +1172,13 @@ cudaError_t launch_ring_split(const DevParams &p, const KDesc *d_k, int nk, cons
         return cudaFuncSetAttribute(oz_ring_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     });
     if (e != cudaSuccess) return e;
-    oz_ring_split_kernel<<<dim3(kp8 / RS_F, p.npad / 32, nk), 256, smem, s>>>(p, d_k, rg, kp8, which);
+    oz_ring_split_kernel<<<dim3(kp8 / RS_F, p.npad / 32, nk), RS_THREADS, smem, s>>>(p, d_k, rg, kp8, which);
     return cudaGetLastError();
 }
 
 cudaError_t launch_ring_x(const DevParams &p, const OzAtomArgs &xa, const OzRing &rg, cudaStream_t s)
 {
-    oz_ring_x_kernel<<<dim3(xa.nrows / 32, p.natmtot), 256, 0, s>>>(p, xa, rg);
+    oz_ring_x_kernel<<<dim3(xa.nrows / 32, xa.lw / 64, p.natmtot), 256, 0, s>>>(p, xa, rg);
     return cudaGetLastError();
 }
 

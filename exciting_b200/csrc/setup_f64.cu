@@ -25,26 +25,23 @@
 
 namespace exs {
 
-// Tiles are EDGE x EDGE, 128 threads, K slabs of 16 in a three-stage cp.async
-// ring.  EDGE 64 and 32: 2 x 2 warps of EDGE/2 x EDGE/2.  EDGE 16: the four
-// warps share one 16 x 16 tile, each taking every fourth K step, and add their
-// sums in a fixed order at the end: a 64 x 64 tile of K = 316 keeps one SM's
-// FP64 pipe busy for 42 us, so a single k-point of the two-atom cell (six
-// tiles) left 142 SMs idle.  gemm_edge picks the edge.  Rows are padded to
-// 4 (mod 16) doubles: the four K rows and four columns that half a warp reads
-// fall into different banks.
+// Tiles are EDGE x EDGE (64, 32 or 16), 128 threads: 2 x 2 warps of EDGE/2 x
+// EDGE/2, K slabs of 16 in a three-stage cp.async ring.  A 64 x 64 tile of
+// K = 316 keeps one SM's FP64 pipe busy for 42 us, so a single k-point of the
+// two-atom cell (six tiles) left 142 SMs idle; gemm_edge picks the edge.
+// Every element is summed over K in the same order whatever the edge, so the
+// results do not depend on the batch that an element's k-point comes in.  Rows
+// are padded to 4 (mod 16) doubles: the four K rows and four columns that half
+// a warp reads fall into different banks.
 constexpr int GB_K = 16, GB_STAGES = 3, GB_THREADS = 128;
 template <int EDGE>
 struct GemmCfg {
-    static constexpr int KS = EDGE == 16 ? 4 : 1;               // warps sharing a tile's K
-    static constexpr int WT = EDGE == 16 ? 16 : EDGE / 2;       // edge of a warp's sub-tile
+    static constexpr int WT = EDGE / 2;                         // edge of a warp's sub-tile
     static constexpr int MT = WT / 8;                           // 8 x 8 MMA tiles per warp and direction
     static constexpr int LDS = EDGE + 4;
     static constexpr int PLANE = GB_K * LDS;                    // doubles per plane per stage
     static constexpr int STAGE = 4 * PLANE;                     // xr, xi, yr, yi
-    static constexpr int RING = GB_STAGES * STAGE;
-    static constexpr int SUMS = KS > 1 ? (KS - 1) * 32 * MT * MT * 4 : 0;       // the other warps' sums
-    static constexpr size_t SMEM = (size_t)(RING > SUMS ? RING : SUMS) * sizeof(double);
+    static constexpr size_t SMEM = (size_t)GB_STAGES * STAGE * sizeof(double);
 };
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool valid)
@@ -106,7 +103,7 @@ zgemm_dmma_kernel(DevParams p, const GemmProb *probs, const TileWork *work, cons
     const GemmProb P = probs[tw.prob];
     const int m0 = tw.tm * EDGE, n0 = tw.tn * EDGE;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wm = C::KS > 1 ? 0 : warp >> 1, wn = C::KS > 1 ? 0 : warp & 1;
+    const int wm = warp >> 1, wn = warp & 1;
     const int mw = wm * C::WT, nw = wn * C::WT;            // this warp's sub-tile
     // upper tiles: sub-tiles below the diagonal are not formed
     const bool idle = GROUP == 1 && m0 + mw > n0 + nw + C::WT - 1;
@@ -135,8 +132,8 @@ zgemm_dmma_kernel(DevParams p, const GemmProb *probs, const TileWork *work, cons
         const double *st = smem + (kt % GB_STAGES) * C::STAGE;
         if (idle) continue;
 #pragma unroll
-        for (int kq = 0; kq < GB_K / 4 / C::KS; kq++) {
-            const int kr = (C::KS > 1 ? warp : kq) * 4 + (lane & 3);
+        for (int kq = 0; kq < GB_K / 4; kq++) {
+            const int kr = kq * 4 + (lane & 3);
             double ar[MT], aim[MT], naim[MT], br[MT], bi[MT];
 #pragma unroll
             for (int i = 0; i < MT; i++) {
@@ -174,39 +171,7 @@ zgemm_dmma_kernel(DevParams p, const GemmProb *probs, const TileWork *work, cons
     cp_async_wait<0>();
     __syncthreads();
 
-    if constexpr (C::KS > 1) {      // warps 1.. hand their sums to warp 0, which adds them in order
-        if (warp > 0) {
-            double *o = smem + (warp - 1) * 32 * MT * MT * 4 + lane;
-#pragma unroll
-            for (int i = 0; i < MT; i++)
-#pragma unroll
-                for (int j = 0; j < MT; j++)
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        o[((i * MT + j) * 4 + h) * 32] = cre[i][j][h];
-                        o[((i * MT + j) * 4 + 2 + h) * 32] = cim[i][j][h];
-                    }
-        }
-        __syncthreads();
-        if (warp == 0)
-            for (int w = 0; w < C::KS - 1; w++) {
-                const double *o = smem + w * 32 * MT * MT * 4 + lane;
-#pragma unroll
-                for (int i = 0; i < MT; i++)
-#pragma unroll
-                    for (int j = 0; j < MT; j++)
-#pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            cre[i][j][h] += o[((i * MT + j) * 4 + h) * 32];
-                            cim[i][j][h] += o[((i * MT + j) * 4 + 2 + h) * 32];
-                        }
-            }
-        __syncthreads();
-    }
-    const bool out = C::KS == 1 || warp == 0;       // warps that hold results
-
     if (GROUP == 0) {
-        if (!out) return;
         if (P.kind == EPI_PLANAR) {
             // split-precision path: column maxima of |B| (rows m of this tile),
             // reduced over the 8 row groups of a warp, then one atomic per column
@@ -282,7 +247,7 @@ zgemm_dmma_kernel(DevParams p, const GemmProb *probs, const TileWork *work, cons
         }
     }
     __syncthreads();
-    if (!out || idle) return;
+    if (idle) return;
     const int ngp = kd.ngp;
 #pragma unroll
     for (int i = 0; i < MT; i++)
@@ -315,7 +280,7 @@ zgemm_dmma_kernel(DevParams p, const GemmProb *probs, const TileWork *work, cons
 // pipe of one SM, so a launch of n tiles takes edge^2 max(1, n / 148) units;
 // the smaller tiles re-read more of their operands (0.9 and 0.7 of the rate).
 // One k-point of the two-atom cell: H and O 156 us in two launches of 64-tiles
-// -> 18 us (16), h_a A and the lo rows 62 -> 8 us; APW-lo rows of 27 k-points
+// -> 14 us (16), h_a A and the lo rows 62 -> 8 us; APW-lo rows of 27 k-points
 // (27 rows) 926 -> 498 us (32); A C of the eight-atom adjoint 178 -> 124 us (32).
 int gemm_edge(const long long n[3])
 {
@@ -462,102 +427,121 @@ cudaError_t launch_gemm(int group, int edge, const DevParams &p, const void *d_p
 }
 
 // ------------------------------------------- lo blocks that need no product
-// O APW-lo (overlapsetup.f90:111-127): for lo function j = (ilo, m) of atom
-// ias, O(G, ngp+idxlo) = sum_io conj(A(G, io, lm) (oalo(io,ilo) + h1loa)),
-// lower = conjugate.  One thread per (G, lo row of the whole lo block).
-__global__ void olp_apwlo_kernel(DevParams p, const KDesc *ks)
+// Local lo row rl of a species as (ilo, m): l of ilo, and m + l in `ml`.
+__device__ __forceinline__ int lo_row(const DevParams &p, int is, int rl, int &l, int &ml)
 {
-    const KDesc k = ks[blockIdx.z];
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    const int r = blockIdx.y;                     // global lo row 0..nlotot-1
-    if (g >= k.ngp) return;
-    // find the atom owning lo row r
-    int ias = 0;
-    while (ias + 1 < p.natmtot && (p.atoms[ias].losize == 0 || r >= p.atoms[ias].lo_off + p.atoms[ias].losize)) ias++;
-    const AtomDesc at = p.atoms[ias];
-    const int is = at.species;
-    const int rl = r - at.lo_off;
-    // decode (ilo, m) of the local lo row
-    int ilo = 0, base = 0, l = 0;
+    int ilo = 0, base = 0;
+    l = 0;
     for (; ilo < p.nlorb[is]; ilo++) {
         l = p.lorbl[ilo + p.nlomax * is];
         if (rl < base + 2 * l + 1) break;
         base += 2 * l + 1;
     }
-    const int m = rl - base - l;
-    // APW row f of (l, m, io=0) inside the atom
-    const int *apw = p.apword + (size_t)(p.lmaxapw + 1) * is;
-    int f = at.apw_off;
-    for (int ll = 0; ll < l; ll++) f += (2 * ll + 1) * apw[ll];
-    f += (m + l) * apw[l];
-    double sr = 0.0, si = 0.0;
-    for (int io = 0; io < apw[l]; io++) {
-        double w = p.oalo[io + (size_t)p.apwordmax * (ilo + (size_t)p.nlomax * ias)];
-        if (p.h1loa) w += p.h1loa[io + (size_t)p.apwordmax * (ilo + (size_t)p.nlomax * ias)];
-        const double are = k.ar[(size_t)(f + io) * p.npad + g], aim = k.ai[(size_t)(f + io) * p.npad + g];
-        sr += are * w;
-        si -= aim * w;
-    }
-    const int j = k.ngp + r;
-    exs_complex v; v.re = sr; v.im = si;
-    exs_complex vc; vc.re = sr; vc.im = -si;
-    k.o[(size_t)g + (size_t)k.nmat * j] = v;
-    k.o[(size_t)j + (size_t)k.nmat * g] = vc;
+    ml = rl - base;
+    return ilo;
 }
 
-// lo-lo blocks of H and O, every element of the nlotot x nlotot block.
-__global__ void lolo_kernel(DevParams p, const KDesc *ks)
+// One atom (blockIdx.y) of one k-point (z).  Blocks x < gx: the APW-lo block
+// of O (overlapsetup.f90:111-127) for 32 G: for lo function j = (ilo, m),
+// O(G, ngp+idxlo) = sum_io conj(A(G, io, lm) (oalo(io,ilo) + h1loa)), and its
+// conjugate, 32 lo rows at a time: the block decodes the rows once, writes
+// O(G, j) column by column and O(j, G) from shared memory, j contiguous.  Blocks
+// x >= gx: the atom's rows of 64 columns of the lo-lo blocks of H and O, zero
+// in the columns of other atoms.  Bound by the writes: 27 k-points of the
+// eight-atom cell 65 us (137 with one thread per element and 16-byte pieces of
+// O(j, G)), 64 atoms 76 us (215).
+constexpr int LO_R = 32, LO_COLS = 64;
+
+__global__ void __launch_bounds__(256) lo_blocks_kernel(DevParams p, const KDesc *ks, int gx)
 {
+    __shared__ double2 T[LO_R][33];
+    __shared__ double sw[LO_R][EXS_APWORD_MAX];
+    __shared__ int sf[LO_R], sn[LO_R];
     const KDesc k = ks[blockIdx.z];
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    const int c = blockIdx.y;
-    if (r >= p.nlotot) return;
-    double hr = 0.0, hi = 0.0, orr = 0.0;
-    int ia = 0, ib = 0;
-    while (ia + 1 < p.natmtot && (p.atoms[ia].losize == 0 || r >= p.atoms[ia].lo_off + p.atoms[ia].losize)) ia++;
-    while (ib + 1 < p.natmtot && (p.atoms[ib].losize == 0 || c >= p.atoms[ib].lo_off + p.atoms[ib].losize)) ib++;
-    if (ia == ib) {
-        const AtomDesc at = p.atoms[ia];
-        const int rl = r - at.lo_off, cl = c - at.lo_off;
-        // H: upper from lolo(r, c); lower = conj(lolo(c, r))   (copy_UL)
-        if (rl <= cl) {
-            const exs_complex v = p.lolo[rl + (size_t)p.maxnlo * (cl + (size_t)p.maxnlo * ia)];
-            hr = v.re; hi = v.im;
-        } else {
-            const exs_complex v = p.lolo[cl + (size_t)p.maxnlo * (rl + (size_t)p.maxnlo * ia)];
-            hr = v.re; hi = -v.im;
+    const int ias = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const AtomDesc &at = p.atoms[ias];
+    const int is = at.species, losize = at.losize, lo_off = at.lo_off;
+    if (losize == 0) return;
+    const size_t nm = (size_t)k.nmat;
+    if ((int)blockIdx.x < gx) {
+        const int g0 = blockIdx.x * 32;
+        if (g0 >= k.ngp) return;
+        for (int r0 = 0; r0 < losize; r0 += LO_R) {
+            const int nr = min(LO_R, losize - r0);
+            if (tid < nr) {
+                int l, ml;
+                const int ilo = lo_row(p, is, r0 + tid, l, ml);
+                const int *apw = p.apword + (size_t)(p.lmaxapw + 1) * is;
+                int f = at.apw_off;                              // APW row of (l, m, io = 0)
+                for (int ll = 0; ll < l; ll++) f += (2 * ll + 1) * apw[ll];
+                sf[tid] = f + ml * apw[l];
+                sn[tid] = apw[l];
+                for (int io = 0; io < apw[l]; io++) {
+                    const size_t q = io + (size_t)p.apwordmax * (ilo + (size_t)p.nlomax * ias);
+                    sw[tid][io] = p.oalo[q] + (p.h1loa ? p.h1loa[q] : 0.0);
+                }
+            }
+            __syncthreads();
+            const int g = g0 + lane;
+            for (int r = warp; r < nr; r += 8) {
+                double sr = 0.0, si = 0.0;
+                if (g < k.ngp) {
+                    for (int io = 0; io < sn[r]; io++) {
+                        const size_t q = (size_t)(sf[r] + io) * p.npad + g;
+                        sr += k.ar[q] * sw[r][io];
+                        si -= k.ai[q] * sw[r][io];
+                    }
+                    exs_complex v;
+                    v.re = sr;
+                    v.im = si;
+                    k.o[(size_t)g + nm * (k.ngp + lo_off + r0 + r)] = v;
+                }
+                T[r][lane] = make_double2(sr, -si);
+            }
+            __syncthreads();
+            for (int q = warp; q < 32; q += 8)                   // lane = lo row
+                if (g0 + q < k.ngp && lane < nr) {
+                    const double2 z = T[lane][q];
+                    exs_complex v;
+                    v.re = z.x;
+                    v.im = z.y;
+                    k.o[(size_t)(k.ngp + lo_off + r0 + lane) + nm * (g0 + q)] = v;
+                }
+            __syncthreads();
         }
-        // O: ololo(ilo1, ilo2) + h1lolo on equal l and m (taken from the upper element)
-        const int is = at.species;
-        const int ru = rl <= cl ? rl : cl, cu = rl <= cl ? cl : rl;
-        int i1 = 0, b1 = 0, l1 = 0, i2 = 0, b2 = 0, l2 = 0;
-        for (; i1 < p.nlorb[is]; i1++) { l1 = p.lorbl[i1 + p.nlomax * is]; if (ru < b1 + 2 * l1 + 1) break; b1 += 2 * l1 + 1; }
-        for (; i2 < p.nlorb[is]; i2++) { l2 = p.lorbl[i2 + p.nlomax * is]; if (cu < b2 + 2 * l2 + 1) break; b2 += 2 * l2 + 1; }
-        if (l1 == l2 && (ru - b1) == (cu - b2)) {
-            orr = p.ololo[i1 + (size_t)p.nlomax * (i2 + (size_t)p.nlomax * ia)];
-            if (p.h1lolo) orr += p.h1lolo[i1 + (size_t)p.nlomax * (i2 + (size_t)p.nlomax * ia)];
-        }
+        return;
     }
-    const size_t idx = (size_t)(k.ngp + r) + (size_t)k.nmat * (k.ngp + c);
-    exs_complex hv; hv.re = hr; hv.im = hi;
-    exs_complex ov; ov.re = orr; ov.im = 0.0;
-    k.h[idx] = hv;
-    k.o[idx] = ov;
+    const int c0 = ((int)blockIdx.x - gx) * LO_COLS;
+    for (int c = c0 + warp; c < min(p.nlotot, c0 + LO_COLS); c += 8)
+        for (int r = lane; r < losize; r += 32) {
+            const int cl = c - lo_off;
+            exs_complex hv, ov;
+            hv.re = hv.im = ov.re = ov.im = 0.0;
+            if (cl >= 0 && cl < losize) {
+                // H: upper from lolo(r, c); lower = conj(lolo(c, r))   (copy_UL)
+                const int ru = min(r, cl), cu = max(r, cl);
+                const exs_complex v = p.lolo[ru + (size_t)p.maxnlo * (cu + (size_t)p.maxnlo * ias)];
+                hv.re = v.re;
+                hv.im = r <= cl ? v.im : -v.im;
+                // O: ololo(ilo1, ilo2) + h1lolo on equal l and m (taken from the upper element)
+                int l1, m1, l2, m2;
+                const int i1 = lo_row(p, is, ru, l1, m1), i2 = lo_row(p, is, cu, l2, m2);
+                if (l1 == l2 && m1 == m2) {
+                    ov.re = p.ololo[i1 + (size_t)p.nlomax * (i2 + (size_t)p.nlomax * ias)];
+                    if (p.h1lolo) ov.re += p.h1lolo[i1 + (size_t)p.nlomax * (i2 + (size_t)p.nlomax * ias)];
+                }
+            }
+            const size_t idx = (size_t)(k.ngp + lo_off + r) + nm * (k.ngp + c);
+            k.h[idx] = hv;
+            k.o[idx] = ov;
+        }
 }
 
-cudaError_t launch_olp_apwlo(const DevParams &p, const KDesc *d_k, int nk, int ngp_max, cudaStream_t s)
-{
-    if (p.nlotot == 0 || ngp_max == 0) return cudaSuccess;
-    dim3 grid((ngp_max + 127) / 128, p.nlotot, nk);
-    olp_apwlo_kernel<<<grid, 128, 0, s>>>(p, d_k);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_lolo_blocks(const DevParams &p, const KDesc *d_k, int nk, cudaStream_t s)
+cudaError_t launch_lo_blocks(const DevParams &p, const KDesc *d_k, int nk, int ngp_max, cudaStream_t s)
 {
     if (p.nlotot == 0) return cudaSuccess;
-    dim3 grid((p.nlotot + 127) / 128, p.nlotot, nk);
-    lolo_kernel<<<grid, 128, 0, s>>>(p, d_k);
+    const int gx = (ngp_max + 31) / 32;
+    lo_blocks_kernel<<<dim3(gx + (p.nlotot + LO_COLS - 1) / LO_COLS, p.natmtot, nk), 256, 0, s>>>(p, d_k, gx);
     return cudaGetLastError();
 }
 
