@@ -423,7 +423,7 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
     int rows = 1;
     for (const AtomDesc &a : c->atoms) rows = std::max(rows, a.napw + a.losize);
     exs::ring_row_blocks(rows, &c->ring_nb, &c->ring_nrows);
-    const size_t xgroups = (size_t)c->natmtot * (mod ? 2 * ring.n : slices * c->oz_nxb);
+    const size_t xgroups = (size_t)c->natmtot * (mod ? 2 * ring.at.n : slices * c->oz_nxb);
     const size_t xs_bytes = xgroups * (mod ? c->ring_nrows : 128) * c->oz_lw;
     c->ozpart_rows = exs::ring_part_rows(c->natmtot, c->ring_nrows);
     const size_t nxsig = (size_t)c->natmtot * (mod ? c->ring_nrows : c->oz_nxb * 64);
@@ -911,7 +911,7 @@ int enqueue_setup(exs_ctx *c, const std::vector<KDesc> &ks, const Uploaded &u, b
         // A; B = h_a A and the APW-lo rows of H from the split h_a and loa
         EXS_CUDA(split(0));
         if (!b64 && mod)
-            EXS_CUDA(exs::launch_ring_atom(&c->ring_mapA, &c->ring_mapX, p, u.d_k, u.d_ozatiles, u.nozatiles,
+            EXS_CUDA(exs::launch_ring_atom(&c->ring_mapA, &c->ring_mapX, p, u.d_k, ks[0].oz_slot, u.d_ozatiles, u.nozatiles,
                                            c->oz_ring, c->oz_atom_args(), c->d_res, c->res_bytes, s));
         else if (!b64)
             EXS_CUDA(exs::launch_oz_atom(c->oz_cfg, &c->oz_mapArow, &c->oz_mapX, p, u.d_k, u.d_ozatiles,
@@ -929,7 +929,7 @@ int enqueue_setup(exs_ctx *c, const std::vector<KDesc> &ks, const Uploaded &u, b
         EXS_CUDA(split(1));
         const int q = c->oz_cfg;
         if (mod)
-            EXS_CUDA(exs::launch_ring_ho(c->ring_cols, &c->ring_mapHO1, &c->ring_mapHO2, p, u.d_k, u.d_oztiles, u.noztiles, c->oz_ring, c->kp8,
+            EXS_CUDA(exs::launch_ring_ho(c->ring_cols, &c->ring_mapHO1, &c->ring_mapHO2, p, u.d_k, ks[0].oz_slot, u.d_oztiles, u.noztiles, c->oz_ring, c->kp8,
                                          c->d_res, c->d_pace, s));
         else
             EXS_CUDA(exs::launch_oz_mma(q, &c->oz_mapA[q], (q & 8) ? &c->oz_mapB2[q] : &c->oz_mapB[q], p, u.d_k,

@@ -76,9 +76,22 @@ struct OzScheme {
     long long wait;                    // limit of the pipeline waits in cycles (0: OZ_WAIT_CYCLES)
 };
 
-// The rings Z_p of the modular products (oz_ring.cu): n moduli p[m] in which
-// i_m^2 = -1 has a solution, two planes each.
+// The recombination of integer products modulo the first n moduli of OzRing,
+// two moduli p, p' at a time.
 constexpr int OZ_RING_MAX = 16;
+struct OzCrt {
+    int n;
+    // weights of the residues in the real and imaginary parts as packed signed bytes, their offset (a
+    // multiple of p p'), round(2^96 / (p p')) in 32-bit words
+    int wlo[2][OZ_RING_MAX / 2], whi[2][OZ_RING_MAX / 2], woff[OZ_RING_MAX / 2];
+    unsigned d96[3][OZ_RING_MAX / 2];
+    int sh;                            // 64-bit window below the top of the 96-bit sum
+    double fin;                        // value of its unit: M 2^-(64+sh) 2^-(bits of the operands)
+};
+
+// The rings Z_p of the modular products (oz_ring.cu): n moduli p[m] in which
+// i_m^2 = -1 has a solution, two planes each; the per-atom products take the
+// first at.n of them.
 struct OzRing {
     int n, b, bx;
     long long wait;                    // limit of the pipeline waits in cycles (0: OZ_WAIT_CYCLES)
@@ -92,12 +105,7 @@ struct OzRing {
     // packed signed bytes; the sums' start values
     int clo[OZ_RING_MAX], chi[OZ_RING_MAX], ilo[OZ_RING_MAX], ihi[OZ_RING_MAX];
     int base[OZ_RING_MAX], icorr[OZ_RING_MAX];
-    // the recombination (two moduli p, p' at a time): weights of the residues in the real and imaginary parts
-    // as packed signed bytes, their offset (a multiple of p p'), round(2^96 / (p p')) in 32-bit words
-    int wlo[2][OZ_RING_MAX / 2], whi[2][OZ_RING_MAX / 2], woff[OZ_RING_MAX / 2];
-    unsigned d96[3][OZ_RING_MAX / 2];
-    int sh, shx;                       // 64-bit window below the top of the 96-bit sum: H/O, per-atom products
-    double fin, finx;                  // value of its unit: M 2^-(64+sh) 2^-2b, M 2^-(64+shx) 2^-(b+bx)
+    OzCrt ho, at;                      // H/O products, per-atom products
 };
 
 // Arrays of one plane: B, A, and with iora* (O = A^H C, C = (I + h1aa) A) C.
@@ -425,10 +433,11 @@ cudaError_t launch_ring_split(const DevParams &p, const KDesc *d_k, int nk, cons
                               cudaStream_t s);
 cudaError_t launch_ring_x(const DevParams &p, const OzAtomArgs &xa, const OzRing &rg, cudaStream_t s);
 cudaError_t launch_ring_ho(int cols, const CUtensorMap *map1, const CUtensorMap *map2, const DevParams &p,
-                           const KDesc *d_k, const void *d_tiles, int ntiles, const OzRing &rg, int kp8, uint8_t *res,
-                           int *pace, cudaStream_t s);
+                           const KDesc *d_k, int slot0, const void *d_tiles, int ntiles, const OzRing &rg, int kp8,
+                           uint8_t *res, int *pace, cudaStream_t s);
+// slot0: the slot of the batch's first k-point (the slots of a batch follow each other)
 cudaError_t launch_ring_atom(const CUtensorMap *mapA, const CUtensorMap *mapX, const DevParams &p, const KDesc *d_k,
-                             const void *d_tiles, int ntiles, const OzRing &rg, const OzAtomArgs &xa, uint8_t *res,
+                             int slot0, const void *d_tiles, int ntiles, const OzRing &rg, const OzAtomArgs &xa, uint8_t *res,
                              size_t res_bytes, cudaStream_t s);
 // Operands of h_a and loa for the active split arithmetic.
 inline cudaError_t launch_x(exs_ctx *c, cudaStream_t s)

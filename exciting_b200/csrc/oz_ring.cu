@@ -24,9 +24,10 @@
 // Plane P = 2m + q holds, as int8 residues in [-127, 127], A-, B+, C+ and h-
 // for q = 0 and A+, B-, C-, h+ for q = 1: product P of the H/O tiles is
 // A_P^T [B_P | A_(P^1)] (with iora* [B_P | C_P]), product P of the per-atom
-// tiles is A_P^T h_P.  n moduli make 2n products of two operands each: 14
-// moduli (104.4 bits) and 28 products at b = 49, where 13 larger moduli
-// (101.8 bits) with real and imaginary planes take 52.
+// tiles is A_P^T h_P.  n moduli make 2n products of two operands each: at
+// b = 49, bx = 45 14 moduli (104.4 bits) and 28 products for H and O, 13 and 26
+// for the per-atom products, where 13 larger moduli (101.8 bits) with real and
+// imaginary planes take 52.
 //
 // oz_plane_kernel forms the products tile by tile and stores the residues
 // z = v mod p in [0, p) of the int32 sums as bytes; oz_crt_kernel (H, O) and
@@ -286,9 +287,9 @@ __global__ void __launch_bounds__(256) oz_ring_x_kernel(DevParams p, OzAtomArgs 
         y[e] = ring_digits(t[1][kl + e][nl], sc);
     }
     const size_t plane = (size_t)xa.nrows * xa.lw;
-    int8_t *out = xa.xs + ((size_t)ias * 2 * rg.n * xa.nrows + n0 + nl) * xa.lw + k0 + kl;
+    int8_t *out = xa.xs + ((size_t)ias * 2 * rg.at.n * xa.nrows + n0 + nl) * xa.lw + k0 + kl;
 #pragma unroll 1
-    for (int m = 0; m < rg.n; m++, out += 2 * plane) ring_emit(rg, m, x, y, out + plane, out);   // h+, h-
+    for (int m = 0; m < rg.at.n; m++, out += 2 * plane) ring_emit(rg, m, x, y, out + plane, out);   // h+, h-
 }
 
 // ------------------------------------------------------------ the products
@@ -472,7 +473,7 @@ __device__ __forceinline__ uint32_t ring_mod_short(int v, int p, uint32_t mf, in
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(RG_THREADS, 1)
 oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, DevParams p,
-                const KDesc *ks, const int *tiles, int ntiles, const __grid_constant__ OzRing rg, OzAtomArgs xa,
+                int slot0, const int *tiles, int ntiles, const __grid_constant__ OzRing rg, OzAtomArgs xa,
                 uint8_t *res, int *pace)
 {
     using C = RingCfg<MODE>;
@@ -486,7 +487,7 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = cluster_ctarank();
     const uint32_t sbase = (smem_u32(rg_smem) + 1023u) & ~1023u;
-    const int cl = (int)(blockIdx.x >> 1), NP = 2 * rg.n;
+    const int cl = (int)(blockIdx.x >> 1), NP = 2 * (MODE == RG_ATOM ? rg.at.n : rg.n);
     RingUnits<MODE == RG_ATOM> units(ntiles, (int)(gridDim.x >> 1), NP, cl);
     const int N = MODE == RG_ATOM ? xa.nb : 256;         // MMA N
     const int b_rows = N / 2;                            // operand rows of a B operand in this CTA
@@ -530,29 +531,41 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                 arr = !o ? 0 : (p.relativity == EXS_REL_IORA ? 2 : 1);
                 flip = o && arr == 1 ? 1 : 0;
             }
+            // H/O: the next product's tile entries are loaded during the current one (among the remaining
+            // tiles every product has another tile)
+            auto entry = [&](int tile, int q) { return units.count > 0 ? tiles[3 * tile + q] : 0; };
+            int k_next = 0, b_next = 0;
+            if (MODE != RG_ATOM) {
+                k_next = entry(units.tile, 0);
+                b_next = entry(units.tile, role == 0 ? 1 : 2);
+            }
+            auto ahead = units;
             for (int u = 0; u < units.count && !bad; u++, units.next()) {
                 const int tile = units.tile, P = units.P;
-                if (tile != last) {      // what depends on the tile: dependent loads, once per tile
+                if (MODE != RG_ATOM) {
+                    slot = slot0 + k_next;
+                    row = role == 0 ? b_next * RG_BM + (int)rank * 128 : b_next * C::BJ + (C::WIDE ? (int)rank * 128 : 0);
+                    if (u + 1 < units.count) {
+                        ahead.next();
+                        k_next = entry(ahead.tile, 0);
+                        b_next = entry(ahead.tile, role == 0 ? 1 : 2);
+                    }
+                } else if (tile != last) {      // dependent loads, once per tile
                     last = tile;
-                    if (MODE == RG_ATOM) {
-                        const int ias = tiles[4 * tile + 1];
-                        const AtomDesc &at = p.atoms[ias];
-                        nch = at.oz_nch;
-                        if (role == 0) {
-                            slot = ks[tiles[4 * tile]].oz_slot;
-                            row = tiles[4 * tile + 2] * RG_BM + (int)rank * 128;
-                            x0 = at.oz_x0;
-                        } else {
-                            slot = ias;
-                            row = tiles[4 * tile + 3] * N + (int)rank * b_rows;
-                        }
+                    const int ias = tiles[4 * tile + 1];
+                    const AtomDesc &at = p.atoms[ias];
+                    nch = at.oz_nch;
+                    if (role == 0) {
+                        slot = slot0 + tiles[4 * tile];
+                        row = tiles[4 * tile + 2] * RG_BM + (int)rank * 128;
+                        x0 = at.oz_x0;
                     } else {
-                        slot = ks[tiles[3 * tile]].oz_slot;
-                        row = role == 0 ? tiles[3 * tile + 1] * RG_BM + (int)rank * 128
-                                        : tiles[3 * tile + 2] * C::BJ + (C::WIDE ? (int)rank * 128 : 0);
+                        slot = ias;
+                        row = tiles[4 * tile + 3] * N + (int)rank * b_rows;
                     }
                 }
-                const int plane = slot * NP + (P ^ flip);
+                // planes per slot of the split operands, per atom of h_a and loa
+                const int plane = slot * (MODE == RG_ATOM && role > 0 ? NP : 2 * rg.n) + (P ^ flip);
                 for (int kb = 0; kb < nch; kb += KCH, chunks += KCH) {
                     if (pacer && chunks % RG_PACE_CHUNKS == 0) ring_pace(pace, cl, units.ncl, chunks / RG_PACE_CHUNKS);
                     if (fills[st] > 0 && !mbar_wait_ab(&empty[st], (fills[st] - 1) & 1, abort, rg.wait)) {
@@ -647,12 +660,17 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         // ------------------------------------------------ epilogue (both CTAs, warps 4..19)
         const int qd = warp & 3, part = (warp - 4) >> 2;
         const int row = qd * 32 + lane;
-        const int nq = N / 16;                                      // 16-column chunks of an accumulator
+        int nq = N / 16, last = -1;                                 // 16-column chunks of an accumulator
         const uint32_t acce0[2] = {mapa_shared(smem_u32(&acce[0]), 0), mapa_shared(smem_u32(&acce[1]), 0)};
         const size_t plane_bytes = (size_t)C::NB * N * 128;         // residues of one product, this CTA's 128 rows
         bool bad = false;
         for (int u = 0; u < units.count && !bad; u++, units.next()) {
             const int P = units.P, m = P >> 1;
+            if (MODE == RG_ATOM && units.tile != last) {            // only the chunks that hold rows of the atom
+                last = units.tile;
+                const AtomDesc &at = p.atoms[tiles[4 * last + 1]];
+                nq = min(N, at.napw + at.losize - tiles[4 * last + 3] * N + 15) / 16;
+            }
             const int pm = rg.p[m], mg = rg.mg[m], up = rg.up[m];
             const uint32_t mf = rg.mf[m];
             uint8_t *out = res + ((size_t)(2 * units.tile + (int)rank) * NP + P) * plane_bytes + (size_t)row * 16;
@@ -739,8 +757,7 @@ __device__ __forceinline__ void ring_load4(const uint8_t *tres, size_t plane, in
 // multiply-adds (the top one needs 32 bits only) per PAIR of moduli, carries
 // propagated once at the end.  The signed 64-bit window sh bits below the top
 // of t is 2^(64+sh) X / M up to the rounding of D (below 2^29 units of 2^-96).
-__device__ __forceinline__ void ring_crt4(const OzRing &rg, const RingWords &z, int sh, double fin, double (&re)[4],
-                                          double (&im)[4])
+__device__ __forceinline__ void ring_crt4(const OzCrt &rg, const RingWords &z, double (&re)[4], double (&im)[4])
 {
     unsigned long long a0[8], a1[8];                    // re 0..3, im 0..3
     uint32_t a2[8];
@@ -773,8 +790,8 @@ __device__ __forceinline__ void ring_crt4(const OzRing &rg, const RingWords &z, 
     for (int e = 0; e < 8; e++) {
         const unsigned long long c1 = a1[e] + (a0[e] >> 32);
         const unsigned long long hi = ((unsigned long long)(a2[e] + (uint32_t)(c1 >> 32)) << 32) | (uint32_t)c1;
-        const unsigned long long top = (hi << sh) | ((a0[e] & 0xffffffffull) >> (32 - sh));
-        const double v = (double)(long long)top * fin;
+        const unsigned long long top = (hi << rg.sh) | ((a0[e] & 0xffffffffull) >> (32 - rg.sh));
+        const double v = (double)(long long)top * rg.fin;
         if (e < 4)
             re[e] = v;
         else
@@ -845,7 +862,7 @@ __global__ void __launch_bounds__(128) oz_crt_kernel(DevParams p, const KDesc *k
 #pragma unroll
     for (int w = 0; w < 2; w++) {
         double re[4], im[4];
-        ring_crt4(rg, z, rg.sh, rg.fin, re, im);
+        ring_crt4(rg.ho, z, re, im);
         if (w == 0) ring_load4(tres + (size_t)BJ * 128, plane, rg.n, 0, z);      // O
 #pragma unroll
         for (int e = 0; e < 4; e++) {
@@ -908,13 +925,13 @@ __global__ void __launch_bounds__(128) oz_bcrt_kernel(DevParams p, const KDesc *
     const int r = warp * 8 + (lane >> 2), cq = lane & 3;
     const int row = (rgrp * RC_R & 127) + r;
     RingWords z;
-    ring_load4(res + (size_t)(2 * tile + rgrp * RC_R / 128) * 2 * rg.n * plane + ((size_t)blockIdx.y * 128 + row) * 16 +
-                   cq * 4,
-               plane, rg.n, 1, z);
+    ring_load4(res + (size_t)(2 * tile + rgrp * RC_R / 128) * 2 * rg.at.n * plane +
+                   ((size_t)blockIdx.y * 128 + row) * 16 + cq * 4,
+               plane, rg.at.n, 1, z);
     const double sa = g0 + r < kd.ngp ? oz_sigma(kd.oz_scale[g0 + r]) : 0.0;
     const double *sig = xa.xsig + (size_t)ias * xa.nrows + n0 + cq * 4;
     double re[4], im[4];
-    ring_crt4(rg, z, rg.shx, rg.finx, re, im);
+    ring_crt4(rg.at, z, re, im);
 #pragma unroll
     for (int e = 0; e < 4; e++) {
         const double sc = sa * sig[e];
@@ -1049,25 +1066,20 @@ int oz_mod_plan(int n, int K, int kx, OzScheme *sch)
 static const int OZ_RINGS[OZ_RING_MAX] = {241, 233, 229, 221, 205, 197, 193, 181, 173,
                                           157, 149, 137, 113, 109, 101, 97};
 
-// Device constants for operands of b and bx bits: the fewest moduli whose
-// product M holds the integer products with one bit of margin,
-// log2 M >= max(2b, b + bx) + 2.
-int oz_ring_plan(int b, int bx, OzRing *out)
+// The recombination constants of products of `bits` bits: the fewest moduli
+// whose product M holds them with one bit of margin, log2 M >= bits + 2.
+static int oz_crt_plan(int bits, OzCrt *out)
 {
-    OzRing r{};
-    const int bits = std::max(2 * b, b + bx) + 2;
-    double lm = 0.0;
-    while (r.n < OZ_RING_MAX && lm - 1e-9 < bits) lm += std::log2((double)OZ_RINGS[r.n++]);
-    if (lm - 1e-9 < bits) return -1;
-    r.b = b;
-    r.bx = bx;
-    double M = 1.0;
-    for (int m = 0; m < r.n; m++) M *= (double)OZ_RINGS[m];
+    OzCrt r{};
+    double lm = 0.0, M = 1.0;
+    while (r.n < OZ_RING_MAX && lm - 1e-9 < bits + 2) {
+        lm += std::log2((double)OZ_RINGS[r.n]);
+        M *= (double)OZ_RINGS[r.n++];
+    }
+    if (lm - 1e-9 < bits + 2) return -1;
     // |X| / M < 2^-(sh + 2): the window's top bit is still the sign
-    r.sh = std::max(0, std::min(20, (int)std::floor(lm - 1e-9 - 2.0 * b - 3.0)));
-    r.shx = std::max(0, std::min(20, (int)std::floor(lm - 1e-9 - (double)(b + bx) - 3.0)));
-    r.fin = std::ldexp(M, -64 - r.sh - 2 * b);
-    r.finx = std::ldexp(M, -64 - r.shx - b - bx);
+    r.sh = std::max(0, std::min(20, (int)std::floor(lm - 1e-9 - (double)bits - 3.0)));
+    r.fin = std::ldexp(M, -64 - r.sh - bits);
     for (int m = 0; m < r.n; m++) {
         const int p = OZ_RINGS[m];
         int im = 0;
@@ -1077,29 +1089,9 @@ int oz_ring_plan(int b, int bx, OzRing *out)
             if (q != m) mm = mm * OZ_RINGS[q] % p;
         const int y = oz_inverse_mod(mm, p), half = oz_inverse_mod(2, p), iinv = oz_inverse_mod(im, p);
         if (im >= p || y < 0 || half < 0 || iinv < 0) return -1;
-        r.p[m] = p;
-        r.mg[m] = (int)((((long long)1 << 32) + p / 2) / p);
-        r.inv[m] = 1.0f / (float)p;
-        // symmetric residues of 2^(8k) and of i_m 2^(8k), k = 0..6, packed as signed bytes
-        auto sym = [p](long long v) { v = ((v % p) + p) % p; return (int)(v > p / 2 ? v - p : v); };
-        unsigned c[2] = {0, 0}, ci[2] = {0, 0};
-        for (int k = 0; k < 7; k++) {
-            const long long w = (1LL << (8 * k)) % p;
-            c[k >> 2] |= (unsigned)(uint8_t)(int8_t)sym(w) << (8 * (k & 3));
-            ci[k >> 2] |= (unsigned)(uint8_t)(int8_t)sym(w * im) << (8 * (k & 3));
-        }
-        r.clo[m] = (int)c[0];
-        r.chi[m] = (int)c[1];
-        r.ilo[m] = (int)ci[0];
-        r.ihi[m] = (int)ci[1];
-        // -2^55 removes the digits' offset; the sums start at the FP32 bits of a multiple of p near 1.5 2^23
-        const int start = 12582912 / p * p;
-        r.base[m] = 0x4B000000 - (1 << 23) + start + sym(-((1LL << 55) % p));
-        r.icorr[m] = sym(-((1LL << 55) % p) * im);
-        r.mf[m] = (unsigned)((1LL << 32) / p);
-        r.up[m] = ((1 << 27) / p + 1) * p;
-        // recombination: e_m times the other modulus of the pair (2q, 2q + 1), symmetric mod their product,
-        // as signed bytes 256 h + l for z+ (and, negated for the imaginary parts, z-)
+        // e_m times the other modulus of the pair (2q, 2q + 1), symmetric mod their product, as signed bytes
+        // 256 h + l for z+ (and, negated for the imaginary parts, z-); an odd count leaves the last pair half
+        // empty: weight 0
         const int other = (m ^ 1) < r.n ? OZ_RINGS[m ^ 1] : 1, pq = p * other, q = m / 2, sft = 16 * (m & 1);
         for (int c = 0; c < 2; c++) {
             long long f = (long long)y * half % p * (c ? iinv : 1) % p * other;
@@ -1122,6 +1114,47 @@ int oz_ring_plan(int b, int bx, OzRing *out)
     return 0;
 }
 
+// Device constants for operands of b and bx bits: the moduli of the H/O
+// products (2b bits) and of the per-atom products (b + bx bits; 13 of the 14 at
+// b = 49, bx = 45: 7 % fewer products and residues than with all of them).
+int oz_ring_plan(int b, int bx, OzRing *out)
+{
+    OzRing r{};
+    if (oz_crt_plan(2 * b, &r.ho) != 0 || oz_crt_plan(b + bx, &r.at) != 0) return -1;
+    r.n = std::max(r.ho.n, r.at.n);
+    r.b = b;
+    r.bx = bx;
+    for (int m = 0; m < r.n; m++) {
+        const int p = OZ_RINGS[m];
+        int im = 0;
+        while (im < p && (im * im + 1) % p != 0) im++;
+        if (im >= p) return -1;
+        r.p[m] = p;
+        r.mg[m] = (int)((((long long)1 << 32) + p / 2) / p);
+        r.mf[m] = (unsigned)((1LL << 32) / p);
+        r.up[m] = ((1 << 27) / p + 1) * p;
+        r.inv[m] = 1.0f / (float)p;
+        // symmetric residues of 2^(8k) and of i_m 2^(8k), k = 0..6, packed as signed bytes
+        auto sym = [p](long long v) { v = ((v % p) + p) % p; return (int)(v > p / 2 ? v - p : v); };
+        unsigned c[2] = {0, 0}, ci[2] = {0, 0};
+        for (int k = 0; k < 7; k++) {
+            const long long w = (1LL << (8 * k)) % p;
+            c[k >> 2] |= (unsigned)(uint8_t)(int8_t)sym(w) << (8 * (k & 3));
+            ci[k >> 2] |= (unsigned)(uint8_t)(int8_t)sym(w * im) << (8 * (k & 3));
+        }
+        r.clo[m] = (int)c[0];
+        r.chi[m] = (int)c[1];
+        r.ilo[m] = (int)ci[0];
+        r.ihi[m] = (int)ci[1];
+        // -2^55 removes the digits' offset; the sums start at the FP32 bits of a multiple of p near 1.5 2^23
+        const int start = 12582912 / p * p;
+        r.base[m] = 0x4B000000 - (1 << 23) + start + sym(-((1LL << 55) % p));
+        r.icorr[m] = sym(-((1LL << 55) % p) * im);
+    }
+    *out = r;
+    return 0;
+}
+
 // Columns of the H/O tiles.  256-column tiles read three quarters of the
 // operand bytes per product, but their epilogue stops the MMAs once per
 // product: 0.85 against 0.81 ms at K = 2592 (16 atoms, 3 k), 1.68 against
@@ -1138,7 +1171,7 @@ size_t ring_slot_bytes(const OzRing &rg, int npad, int kp8, int relativity)
 
 size_t ring_ho_tile_bytes(const OzRing &rg, int cols) { return (size_t)2 * rg.n * RG_BM * 2 * cols; }
 
-size_t ring_atom_tile_bytes(const OzRing &rg, int nb) { return (size_t)2 * rg.n * RG_BM * nb; }
+size_t ring_atom_tile_bytes(const OzRing &rg, int nb) { return (size_t)2 * rg.at.n * RG_BM * nb; }
 
 size_t ring_pace_bytes() { return sizeof(int) * RG_PACE_MAX; }
 
@@ -1220,8 +1253,8 @@ static cudaError_t plane_grid(int ntiles, int np, cudaStream_t s, int *ncl)
 constexpr size_t RG_PACE_BYTES = (size_t)100 << 20;
 
 template <int MODE>
-static cudaError_t launch_ho(const CUtensorMap *map, const DevParams &p, const KDesc *d_k, const int *d_tiles,
-                             int ntiles, const OzRing &rg, int kp8, uint8_t *res, int *pace, cudaStream_t s)
+static cudaError_t launch_ho(const CUtensorMap *map, const DevParams &p, const KDesc *d_k, int slot0,
+                             const int *d_tiles, int ntiles, const OzRing &rg, int kp8, uint8_t *res, int *pace, cudaStream_t s)
 {
     using C = RingCfg<MODE>;
     int ncl = 0;
@@ -1232,7 +1265,7 @@ static cudaError_t launch_ho(const CUtensorMap *map, const DevParams &p, const K
         e = cudaMemsetAsync(pace, 0, sizeof(int) * ncl, s);
         if (e != cudaSuccess) return e;
     }
-    oz_plane_kernel<MODE><<<2 * ncl, RG_THREADS, C::SMEM, s>>>(*map, *map, p, d_k, d_tiles, ntiles, rg, OzAtomArgs{},
+    oz_plane_kernel<MODE><<<2 * ncl, RG_THREADS, C::SMEM, s>>>(*map, *map, p, slot0, d_tiles, ntiles, rg, OzAtomArgs{},
                                                                res, paced ? pace : nullptr);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -1241,18 +1274,18 @@ static cudaError_t launch_ho(const CUtensorMap *map, const DevParams &p, const K
 }
 
 cudaError_t launch_ring_ho(int cols, const CUtensorMap *map1, const CUtensorMap *map2, const DevParams &p,
-                           const KDesc *d_k, const void *d_tiles, int ntiles, const OzRing &rg, int kp8, uint8_t *res,
-                           int *pace, cudaStream_t s)
+                           const KDesc *d_k, int slot0, const void *d_tiles, int ntiles, const OzRing &rg, int kp8,
+                           uint8_t *res, int *pace, cudaStream_t s)
 {
     if (ntiles <= 0) return cudaSuccess;
     const int *t = (const int *)d_tiles;
-    return cols == 256 ? launch_ho<RG_WIDE>(map1, p, d_k, t, ntiles, rg, kp8, res, pace, s)
-                       : launch_ho<RG_HO>(map2, p, d_k, t, ntiles, rg, kp8, res, pace, s);
+    return cols == 256 ? launch_ho<RG_WIDE>(map1, p, d_k, slot0, t, ntiles, rg, kp8, res, pace, s)
+                       : launch_ho<RG_HO>(map2, p, d_k, slot0, t, ntiles, rg, kp8, res, pace, s);
 }
 
 // Per-atom products in chunks of tiles whose residues fit the residue buffer.
 cudaError_t launch_ring_atom(const CUtensorMap *mapA, const CUtensorMap *mapX, const DevParams &p, const KDesc *d_k,
-                             const void *d_tiles, int ntiles, const OzRing &rg, const OzAtomArgs &xa, uint8_t *res,
+                             int slot0, const void *d_tiles, int ntiles, const OzRing &rg, const OzAtomArgs &xa, uint8_t *res,
                              size_t res_bytes, cudaStream_t s)
 {
     const int cap = (int)std::min<size_t>(res_bytes / ring_atom_tile_bytes(rg, xa.nb), 1 << 24);
@@ -1261,9 +1294,9 @@ cudaError_t launch_ring_atom(const CUtensorMap *mapA, const CUtensorMap *mapX, c
         const int nt = std::min(cap, ntiles - t0);
         const int *tiles = (const int *)d_tiles + 4 * (size_t)t0;
         int ncl = 0;
-        cudaError_t e = plane_grid<RG_ATOM>(nt, 2 * rg.n, s, &ncl);
+        cudaError_t e = plane_grid<RG_ATOM>(nt, 2 * rg.at.n, s, &ncl);
         if (e != cudaSuccess) return e;
-        oz_plane_kernel<RG_ATOM><<<2 * ncl, RG_THREADS, RingCfg<RG_ATOM>::SMEM, s>>>(*mapA, *mapX, p, d_k, tiles, nt, rg, xa, res,
+        oz_plane_kernel<RG_ATOM><<<2 * ncl, RG_THREADS, RingCfg<RG_ATOM>::SMEM, s>>>(*mapA, *mapX, p, slot0, tiles, nt, rg, xa, res,
                                                                       nullptr);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
