@@ -753,10 +753,11 @@ __device__ __forceinline__ void ring_load4(const uint8_t *tres, size_t plane, in
 // weights reduced to symmetric residues mod p p' (|.| < 2^15), in two signed
 // bytes: two dot products with the bytes z+, z-, z+', z-' of the value, the
 // low one started at a multiple of p p' that keeps 0 <= w < 2^27.  Then
-// t += w D (mod 2^96), D = round(2^96 / (p p')): three 32 x 32-bit
-// multiply-adds (the top one needs 32 bits only) per PAIR of moduli, carries
-// propagated once at the end.  The signed 64-bit window sh bits below the top
-// of t is 2^(64+sh) X / M up to the rounding of D (below 2^29 units of 2^-96).
+// t += w D (mod 2^96), D = round(2^(96+sh) / (p p')) mod 2^96: three 32 x
+// 32-bit multiply-adds (the top one needs 32 bits only) per PAIR of moduli,
+// carries propagated once at the end.  The top sh bits of 2^96 X / M are copies
+// of its sign, so the top 64 bits of t as a signed integer are 2^(64+sh) X / M
+// up to the rounding of D (below 2^29 units of 2^-96).
 __device__ __forceinline__ void ring_crt4(const OzCrt &rg, const RingWords &z, double (&re)[4], double (&im)[4])
 {
     unsigned long long a0[8], a1[8];                    // re 0..3, im 0..3
@@ -789,8 +790,7 @@ __device__ __forceinline__ void ring_crt4(const OzCrt &rg, const RingWords &z, d
 #pragma unroll
     for (int e = 0; e < 8; e++) {
         const unsigned long long c1 = a1[e] + (a0[e] >> 32);
-        const unsigned long long hi = ((unsigned long long)(a2[e] + (uint32_t)(c1 >> 32)) << 32) | (uint32_t)c1;
-        const unsigned long long top = (hi << rg.sh) | ((a0[e] & 0xffffffffull) >> (32 - rg.sh));
+        const unsigned long long top = ((unsigned long long)(a2[e] + (uint32_t)(c1 >> 32)) << 32) | (uint32_t)c1;
         const double v = (double)(long long)top * rg.fin;
         if (e < 4)
             re[e] = v;
@@ -800,15 +800,18 @@ __device__ __forceinline__ void ring_crt4(const OzCrt &rg, const RingWords &z, d
 }
 
 // Recombination, scaling, interstitial term and store of the H/O tiles: a
-// block of four warps takes 32 rows x 16 columns of both matrices.  Lane l
-// of a warp recombines row l / 4 of its eight, columns 4 (l % 4) .. + 3, so a
-// warp reads 128 contiguous residue bytes per plane; the index of G_i - G_j
-// is looked up once for H and O.  The values are staged in shared memory and
-// leave as whole column segments: 512 bytes of the upper triangle, 256 bytes
-// of the mirror.  Bound by the residue reads and the H/O writes (HBM) and
-// by the integer multiply-adds.  27 k-points of the eight-atom cell 0.54 ms, 64
-// atoms 1.36 ms; one thread per row and eight columns, the mirror stored from
-// registers, took 0.88 and 2.18 ms.
+// block of four warps takes 32 rows x 16 columns of both matrices.  First lane
+// l of a warp recombines row l / 4 of its eight, columns 4 (l % 4) .. + 3, so a
+// warp reads 128 contiguous residue bytes per plane, and stages the values in
+// shared memory.  Then a lane takes a row and every fourth column: the index of
+// G_i - G_j, looked up once for H and O before the recombination, and the table
+// entries, all in flight together; the values leave as whole column segments,
+// 512 bytes of the upper triangle, 256 bytes of the mirror.  The blocks of a
+// tile follow each other, so that the pieces of a column meet in the L2 before
+// they go to HBM.  Bound by the residue reads and the H/O writes: 27 k-points of
+// the eight-atom cell 0.48 ms, 64 atoms 1.19 ms (0.52 and 1.31 with the column
+// groups launched apart, 0.88 and 2.18 with one thread per row and eight
+// columns and the mirror stored from registers).
 constexpr int RC_R = 32, RC_C = 16;
 
 template <int BJ>
@@ -818,18 +821,19 @@ __global__ void __launch_bounds__(128) oz_crt_kernel(DevParams p, const KDesc *k
     __shared__ exs_complex T[2][RC_R][RC_C + 1];
     __shared__ double sv[RC_R + RC_C][3], ssig[RC_R + 2 * RC_C];
     __shared__ int siv[RC_R + RC_C][3];
-    constexpr int NR = RG_BM / RC_R;                             // row groups of a tile
-    const int tile = blockIdx.x / NR, rgrp = blockIdx.x % NR;
+    constexpr int NR = RG_BM / RC_R, NC = RC_C / 4;              // row groups of a tile; columns of a lane
+    constexpr int NB = BJ / RC_C;                                // column groups, fastest: see above
+    const int cgrp = blockIdx.x % NB, rgrp = blockIdx.x / NB % NR, tile = blockIdx.x / (NB * NR);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const KDesc kd = ks[tiles[3 * tile]];
     const int i0 = tiles[3 * tile + 1] * RG_BM + rgrp * RC_R;
-    const int j0 = tiles[3 * tile + 2] * BJ + blockIdx.y * RC_C;
+    const int j0 = tiles[3 * tile + 2] * BJ + cgrp * RC_C;
     if (i0 >= kd.ngp || j0 >= kd.ngp || j0 + RC_C - 1 < i0) return;    // no element i <= j < ngp here
     constexpr size_t plane = 2 * BJ * 128;
     const int r = warp * 8 + (lane >> 2), cq = lane & 3;
     const int row = (rgrp * RC_R & 127) + r;                     // of the 128-row tile
     const uint8_t *tres = res + (size_t)(2 * tile + rgrp * RC_R / 128) * 2 * rg.n * plane +
-                          ((size_t)blockIdx.y * 128 + row) * 16 + cq * 4;
+                          ((size_t)cgrp * 128 + row) * 16 + cq * 4;
     RingWords z;
     ring_load4(tres, plane, rg.n, 0, z);                         // H
     if (tid < RC_R + RC_C) {                                     // G vectors and scales of the rows and columns
@@ -853,11 +857,12 @@ __global__ void __launch_bounds__(128) oz_crt_kernel(DevParams p, const KDesc *k
         }
     }
     __syncthreads();
-    int ig[4];
+    const int i = i0 + lane;                                     // this lane's row of the second part
+    int ig[NC];
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-        const int c = RC_R + cq * 4 + e, j = j0 + cq * 4 + e;
-        ig[e] = (i0 + r <= j && j < kd.ngp) ? interstitial_index(p, siv[r], siv[c]) : 0;
+    for (int q = 0; q < NC; q++) {
+        const int c = warp + 4 * q, j = j0 + c;
+        ig[q] = i <= j && j < kd.ngp ? interstitial_index(p, siv[lane], siv[RC_R + c]) : 0;
     }
 #pragma unroll
     for (int w = 0; w < 2; w++) {
@@ -866,37 +871,54 @@ __global__ void __launch_bounds__(128) oz_crt_kernel(DevParams p, const KDesc *k
         if (w == 0) ring_load4(tres + (size_t)BJ * 128, plane, rg.n, 0, z);      // O
 #pragma unroll
         for (int e = 0; e < 4; e++) {
-            const int c = RC_R + cq * 4 + e;
-            const double sc = ssig[r] * ssig[c + w * RC_C];
+            const double sc = ssig[r] * ssig[RC_R + w * RC_C + cq * 4 + e];
             exs_complex v;
             v.re = re[e] * sc;
             v.im = im[e] * sc;
-            if (ig[e] > 0) {
-                double ar, ai;
-                interstitial_value(p, w == 0 ? EPI_HAM : EPI_OVL, ig[e], sv[r], sv[c], ar, ai);
-                v.re += ar;
-                v.im += ai;
-            }
             T[w][r][cq * 4 + e] = v;
+        }
+    }
+    // the interstitial terms of this lane's elements
+    double2 hi[NC], oi[NC];
+#pragma unroll
+    for (int q = 0; q < NC; q++) {
+        hi[q] = oi[q] = make_double2(0.0, 0.0);
+        if (ig[q] > 0) {
+            const int c = RC_R + warp + 4 * q;
+            interstitial_value(p, EPI_HAM, ig[q], sv[lane], sv[c], hi[q].x, hi[q].y);
+            interstitial_value(p, EPI_OVL, ig[q], sv[lane], sv[c], oi[q].x, oi[q].y);
         }
     }
     __syncthreads();
     const size_t nm = (size_t)kd.nmat;
 #pragma unroll
+    for (int q = 0; q < NC; q++) {                               // upper: lane = row
+        const int c = warp + 4 * q, j = j0 + c;
+        if (j < kd.ngp && i <= j) {
+            exs_complex h = T[0][lane][c], o = T[1][lane][c];
+            if (ig[q] > 0) {
+                h.re += hi[q].x;
+                h.im += hi[q].y;
+                o.re += oi[q].x;
+                o.im += oi[q].y;
+                T[0][lane][c] = h;
+                T[1][lane][c] = o;
+            }
+            kd.h[(size_t)i + nm * j] = h;
+            kd.o[(size_t)i + nm * j] = o;
+        }
+    }
+    __syncthreads();
+#pragma unroll
     for (int w = 0; w < 2; w++) {
         exs_complex *out = w == 0 ? kd.h : kd.o;
 #pragma unroll
-        for (int q = 0; q < RC_C / 4; q++) {                     // upper: lane = row
-            const int c = warp + 4 * q, i = i0 + lane, j = j0 + c;
-            if (j < kd.ngp && i <= j) out[(size_t)i + nm * j] = T[w][lane][c];
-        }
-#pragma unroll
         for (int q = 0; q < RC_R / 8; q++) {                     // mirror: lanes = two rows of 16 columns
-            const int rr = warp * 8 + 2 * q + (lane >> 4), i = i0 + rr, j = j0 + (lane & 15);
-            if (j < kd.ngp && i < j) {
+            const int rr = warp * 8 + 2 * q + (lane >> 4), ii = i0 + rr, j = j0 + (lane & 15);
+            if (j < kd.ngp && ii < j) {
                 exs_complex v = T[w][rr][lane & 15];
                 v.im = -v.im;
-                out[(size_t)j + nm * i] = v;
+                out[(size_t)j + nm * ii] = v;
             }
         }
     }
@@ -904,9 +926,10 @@ __global__ void __launch_bounds__(128) oz_crt_kernel(DevParams p, const KDesc *k
 
 // Recombination of the per-atom tiles, organised like oz_crt_kernel (32 G x
 // 16 rows of X per block): the B planes, 256 contiguous bytes per row, and the
-// APW-lo rows of H with their mirror.  64 atoms 1.07 ms (one thread per G and
-// eight rows: 1.36 ms).
-__global__ void __launch_bounds__(128) oz_bcrt_kernel(DevParams p, const KDesc *ks, const int *tiles,
+// APW-lo rows of H with their mirror.  64 atoms 1.04 ms (one thread per G and
+// eight rows: 1.36 ms); 27 k-points of the eight-atom cell 0.71 ms, 0.47 of it
+// without the arithmetic.
+__global__ void __launch_bounds__(128, 6) oz_bcrt_kernel(DevParams p, const KDesc *ks, const int *tiles,
                                                       const __grid_constant__ OzRing rg, OzAtomArgs xa,
                                                       const uint8_t *res)
 {
@@ -1106,8 +1129,8 @@ static int oz_crt_plan(int bits, OzCrt *out)
         }
         if ((m & 1) == 0) {
             r.woff[q] = (((1 << 26) + pq - 1) / pq) * pq;   // |w| <= 4 * 255 * 2^15 < 2^26 before the offset
-            const unsigned __int128 d = (((unsigned __int128)1 << 96) + pq / 2) / pq;
-            for (int w = 0; w < 3; w++) r.d96[w][q] = (unsigned)(d >> (32 * w));
+            const unsigned __int128 d = (((unsigned __int128)1 << (96 + r.sh)) + pq / 2) / pq;
+            for (int w = 0; w < 3; w++) r.d96[w][q] = (unsigned)(d >> (32 * w));       // mod 2^96
         }
     }
     *out = r;
@@ -1269,7 +1292,7 @@ static cudaError_t launch_ho(const CUtensorMap *map, const DevParams &p, const K
                                                                res, paced ? pace : nullptr);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    oz_crt_kernel<C::BJ><<<dim3(ntiles * (RG_BM / RC_R), C::BJ / RC_C), 128, 0, s>>>(p, d_k, d_tiles, rg, res);
+    oz_crt_kernel<C::BJ><<<(unsigned)ntiles * (RG_BM / RC_R) * (C::BJ / RC_C), 128, 0, s>>>(p, d_k, d_tiles, rg, res);
     return cudaGetLastError();
 }
 

@@ -137,16 +137,16 @@ def test_products_recombine(n):
                     assert -128 <= (sgn * f - lo) // 256 <= 127
                 w[c] += f * (zp + (-1) ** c * zm).astype(object)
         assert w.min() >= 0 and w.max() < 2 ** 27
-        t += w * (((1 << 96) + pq // 2) // pq)
+        t += w * ((((1 << (96 + sh)) + pq // 2) // pq) % 2 ** 96)
         bound += 2 ** 27 / 2
     for part, exact in ((0, lambda i, j: ar[:, i].astype(object) @ br[:, j] + ai[:, i].astype(object) @ bi[:, j]),
                         (1, lambda i, j: ar[:, i].astype(object) @ bi[:, j] - ai[:, i].astype(object) @ br[:, j])):
         for i in range(4):
             for j in range(4):
-                top = (int(t[part, i, j]) >> (32 - sh)) % 2 ** 64
+                top = (int(t[part, i, j]) >> 32) % 2 ** 64
                 top -= 2 ** 64 if top >= 2 ** 63 else 0
                 err = abs(top * M - int(exact(i, j)) * 2 ** (64 + sh))
-                assert err <= (bound / 2 ** (32 - sh) + 1) * M
+                assert err <= (bound / 2 ** 32 + 1) * M
 
 
 @pytest.mark.parametrize("runs", [False, True])
