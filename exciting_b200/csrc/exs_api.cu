@@ -428,9 +428,12 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
     c->ozpart_rows = exs::ring_part_rows(c->natmtot, c->ring_nrows);
     const size_t nxsig = (size_t)c->natmtot * (mod ? c->ring_nrows : c->oz_nxb * 64);
     // moduli: the residues of the H/O products of a whole batch (the upper tiles of ngkmax G+k per
-    // k-point); the per-atom products run before them in the same buffer, in chunks that fit it, of at
-    // least 256 MB where there is that much
-    size_t res = 0;
+    // k-point), at most RES_MAX of them at a time; the per-atom products run before them in the same
+    // buffer, in chunks of at least 256 MB where there is that much.  RES_MAX: the 64-atom cell and the
+    // batches of the eight-atom cell (up to 2.0 GB) run in one chunk; one k-point of 216 atoms would take
+    // 21 GB, beside 85 GB of operands, and takes six chunks of ~90 ms instead
+    constexpr size_t RES_MAX = (size_t)4 << 30;
+    size_t res = 0, res_tile = 0;
     if (mod) {
         size_t tiles = 0, atiles = 0;
         const int nib = (c->ngkmax + 255) / 256;
@@ -439,20 +442,30 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
             for (int jb = 0; jb < (c->ngkmax + cols - 1) / cols; jb++)
                 if (jb * cols + cols - 1 >= ib * 256) tiles++;
         atiles = (size_t)c->natmtot * nib * (c->ring_nrows / c->ring_nb);
-        res = std::max(tiles * exs::ring_ho_tile_bytes(ring, cols) * c->max_batch,
-                       std::min((size_t)256 << 20, atiles * exs::ring_atom_tile_bytes(ring, c->ring_nb) * c->max_batch));
+        const size_t ho = exs::ring_ho_tile_bytes(ring, cols), at = exs::ring_atom_tile_bytes(ring, c->ring_nb);
+        res_tile = std::max(ho, at);
+        res = std::min(RES_MAX, std::max(tiles * ho * c->max_batch,
+                                         std::min((size_t)256 << 20, atiles * at * c->max_batch)));
+        res = std::max(res, res_tile);
     }
     cudaError_t e = cudaMalloc((void **)&c->d_oz, slot * c->max_batch);
-    if (e == cudaSuccess && res > 0) {
-        e = cudaMalloc((void **)&c->d_res, res);
-        if (e == cudaSuccess) c->res_bytes = res;
-        if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_pace, exs::ring_pace_bytes());
-    }
+    if (e == cudaSuccess && mod) e = cudaMalloc((void **)&c->d_pace, exs::ring_pace_bytes());
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_ozscale, sizeof(double) * 3 * c->npad * c->max_batch);
     if (e == cudaSuccess && mod)
         e = cudaMalloc((void **)&c->d_ozpart, sizeof(double) * c->ozpart_rows * c->npad * c->max_batch);
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_xs, xs_bytes);
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_xsig, sizeof(double) * nxsig);
+    // last, so that a nearly full device takes smaller chunks instead of failing
+    for (; e == cudaSuccess && res > 0; res = std::max(res / 2, res_tile)) {
+        e = cudaMalloc((void **)&c->d_res, res);
+        if (e == cudaSuccess) {
+            c->res_bytes = res;
+            break;
+        }
+        if (e != cudaErrorMemoryAllocation || res <= res_tile) break;
+        e = cudaSuccess;
+        (void)cudaGetLastError();
+    }
     if (e != cudaSuccess || c->oz_xseg < 1) {
         c->prec_mode = EXS_PREC_FP64;
         return fail(c, e != cudaSuccess ? EXS_ERR_NOMEM : EXS_ERR_SIZE, "split-precision work space");
@@ -930,7 +943,7 @@ int enqueue_setup(exs_ctx *c, const std::vector<KDesc> &ks, const Uploaded &u, b
         const int q = c->oz_cfg;
         if (mod)
             EXS_CUDA(exs::launch_ring_ho(c->ring_cols, &c->ring_mapHO1, &c->ring_mapHO2, p, u.d_k, ks[0].oz_slot, u.d_oztiles, u.noztiles, c->oz_ring, c->kp8,
-                                         c->d_res, c->d_pace, s));
+                                         c->d_res, c->res_bytes, c->d_pace, s));
         else
             EXS_CUDA(exs::launch_oz_mma(q, &c->oz_mapA[q], (q & 8) ? &c->oz_mapB2[q] : &c->oz_mapB[q], p, u.d_k,
                                         u.d_oztiles, u.noztiles, c->oz_sch, c->kp8, s));

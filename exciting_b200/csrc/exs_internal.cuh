@@ -434,7 +434,7 @@ cudaError_t launch_ring_split(const DevParams &p, const KDesc *d_k, int nk, cons
 cudaError_t launch_ring_x(const DevParams &p, const OzAtomArgs &xa, const OzRing &rg, cudaStream_t s);
 cudaError_t launch_ring_ho(int cols, const CUtensorMap *map1, const CUtensorMap *map2, const DevParams &p,
                            const KDesc *d_k, int slot0, const void *d_tiles, int ntiles, const OzRing &rg, int kp8,
-                           uint8_t *res, int *pace, cudaStream_t s);
+                           uint8_t *res, size_t res_bytes, int *pace, cudaStream_t s);
 // slot0: the slot of the batch's first k-point (the slots of a batch follow each other)
 cudaError_t launch_ring_atom(const CUtensorMap *mapA, const CUtensorMap *mapX, const DevParams &p, const KDesc *d_k,
                              int slot0, const void *d_tiles, int ntiles, const OzRing &rg, const OzAtomArgs &xa, uint8_t *res,

@@ -1269,7 +1269,8 @@ static cudaError_t plane_grid(int ntiles, int np, cudaStream_t s, int *ncl)
     return cudaSuccess;
 }
 
-// H/O: the products of all tiles, then their recombination.  Large problems
+// H/O: the products, then their recombination, in equal chunks of tiles whose
+// residues fit the residue buffer (one chunk up to 4 GB of them).  Large problems
 // are paced: when the operand planes of one product (three arrays of npad x
 // kp8 bytes) exceed RG_PACE_BYTES, clusters that drift apart stream them from
 // HBM again and again.
@@ -1277,33 +1278,40 @@ constexpr size_t RG_PACE_BYTES = (size_t)100 << 20;
 
 template <int MODE>
 static cudaError_t launch_ho(const CUtensorMap *map, const DevParams &p, const KDesc *d_k, int slot0,
-                             const int *d_tiles, int ntiles, const OzRing &rg, int kp8, uint8_t *res, int *pace, cudaStream_t s)
+                             const int *d_tiles, int ntiles, const OzRing &rg, int kp8, uint8_t *res, size_t res_bytes,
+                             int *pace, cudaStream_t s)
 {
     using C = RingCfg<MODE>;
-    int ncl = 0;
-    cudaError_t e = plane_grid<MODE>(ntiles, 2 * rg.n, s, &ncl);
-    if (e != cudaSuccess) return e;
+    const int cap = (int)std::min<size_t>(res_bytes / ring_ho_tile_bytes(rg, C::BJ), 1 << 24);
+    if (cap < 1) return cudaErrorInvalidValue;
+    const int nchunk = (ntiles + cap - 1) / cap, chunk = (ntiles + nchunk - 1) / nchunk;
     const bool paced = (size_t)3 * p.npad * kp8 > RG_PACE_BYTES;
-    if (paced) {
-        e = cudaMemsetAsync(pace, 0, sizeof(int) * ncl, s);
+    for (int t0 = 0; t0 < ntiles; t0 += chunk) {
+        const int nt = std::min(chunk, ntiles - t0);
+        const int *tiles = d_tiles + 3 * (size_t)t0;
+        int ncl = 0;
+        cudaError_t e = plane_grid<MODE>(nt, 2 * rg.n, s, &ncl);
+        if (e == cudaSuccess && paced) e = cudaMemsetAsync(pace, 0, sizeof(int) * ncl, s);
+        if (e != cudaSuccess) return e;
+        oz_plane_kernel<MODE><<<2 * ncl, RG_THREADS, C::SMEM, s>>>(*map, *map, p, slot0, tiles, nt, rg, OzAtomArgs{}, res,
+                                                                   paced ? pace : nullptr);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        oz_crt_kernel<C::BJ><<<(unsigned)nt * (RG_BM / RC_R) * (C::BJ / RC_C), 128, 0, s>>>(p, d_k, tiles, rg, res);
+        e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    oz_plane_kernel<MODE><<<2 * ncl, RG_THREADS, C::SMEM, s>>>(*map, *map, p, slot0, d_tiles, ntiles, rg, OzAtomArgs{},
-                                                               res, paced ? pace : nullptr);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    oz_crt_kernel<C::BJ><<<(unsigned)ntiles * (RG_BM / RC_R) * (C::BJ / RC_C), 128, 0, s>>>(p, d_k, d_tiles, rg, res);
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 cudaError_t launch_ring_ho(int cols, const CUtensorMap *map1, const CUtensorMap *map2, const DevParams &p,
                            const KDesc *d_k, int slot0, const void *d_tiles, int ntiles, const OzRing &rg, int kp8,
-                           uint8_t *res, int *pace, cudaStream_t s)
+                           uint8_t *res, size_t res_bytes, int *pace, cudaStream_t s)
 {
     if (ntiles <= 0) return cudaSuccess;
     const int *t = (const int *)d_tiles;
-    return cols == 256 ? launch_ho<RG_WIDE>(map1, p, d_k, slot0, t, ntiles, rg, kp8, res, pace, s)
-                       : launch_ho<RG_HO>(map2, p, d_k, slot0, t, ntiles, rg, kp8, res, pace, s);
+    return cols == 256 ? launch_ho<RG_WIDE>(map1, p, d_k, slot0, t, ntiles, rg, kp8, res, res_bytes, pace, s)
+                       : launch_ho<RG_HO>(map2, p, d_k, slot0, t, ntiles, rg, kp8, res, res_bytes, pace, s);
 }
 
 // Per-atom products in chunks of tiles whose residues fit the residue buffer.
