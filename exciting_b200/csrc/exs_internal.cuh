@@ -55,7 +55,7 @@ struct OzAtomArgs {
     int lw;                      // window bytes per row (multiple of 128)
     int8_t *xs;                  // slices [atom][slice][block][re, im][64][lw]
     double *xsig;                // row scales [atom][block][64]
-    // moduli: rows n = h_a rows, then lo rows, in blocks of nb (a multiple of 32); planes
+    // moduli: rows n = h_a rows, then lo rows, in blocks of nb (a multiple of 16); planes
     // [atom][plane][nrows][lw] in xs, scales [atom][nrows] in xsig
     int nb, nrows;
 };

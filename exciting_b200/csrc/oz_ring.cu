@@ -302,7 +302,8 @@ __global__ void __launch_bounds__(256) oz_ring_x_kernel(DevParams p, OzAtomArgs 
 //   RG_WIDE  tiles {k, ib, jb}: 256 G_i x 256 G_j, two MMAs of N = 256 on the
 //            same A operand, one for H and one for O
 //   RG_ATOM  tiles {k, atom, ib, xb}: 256 G x nb rows of h_a and loa of one
-//            atom (N = nb, a multiple of 32), over the atom's K window
+//            atom (N = nb rounded up to 32; the rows past nb belong to the next
+//            tile), over the atom's K window
 // The work list is flat in (tile, plane): while full rounds of one tile per
 // cluster last, a cluster takes a tile and walks its 2n planes; the (tile,
 // plane) pairs of the remaining tiles are dealt out in equal shares, so that a
@@ -489,7 +490,7 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
     const uint32_t sbase = (smem_u32(rg_smem) + 1023u) & ~1023u;
     const int cl = (int)(blockIdx.x >> 1), NP = 2 * (MODE == RG_ATOM ? rg.at.n : rg.n);
     RingUnits<MODE == RG_ATOM> units(ntiles, (int)(gridDim.x >> 1), NP, cl);
-    const int N = MODE == RG_ATOM ? xa.nb : 256;         // MMA N
+    const int N = MODE == RG_ATOM ? (xa.nb + 31) / 32 * 32 : 256;         // MMA N
     const int b_rows = N / 2;                            // operand rows of a B operand in this CTA
 
     if (warp == 3) {
@@ -561,7 +562,7 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                         x0 = at.oz_x0;
                     } else {
                         slot = ias;
-                        row = tiles[4 * tile + 3] * N + (int)rank * b_rows;
+                        row = tiles[4 * tile + 3] * xa.nb + (int)rank * b_rows;
                     }
                 }
                 // planes per slot of the split operands, per atom of h_a and loa
@@ -662,14 +663,15 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
         const int row = qd * 32 + lane;
         int nq = N / 16, last = -1;                                 // 16-column chunks of an accumulator
         const uint32_t acce0[2] = {mapa_shared(smem_u32(&acce[0]), 0), mapa_shared(smem_u32(&acce[1]), 0)};
-        const size_t plane_bytes = (size_t)C::NB * N * 128;         // residues of one product, this CTA's 128 rows
+        // residues of one product, this CTA's 128 rows
+        const size_t plane_bytes = (size_t)(MODE == RG_ATOM ? xa.nb : C::NB * N) * 128;
         bool bad = false;
         for (int u = 0; u < units.count && !bad; u++, units.next()) {
             const int P = units.P, m = P >> 1;
             if (MODE == RG_ATOM && units.tile != last) {            // only the chunks that hold rows of the atom
                 last = units.tile;
                 const AtomDesc &at = p.atoms[tiles[4 * last + 1]];
-                nq = min(N, at.napw + at.losize - tiles[4 * last + 3] * N + 15) / 16;
+                nq = min(xa.nb, at.napw + at.losize - tiles[4 * last + 3] * xa.nb + 15) / 16;
             }
             const int pm = rg.p[m], mg = rg.mg[m], up = rg.up[m];
             const uint32_t mf = rg.mf[m];
@@ -1199,12 +1201,14 @@ size_t ring_atom_tile_bytes(const OzRing &rg, int nb) { return (size_t)2 * rg.at
 size_t ring_pace_bytes() { return sizeof(int) * RG_PACE_MAX; }
 
 // Row blocks of the per-atom tiles: rows (h_a rows and lo rows of the largest
-// species) in equal blocks of nb <= 256, a multiple of 32 (the MMA's N).
+// species) in as few blocks of nb <= 256 rows as hold them, nb a multiple of 16.
+// (In multiples of the MMA's 32 the 269 rows of the eight-atom cell went 160 + 109:
+// every other cluster had the long tiles, and the two that share A drifted apart.)
 void ring_row_blocks(int rows, int *nb, int *nrows)
 {
     const int blocks = (rows + 255) / 256;
-    *nb = ((rows + blocks - 1) / blocks + 31) / 32 * 32;
-    *nrows = blocks * *nb;
+    *nb = ((rows + blocks - 1) / blocks + 15) / 16 * 16;
+    *nrows = (blocks * *nb + 31) / 32 * 32;
 }
 
 size_t ring_part_rows(int natmtot, int nrows) { return (size_t)natmtot * (nrows / RC_C); }
@@ -1346,7 +1350,7 @@ cudaError_t launch_ring_atom(const CUtensorMap *mapA, const CUtensorMap *mapX, c
 //         128, 1, 1}: a K chunk starting at any multiple of 16 bytes (the atom
 //         windows are not chunk aligned)
 //   x     the per-atom operands as 4D (K byte in a chunk, row, atom x plane,
-//         K chunk), box {128, nb / 2, 1, 1}
+//         K chunk), box {128, N / 2, 1, 1}, N = nb rounded up to 32
 // Rows past npad (or past the rows of X) and K chunks past kp8 arrive as zeros.
 bool make_ring_maps(void *base, size_t nsp, int npad, int kp8, int narr, void *xbase, size_t xgroups, int nrows,
                     int nb, int lw, CUtensorMap *ho1, CUtensorMap *ho2, CUtensorMap *arow, CUtensorMap *x)
@@ -1359,7 +1363,7 @@ bool make_ring_maps(void *base, size_t nsp, int npad, int kp8, int narr, void *x
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess || !fn)
         return false;
     EncodeFn encode = (EncodeFn)fn;
-    if (kp8 % RG_CHUNK != 0 || lw % RG_CHUNK != 0 || nb % 32 != 0) return false;
+    if (kp8 % RG_CHUNK != 0 || lw % RG_CHUNK != 0 || nb % 16 != 0) return false;
     const cuuint32_t es[5] = {1, 1, 1, 1, 1};
     auto make = [&](CUtensorMap *m, int rank, void *b, const cuuint64_t *dims, const cuuint64_t *strides,
                     const cuuint32_t *box) {
@@ -1374,7 +1378,7 @@ bool make_ring_maps(void *base, size_t nsp, int npad, int kp8, int narr, void *x
     const cuuint32_t bar[4] = {RG_CHUNK, 128, 1, 1};
     const cuuint64_t L = lw, R = nrows;
     const cuuint64_t dx[4] = {RG_CHUNK, R, xgroups, L / RG_CHUNK}, sx[3] = {L, R * L, RG_CHUNK};
-    const cuuint32_t bx[4] = {RG_CHUNK, (cuuint32_t)(nb / 2), 1, 1};
+    const cuuint32_t bx[4] = {RG_CHUNK, (cuuint32_t)((nb + 31) / 32 * 16), 1, 1};
     return make(ho1, 5, base, dho, sho, bho1) && make(ho2, 5, base, dho, sho, bho2) &&
            make(arow, 4, base, dar, sar, bar) && make(x, 4, xbase, dx, sx, bx);
 }
