@@ -21,6 +21,7 @@ from __future__ import annotations
 
 import argparse
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -178,107 +179,93 @@ def _hbm_peak():
         return 6650.0      # earlier measurement on this pool's B200s
 
 
+# The moduli the products run in (pairwise coprime, every prime factor 1 mod 4: two int8 products per
+# modulus make a complex one), largest first; the fewest that hold products of 2 b bits with one bit of margin.
+RINGS = (241, 233, 229, 221, 205, 197, 193, 181, 173, 157, 149, 137, 113, 109, 101, 97)
+
+
+def rings_for(bits):
+    lm, n = 0.0, 0
+    while lm - 1e-9 < bits + 2:
+        lm += math.log2(RINGS[n])
+        n += 1
+    return n
+
+
 def split_scheme(args, sys_):
-    """(int8 planes per operand, int8 products per output tile, dtype text,
+    """(int8 planes per operand, int8 products per H/O tile, dtype text,
     precision text) of the split-precision mode args.precision."""
     if args.precision == "ozaki":
         S = args.slices
         return (S, S * (S + 1) // 2, "i8 slices, f64 recombination",
                 "split int8 x%d slices (tcgen05), FP64 recombination" % S)
     from exciting_b200.fvsystem import ozaki_moduli
-    K = sum(sys_.basis.napw_atom(a) for a in range(sys_.natmtot))
-    ps, _, b, bx, h = ozaki_moduli(args.moduli, K, sys_.basis.maxaa)
-    n = len(ps)
-    return (n, n, "i8 residues mod %d coprime moduli, CRT in 64-bit fixed point, f64 scaling" % n,
-            "split int8, residues modulo %d moduli (columns scaled by their 2-norms to %d bits, %d headroom bits "
-            "in the 64-bit recombination; tcgen05), Chinese-remainder recombination" % (n, b, h))
+    K = apw_rows(sys_)
+    ps, _, b, bx, _ = ozaki_moduli(args.moduli, K, sys_.basis.maxaa)
+    r = rings_for(2 * b)
+    return (2 * r, 2 * r, "i8 residues mod %d coprime moduli, CRT in 96-bit fixed point, f64 scaling" % r,
+            "split int8 (the %d-modulus plan: columns scaled by their 2-norms to %d bits, exact integer products "
+            "modulo %d moduli, two per modulus; tcgen05), Chinese-remainder recombination" % (len(ps), b, r))
 
 
-def ozaki_tiles128(g, cols=64):
-    """128-row upper residue tiles of one k-point (128 x cols)."""
-    n = g.ngp
-    return sum(1 for ib in range((n + 127) // 128) for jb in range((n + cols - 1) // cols)
-               if jb * cols + cols - 1 >= ib * 128)
+def apw_rows(sys_):
+    return sum(sys_.basis.napw_atom(a) for a in range(sys_.natmtot))
 
 
-def residue_bytes(sys_, g, moduli):
-    """Algorithmic DRAM bytes of the residue kernel for one k-point: the
-    residues of Ar, Ai, Br, Bi (npad rows x kp8 bytes per modulus) read once
-    and the residues of the four H/O values written once (128 x 64 bytes per
-    value, tile and modulus)."""
-    K = sum(sys_.basis.napw_atom(a) for a in range(sys_.natmtot))
-    kp8 = (K + 255) // 256 * 256
+def ho_cols(precision, K):
+    """Columns of the H/O tiles: 256 x 128 with moduli (256 x 256 above K = 8192), 128 x 32 with slices."""
+    return 32 if precision != "ozaki_mod" else (256 if K > 8192 else 128)
+
+
+def ho_tiles(n, rows, cols):
+    return sum(1 for ib in range((n + rows - 1) // rows) for jb in range((n + cols - 1) // cols)
+               if jb * cols + cols - 1 >= ib * rows)
+
+
+def residue_bytes(sys_, g, planes):
+    """Algorithmic DRAM bytes of the product kernel for one k-point: `planes`
+    residue planes of A and of B (npad rows x K bytes) read once, and as many
+    residues of every H and O element of the upper tiles written once."""
+    K = apw_rows(sys_)
+    cols = ho_cols("ozaki_mod", K)
     npad = (g.ngp + 63) // 64 * 64
-    return 4.0 * moduli * npad * kp8 + 4.0 * moduli * 128 * 64 * ozaki_tiles128(g)
+    return 2.0 * planes * npad * ((K + 127) // 128 * 128) + 2.0 * planes * 256 * cols * ho_tiles(g.ngp, 256, cols)
 
 
-def ozaki_int8_ops(sys_, gks, products, cols=32):
-    """int8 MMA operations the split-precision H/O kernel issues: per 128 x
-    cols tile (B operand [Br|Bi|Ar|Ai] -> N = 4 cols), `products` int8
-    products (S(S+1)/2 slice pairs, or one per modulus) x two A operands
-    (Ar, Ai) x 2 x 128 x N x kp8 (K padded to 256)."""
-    K = sum(sys_.basis.napw_atom(a) for a in range(sys_.natmtot))
-    kp8 = (K + 255) // 256 * 256
-    tiles = 0
-    for g in gks:
-        n = g.ngp
-        for ib in range((n + 127) // 128):
-            for jb in range((n + cols - 1) // cols):
-                if jb * cols + cols - 1 >= ib * 128:
-                    tiles += 1
-    return tiles * products * 2.0 * 2 * 128 * (4 * cols) * kp8
-
-
-HO_KERNEL = {"ozaki_mod": "oz_res_kernel (residue tiles, tcgen05.mma kind::i8) + oz_crt_kernel (96-bit CRT), "
-                          "MT contraction phase",
-             "ozaki": "oz_mma_kernel (tcgen05.mma kind::i8, FP64 fold), MT contraction phase"}
-
-
-def ho_kernel(precision, kernel_config):
-    if precision == "ozaki_mod" and kernel_config >= 0 and (kernel_config & 8):
-        how = "persistent paced clusters, " if kernel_config & 2 else ""
-        return HO_KERNEL[precision].replace("oz_res_kernel (residue tiles", "oz_res2_kernel (256 x 64 residue tiles "
-                                            "on SM pairs, %stcgen05.mma.cta_group::2" % how)
-    return HO_KERNEL[precision]
-
-
-def ho_tile_cols(precision, kernel_config):
-    """Columns of the H/O tiles: 64 or 32 for the modular residue tiles
-    (configuration bit 0; the two-SM tiles of bit 3 are 64 wide), 32 for the
-    slice kernel.  The operation count is that of the 128-row tiles either
-    way: the two-SM tiles' extra tiles below the diagonal are not counted."""
+def int8_ops(sys_, gks, precision, products):
+    """int8 MMA operations the split-precision H/O kernel issues.  Moduli: per
+    256 x cols tile and product one M = 256, N = 2 cols MMA (H and O) over K
+    padded to 32.  Slices: per 128 x 32 tile (B operand [Br|Bi|Ar|Ai], N =
+    128) and slice pair two A operands, K padded to 256."""
+    K = apw_rows(sys_)
+    cols = ho_cols(precision, K)
     if precision == "ozaki_mod":
-        return 32 if (kernel_config & 1) and not (kernel_config & 8) else 64
-    return 32
+        return sum(ho_tiles(g.ngp, 256, cols) for g in gks) * products * 2.0 * 256 * 2 * cols * ((K + 31) // 32 * 32)
+    return sum(ho_tiles(g.ngp, 128, cols) for g in gks) * products * 2.0 * 2 * 128 * 4 * cols * ((K + 255) // 256 * 256)
 
+
+HO_KERNEL = {"ozaki_mod": "oz_plane_kernel (256-row tiles on SM pairs, tcgen05.mma.cta_group::2 kind::i8) + "
+                          "oz_crt_kernel (96-bit CRT), MT contraction phase",
+             "ozaki": "oz_mma_kernel (tcgen05.mma kind::i8, FP64 fold), MT contraction phase"}
 
 # DRAM bytes of the dominant kernel, from ncu captures (dram__bytes_read.sum +
 # dram__bytes_write.sum) of the same kernels; a kernel change needs a new
-# capture.  The 8-atom batch, per k-point (a 2 k-point capture divided by 2;
-# the traffic grows with the k-points: each k-point's operands are read once
-# and its H/O written once):
-#   slices, oz_mma_kernel<OZ_HO,2,2>, 7 slices: 131.6 MB read + 35.2 MB written;
-#   moduli, oz_res_kernel<64> (configurations without bit 3): 218.4 MB read +
-#     47.4 MB written; oz_res2_kernel<64> (bit 3): 253.9 MB + 56.9 MB;
+# capture.  The 8-atom batch, per k-point:
+#   moduli, oz_plane_kernel<0>, 27 k-points: 4.77 GB read + 0.98 GB written;
+#   slices, oz_mma_kernel<OZ_HO,2,2>, 7 slices, 2 k-points: 131.6 MB + 35.2 MB;
 #   FP64, zgemm_dmma_kernel<1> + <2>, 6 k-points: 673.5 MB read + 143.1 MB written.
-# The 216-atom cell, per k-point (one launch, captured at full size in one
-# pass): oz_res2_kernel<64> in configuration 10 (paced persistent pairs),
-# 1.23 TB read + 19.6 GB written; configuration 8, 4.61 TB + 19.9 GB.
+# The 216-atom cell, per k-point (the chunks of one setup, captured at full
+# size in one pass): oz_plane_kernel<2>, 832.7 GB read + 21.2 GB written.
 PROFILED_DRAM_BYTES_PER_K = {"ozaki": (131.6e6 + 35.2e6) / 2, "fp64": (673.5e6 + 143.1e6) / 6,
-                             "ozaki_mod": (218.4e6 + 47.4e6) / 2, "ozaki_mod_pairs": (253.9e6 + 56.9e6) / 2}
-PROFILED_DRAM_BYTES_216 = {10: 1.23e12 + 19.6e9, 8: 4.61e12 + 19.9e9}
-
-
-def profiled_traffic_per_k(precision, kernel_config):
-    if precision == "ozaki_mod" and kernel_config >= 0 and (kernel_config & 8):
-        return PROFILED_DRAM_BYTES_PER_K["ozaki_mod_pairs"]
-    return PROFILED_DRAM_BYTES_PER_K[precision]
+                             "ozaki_mod": (4.77e9 + 0.98e9) / 27}
+PROFILED_DRAM_BYTES_216 = 832.7e9 + 21.2e9
 
 
 def main_bytes(sys_, gks, precision, slices):
     """Algorithmic DRAM bytes of the MT contraction launch(es): operands read
-    once (int8 slices or residues of Ar, Ai, Br, Bi, `slices` planes each; or
-    the FP64 A and B planes) and the N x N block of H and O written once."""
+    once (int8 slices of Ar, Ai, Br, Bi, `slices` planes each; residues of A
+    and B, `slices` planes each; or the FP64 A and B planes) and the N x N
+    block of H and O written once."""
     K = sum(sys_.basis.napw_atom(a) for a in range(sys_.natmtot))
     total = 0.0
     for g in gks:
@@ -286,7 +273,7 @@ def main_bytes(sys_, gks, precision, slices):
         npad = (n + 63) // 64 * 64
         if precision != "fp64":
             kp8 = (K + 255) // 256 * 256
-            total += 4.0 * slices * npad * kp8
+            total += (2.0 if precision == "ozaki_mod" else 4.0) * slices * npad * kp8
         else:
             total += 4.0 * 8 * K * npad
         total += 2.0 * 16 * n * n
@@ -384,13 +371,32 @@ def run_reference(args):
     return 0
 
 
-def launches_per_setup(precision):
-    """Kernel launches of one batched setup call: match, (modular: the A column
-    norms), the A split, the per-atom products, (modular: the B column norms),
-    the B split, the H/O tiles (modular: residue tiles, then their
-    recombination), the O APW-lo block and the lo-lo blocks; the FP64 path:
-    match, four grouped DMMA products, APW-lo and lo-lo."""
-    return 10 if precision == "ozaki_mod" else 7
+def launches_per_setup(precision, sys_=None, ngp=(), planes=0):
+    """Kernel launches of one batched setup call.  Moduli: match, the column
+    norms and residues of A, the per-atom products and their recombination, the
+    norms and residues of B, the H/O products and their recombination, the
+    local-orbital blocks; the products in chunks of at most 4 GB of residues
+    (sys_, ngp, planes: more than one for the 216-atom cell).  Slices: match, the
+    A split, the per-atom products, the B split, the H/O tiles, the blocks.
+    FP64: match, h_a A, the APW-lo rows, H and O, the blocks."""
+    if precision != "ozaki_mod":
+        return 6 if precision == "ozaki" else 5
+    chunks = [1, 1]
+    if sys_ is not None:
+        K = apw_rows(sys_)
+        cols = ho_cols(precision, K)
+        b = sys_.basis
+        rows = [b.napw_atom(a) + sum(2 * l + 1 for l in b.lorbl[b.atom_species[a]]) for a in range(sys_.natmtot)]
+        blocks = (max(rows) + 255) // 256
+        nb = ((max(rows) + blocks - 1) // blocks + 15) // 16 * 16
+        at_planes = planes - 2 if planes == 28 else planes                     # 13 of the 14 moduli at b = 49, bx = 45
+        tile = [planes * 512 * cols, at_planes * 256 * nb]
+        n = [sum(ho_tiles(g, 256, cols) for g in ngp),
+             sum((g + 255) // 256 for g in ngp) * sum((r + nb - 1) // nb for r in rows)]
+        top = len(ngp) * ho_tiles(max(ngp), 256, cols)                         # the buffer is sized for ngkmax
+        res = min(4 << 30, max(top * tile[0], min(256 << 20, n[1] * tile[1])))
+        chunks = [-(-n[q] // (res // tile[q])) for q in range(2)]
+    return 6 + 2 * chunks[0] + 2 * chunks[1]
 
 
 def _e2e(args, st, stream, ig, vg, ngp, nmat, ws, barrier, mode="auto", pinned=True):
@@ -615,6 +621,7 @@ def run_ours(args, emit=True):
     gks = s.gksets()[: args.nk]
     nk = len(gks)
     st = Setup(s, max_batch=nk)
+    planes = 0
     if args.precision != "fp64":
         st.set_precision(args.precision, args.slices if args.precision == "ozaki" else args.moduli)
         planes, products, dtype_text, prec_text = split_scheme(args, s)
@@ -804,15 +811,15 @@ def run_ours(args, emit=True):
         peak64 = _measured_fp64_peak(torch)
         achieved = fl / (main_ms * 1e-3) / 1e12
         if args.precision != "fp64":
-            ops = ozaki_int8_ops(s, gks, products, ho_tile_cols(args.precision, tuned))
+            ops = int8_ops(s, gks, args.precision, products)
             peak8 = _measured_int8_peak(torch)
             a8 = ops / (main_ms * 1e-3) / 1e12
-            roof = {"bound": "tensor", "kernel": ho_kernel(args.precision, tuned),
+            roof = {"bound": "tensor", "kernel": HO_KERNEL[args.precision],
                     "achieved": a8, "peak": peak8, "unit": "TOP/s (int8)", "frac": a8 / peak8,
                     "peak_source": "cuBLASLt int8 GEMM 8192^3 (torch._int_mm) measured in this run",
-                    "int8_ops_per_step": ops, "traffic": profiled_traffic_per_k(args.precision, tuned) * nk,
-                    "traffic_note": "bytes per launch: ncu dram__bytes_read+write of a 2 k-point capture scaled "
-                                    "by k-points; algorithmic %.3g" % main_bytes(s, gks, args.precision, planes),
+                    "int8_ops_per_step": ops, "traffic": PROFILED_DRAM_BYTES_PER_K[args.precision] * nk,
+                    "traffic_note": "bytes per launch: ncu dram__bytes_read+write of a capture scaled by "
+                                    "k-points; algorithmic %.3g" % main_bytes(s, gks, args.precision, planes),
                     "fp64_equivalent": {"achieved": achieved, "peak": peak64, "unit": "TFLOP/s",
                                         "frac": achieved / peak64,
                                         "peak_source": "cuBLAS DGEMM 8192^3 measured in this run"}}
@@ -862,7 +869,7 @@ def run_ours(args, emit=True):
                 "sample": f"{cpu_n} k-points of the 27-k set in {cpu_dt:.1f} s by the FP64 CPU "
                           "restatement (C + OpenMP + OpenBLAS zgemm)"},
             "clocks": clocks,
-            "gpu_launches": launches_per_setup(args.precision) * args.steps,
+            "gpu_launches": launches_per_setup(args.precision, s, ngp, planes) * args.steps,
             "setup_flops_per_step": setup_flops(s, gks),
             "accuracy": accuracy,
             "fp64_path_value": fp64_value,
@@ -1206,8 +1213,7 @@ def run_large(args):
     args.precision = prec
     if args.kernel_config >= 0:
         st.set_kernel_config(args.kernel_config)
-    # the library's default until a configuration is chosen: paced persistent two-SM residue tiles with moduli
-    kcfg = args.kernel_config if args.kernel_config >= 0 else (10 if prec == "ozaki_mod" else 0)
+    kcfg = max(args.kernel_config, 0)                       # the library's default until one is chosen: 0
     planes, products, dtype_text, prec_text = split_scheme(args, s)
     ms, phase, rows = timed(args.steps, args.warmup, True)
     value = ws * args.steps / (ms * 1e-3)
@@ -1337,7 +1343,7 @@ def run_large(args):
     if ws > 1:
         dist.barrier()
     if rank == 0:
-        ops = ozaki_int8_ops(s, gks_all, products, ho_tile_cols(prec, kcfg)) / len(gks_all)   # per k-point
+        ops = int8_ops(s, gks_all, prec, products) / len(gks_all)   # per k-point
         fl = main_flops(s, gks_all) / len(gks_all)
         peak8 = _measured_int8_peak(torch)
         peak8s, clk8s = _measured_int8_sustained(torch)
@@ -1375,26 +1381,26 @@ def run_large(args):
                        "ngp": [min(g.ngp for g in gks_all), max(g.ngp for g in gks_all)],
                        "nmat": [min(g.ngp for g in gks_all) + nlotot, max(g.ngp for g in gks_all) + nlotot],
                        "precision": prec_text, "kernel_config": kcfg,
-                       "l2": "working set (A/B planes 30 GB, %d int8 planes of 4 arrays, H/O 27 GB) far above "
-                             "L2, no flush" % planes},
+                       "l2": "working set (A/B planes 30 GB, %d int8 planes of %d arrays, H/O 27 GB) far above "
+                             "L2, no flush" % (planes, 2 if prec == "ozaki_mod" else 4)},
             "e2e": e2e,
             "phases_ms_per_step": {"match": phase[0], "h_a_A": phase[1], "mt_contraction": phase[2],
                                    "lo_blocks": phase[3], "total": phase[4]},
-            "roofline": {"bound": "tensor", "kernel": ho_kernel(prec, kcfg),
+            "roofline": {"bound": "tensor", "kernel": HO_KERNEL[prec],
                          "achieved": a8, "peak": peak8s, "unit": "TOP/s (int8)", "frac": a8 / peak8s,
                          "peak_source": "cuBLASLt int8 GEMM 8192^3 (torch._int_mm) back to back for 4 s in this "
                                         "run (sustained, under the power cap: the H/O kernel runs for seconds)",
                          "peak_burst": peak8, "frac_of_burst": a8 / peak8, "peak_sustained_clocks": clk8s,
                          **_int8_from_bf16_peaks(a8),
-                         "int8_ops_per_step": ops, "traffic": PROFILED_DRAM_BYTES_216.get(kcfg),
-                         "traffic_note": "bytes per launch of the residue kernel: ncu dram__bytes_read+write of "
-                                         "one full-size launch (one pass); algorithmic %.3g (residue planes read "
+                         "int8_ops_per_step": ops, "traffic": PROFILED_DRAM_BYTES_216 if prec == "ozaki_mod" else None,
+                         "traffic_note": "bytes per k-point of the product kernel: ncu dram__bytes_read+write of "
+                                         "the launches of one setup (one pass); algorithmic %.3g (residue planes read "
                                          "once, residues written once)" % residue_bytes(s, gks_all[0], planes),
                          "fp64_equivalent": {"achieved": fl / (mt_ms * 1e-3) / 1e12, "peak": peak64,
                                              "unit": "TFLOP/s", "frac": fl / (mt_ms * 1e-3) / 1e12 / peak64}},
             "cpu_baseline": cpu,
             "clocks": clocks,
-            "gpu_launches": launches_per_setup(prec) * args.steps,
+            "gpu_launches": launches_per_setup(prec, s, [gks_all[0].ngp], planes) * args.steps,
             "setup_flops_per_step": setup_flops(s, gks_all) / len(gks_all),
             "accuracy": acc,
             "fp64_path_value": fp64_value,

@@ -431,7 +431,7 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
     // k-point), at most RES_MAX of them at a time; the per-atom products run before them in the same
     // buffer, in chunks of at least 256 MB where there is that much.  RES_MAX: the 64-atom cell and the
     // batches of the eight-atom cell (up to 2.0 GB) run in one chunk; one k-point of 216 atoms would take
-    // 21 GB, beside 85 GB of operands, and takes six chunks of ~90 ms instead
+    // 21 GB, beside 85 GB of operands, and takes five chunks of ~0.1 s instead
     constexpr size_t RES_MAX = (size_t)4 << 30;
     size_t res = 0, res_tile = 0;
     if (mod) {

@@ -141,12 +141,13 @@ struct KDesc {
     double *ar, *ai;         // A planes  [Kpad][npad]
     double *br, *bi;         // B = blockdiag(h_a) A planes
     double *cr, *ci;         // (I + h1) A planes (iora* only) else == ar/ai
-    int8_t *oz_slices;       // split-precision path: int8 slices of this slot [S][4 arrays][npad][kp8]
-    double *oz_scale;        // split-precision path: column bounds of A and B [2][npad] (maxima with slices,
+    int8_t *oz_slices;       // split-precision path: this slot's slices [S][4 or 6 arrays][npad][kp8], or residues
+                             // [plane][2 or 3 arrays][npad][kp8]
+    double *oz_scale;        // split-precision path: column bounds of A, B and C [3][npad] (maxima with slices,
                              // 2-norms with moduli; the scale is the power of two above; null: FP64 path)
     double *oz_part;         // moduli: sums of squares of the A columns per atom, then of the B columns per 16
                              // rows of an atom [rows][npad]; else null
-    int oz_slot;             // split-precision path: slot index in the slice tensor maps
+    int oz_slot;             // split-precision path: slot index in the tensor maps
 };
 
 // Column scale sigma(G) = 2^e with m < 2^e (frexp) for the column bound m in

@@ -329,8 +329,8 @@ __global__ void __launch_bounds__(256) oz_ring_x_kernel(DevParams p, OzAtomArgs 
 // 10,368: 13.9 - 14.6 ms from box to box, 2.8 POP/s, the SM clock down to
 // 1.5 GHz; the form with real and imaginary planes, 13 moduli and 256 x 64
 // tiles took 23.1 ms); HBM for the per-atom products (64 atoms 1.25 ms, the 27
-// k-points of the eight-atom cell 0.95 ms at about 4.5 TB/s of residues out
-// and operands in).  H/O of the 27 k-points 1.46 - 1.57 ms (was 2.65).
+// k-points of the eight-atom cell 0.89 ms at about 4 TB/s of residues out
+// and operands in).  H/O of the 27 k-points 1.5 - 1.6 ms (was 2.65).
 enum : int { RG_HO = 0, RG_ATOM = 1, RG_WIDE = 2 };
 
 template <int MODE>
