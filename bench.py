@@ -394,7 +394,7 @@ def launches_per_setup(precision, sys_=None, ngp=(), planes=0):
         n = [sum(ho_tiles(g, 256, cols) for g in ngp),
              sum((g + 255) // 256 for g in ngp) * sum((r + nb - 1) // nb for r in rows)]
         top = len(ngp) * ho_tiles(max(ngp), 256, cols)                         # the buffer is sized for ngkmax
-        res = min(4 << 30, max(top * tile[0], min(256 << 20, n[1] * tile[1])))
+        res = min(4 << 30, max(top * tile[0], min(512 << 20, n[1] * tile[1])))
         chunks = [-(-n[q] // (res // tile[q])) for q in range(2)]
     return 6 + 2 * chunks[0] + 2 * chunks[1]
 

@@ -429,7 +429,8 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
     const size_t nxsig = (size_t)c->natmtot * (mod ? c->ring_nrows : c->oz_nxb * 64);
     // moduli: the residues of the H/O products of a whole batch (the upper tiles of ngkmax G+k per
     // k-point), at most RES_MAX of them at a time; the per-atom products run before them in the same
-    // buffer, in chunks of at least 256 MB where there is that much.  RES_MAX: the 64-atom cell and the
+    // buffer, in chunks of at least 512 MB where there is that much (three k-points of 16 atoms: one chunk,
+    // 0.58 ms, instead of two of 370 and 80 MB, 0.60).  RES_MAX: the 64-atom cell and the
     // batches of the eight-atom cell (up to 2.0 GB) run in one chunk; one k-point of 216 atoms would take
     // 21 GB, beside 85 GB of operands, and takes five chunks of ~0.1 s instead
     constexpr size_t RES_MAX = (size_t)4 << 30;
@@ -445,7 +446,7 @@ int exs_set_precision(exs_ctx *c, int mode, int slices)
         const size_t ho = exs::ring_ho_tile_bytes(ring, cols), at = exs::ring_atom_tile_bytes(ring, c->ring_nb);
         res_tile = std::max(ho, at);
         res = std::min(RES_MAX, std::max(tiles * ho * c->max_batch,
-                                         std::min((size_t)256 << 20, atiles * at * c->max_batch)));
+                                         std::min((size_t)512 << 20, atiles * at * c->max_batch)));
         res = std::max(res, res_tile);
     }
     cudaError_t e = cudaMalloc((void **)&c->d_oz, slot * c->max_batch);
