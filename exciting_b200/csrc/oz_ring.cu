@@ -321,9 +321,10 @@ __global__ void __launch_bounds__(256) oz_ring_x_kernel(DevParams p, OzAtomArgs 
 // where the reduction of a short product is a chain of latencies.)
 // CTA 0's full barriers count the bytes of both CTAs' copies; MMA completion
 // is committed to both CTAs; both epilogues report to CTA 0's barrier.
-// Every wait is bounded and gives up when another role of the CTA gave up;
-// the kernel then lets its copies and MMAs drain, records DEV_ERR_TIMEOUT,
-// frees tensor memory and returns.
+// Every wait is bounded and gives up when another role of the CTA gave up.
+// The issuer always waits for its last MMAs; once all roles are out, a CTA in
+// which one gave up records DEV_ERR_TIMEOUT and lets its copies land, then
+// tensor memory is freed.
 //
 // What bounds it: the power cap while K is long (64 atoms, N = 8075, K =
 // 10,368: 13.9 - 14.6 ms from box to box, 2.8 POP/s, the SM clock down to
@@ -594,14 +595,6 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                 }
             }
             if (pacer) st_relaxed_gpu(pace + cl, 0x7fffffff);     // done: nobody waits for this cluster
-            // copies already issued (both CTAs') must land before the pair goes away: CTA 0 waits on its full
-            // barriers, CTA 1, whose copies signal CTA 0's barriers, lets far more than their time pass
-            if (bad && rank == 0)
-                for (int q = 0; q < NST; q++)
-                    if (fills[q] > 0) mbar_drain(&full[q], (fills[q] - 1) & 1);
-            if (bad && rank == 1)
-                for (const long long t0 = clock64(); clock64() - t0 < 1000000;) {
-                }
         }
     } else if (warp == 3) {
         // ------------------------------------------------ MMA issuer (CTA 0)
@@ -633,6 +626,10 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                         // the epilogues of both CTAs must have read this accumulator's previous product
                         if (k0 == 0 && use > 0 && !mbar_wait_ab(&acce[buf + o], (use - 1) & 1, abort, rg.wait)) {
                             bad = true;
+                            if (o > 0) {             // H's MMAs of this stage are under way: commit them too
+                                umma_commit_2sm(&empty[st]);
+                                uses[st]++;
+                            }
                             break;
                         }
                         tc_fence_after();
@@ -653,9 +650,9 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
                 }
                 if (!C::WIDE && !bad) umma_commit_2sm(&accf[buf]);
             }
-            if (bad)
-                for (int q = 0; q < NST; q++)
-                    if (uses[q] > 0) mbar_drain(&empty[q], (uses[q] - 1) & 1);
+            // every MMA is done before the pair may go away, also when only an epilogue gave up
+            for (int q = 0; q < NST; q++)
+                if (uses[q] > 0) mbar_drain(&empty[q], (uses[q] - 1) & 1);
         }
     } else if (warp >= 4) {
         // ------------------------------------------------ epilogue (both CTAs, warps 4..19)
@@ -718,9 +715,12 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
             }
         }
     }
-    if (tid == 0 && *abort) atomicOr(p.err, DEV_ERR_TIMEOUT);
     tc_fence_before();
-    __syncthreads();
+    __syncthreads();                     // every role is out: the flag is final
+    if (*abort) {                        // if CTA 0's issuer gave up, CTA 1's epilogue misses a product and does too
+        if (tid == 0) atomicOr(p.err, DEV_ERR_TIMEOUT);
+        abort_settle();
+    }
     cluster_sync_all();                  // neither CTA leaves while the pair still uses its memory
     if (warp == 3) {
         tc_fence_after();

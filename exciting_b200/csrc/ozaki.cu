@@ -523,9 +523,6 @@ oz_mma_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
                         }
                     }
             }
-            if (bad)   // copies already issued must land before the CTA goes away
-                for (int q = 0; q < NST; q++)
-                    if (fills[q] > 0) mbar_drain(&full[q], (fills[q] - 1) & 1);
         }
     } else if (warp == 3) {
         // ------------------------------------------------ MMA issuer
@@ -577,9 +574,9 @@ oz_mma_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
                         }
                     }
             }
-            if (bad)   // MMAs already issued must finish before tensor memory is freed
-                for (int q = 0; q < NST; q++)
-                    if (uses[q] > 0) mbar_drain(&empty[q], (uses[q] - 1) & 1);
+            // every MMA is done before tensor memory is freed, also when only an epilogue gave up
+            for (int q = 0; q < NST; q++)
+                if (uses[q] > 0) mbar_drain(&empty[q], (uses[q] - 1) & 1);
         }
     } else {
         // ------------------------------------------------ epilogue (warps 4..11)
@@ -692,9 +689,12 @@ oz_mma_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
             tc_fence_before();
         }
     }
-    if (tid == 0 && *abort) atomicOr(p.err, DEV_ERR_TIMEOUT);
     tc_fence_before();
-    __syncthreads();
+    __syncthreads();                     // every role is out: the flag is final
+    if (*abort) {
+        if (tid == 0) atomicOr(p.err, DEV_ERR_TIMEOUT);
+        abort_settle();
+    }
     if (warp == 3) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tbase), "r"(OZ_TMEM_COLS));
@@ -787,11 +787,6 @@ oz_mma2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                         st = (st + 1 == NST) ? 0 : st + 1;
                     }
                 }
-            // CTA 0: copies already issued (both CTAs') must land before the pair goes away;
-            // CTA 1 stopped issuing at least one bounded wait ago
-            if (bad && rank == 0)
-                for (int q = 0; q < NST; q++)
-                    if (fills[q] > 0) mbar_drain(&full[q], (fills[q] - 1) & 1);
         }
     } else if (warp == 3) {
         // ------------------------------------------------ MMA issuer (CTA 0)
@@ -839,9 +834,9 @@ oz_mma2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                         nseg++;
                     }
                 }
-            if (bad)
-                for (int q = 0; q < NST; q++)
-                    if (uses[q] > 0) mbar_drain(&empty[q], (uses[q] - 1) & 1);
+            // every MMA is done before the pair may go away, also when only an epilogue gave up
+            for (int q = 0; q < NST; q++)
+                if (uses[q] > 0) mbar_drain(&empty[q], (uses[q] - 1) & 1);
         }
     } else if (warp >= 4) {
         // ------------------------------------------------ epilogue (both CTAs, warps 4..11)
@@ -896,9 +891,12 @@ oz_mma2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         if (__all_sync(0xffffffffu, mbar_wait_ab(&stg, 0, abort, sch.wait) && !*abort))
             oz_store_mirror(kd, i0, j0, mirror, warp - 4, lane);
     }
-    if (tid == 0 && *abort) atomicOr(p.err, DEV_ERR_TIMEOUT);
     tc_fence_before();
-    __syncthreads();
+    __syncthreads();                     // every role is out: the flag is final
+    if (*abort) {
+        if (tid == 0) atomicOr(p.err, DEV_ERR_TIMEOUT);
+        abort_settle();
+    }
     cluster_sync_all();                  // neither CTA leaves while the pair still uses its memory
     if (warp == 3) {
         tc_fence_after();

@@ -61,11 +61,22 @@ __device__ __forceinline__ bool mbar_wait_ab(uint64_t *bar, uint32_t parity, vol
     }
 }
 
-// Bounded wait used while draining after an abort.
+// Bounded wait of an MMA issuer for the last commit of a stage, on its way out.
 __device__ __forceinline__ void mbar_drain(uint64_t *bar, uint32_t parity)
 {
     const long long t0 = clock64();
     while (!mbar_try(bar, parity) && clock64() - t0 < OZ_WAIT_CYCLES) {
+    }
+}
+
+// After a role gave up, copies that no MMA waited for may still be landing in
+// this CTA's shared memory.  Their barriers cannot tell (the producers stopped
+// at different fills, so a phase may never complete): the CTA stays for some
+// hundred times a copy's latency instead.
+constexpr long long OZ_SETTLE_CYCLES = 2000000LL;    // ~1 ms
+__device__ __forceinline__ void abort_settle()
+{
+    for (const long long t0 = clock64(); clock64() - t0 < OZ_SETTLE_CYCLES;) {
     }
 }
 
