@@ -536,6 +536,7 @@ int exs_set_scf_inputs(exs_ctx *c, const exs_scf_inputs *in)
     const int nat = c->natmtot, maxaa = c->maxaa, maxnlo = std::max(c->maxnlo, 1);
     // h_a: aa(f, f', ias) -> planar [ias][f'][f] with leading dim ldh
     if (!keep_mt) {
+        c->x_valid = false;
         std::vector<double> re((size_t)nat * c->ldh * c->ldh, 0.0), im(re.size(), 0.0);
         for (int ias = 0; ias < nat; ias++)
             for (int f2 = 0; f2 < maxaa; f2++)
@@ -592,7 +593,6 @@ int exs_set_scf_inputs(exs_ctx *c, const exs_scf_inputs *in)
     // the matching systems D_l depend only on the tails: factorised once here
     if (!c->d_dlu) EXS_CUDA(dalloc(&c->d_dlu, (size_t)nat * (c->lmaxapw + 1) * exs::DLU_STRIDE));
     EXS_CUDA(exs::launch_match_dlu(c->params(), c->d_dlu, s));
-    if (!keep_mt) c->x_valid = false;
     if (c->oz_on() && !c->x_valid)   // slices of the new h_a and loa, in place
         EXS_CUDA(exs::launch_x(c, s));
     EXS_CUDA(cudaStreamSynchronize(s));

@@ -443,8 +443,9 @@ cudaError_t launch_ring_atom(const CUtensorMap *mapA, const CUtensorMap *mapX, c
 // Operands of h_a and loa for the active split arithmetic.
 inline cudaError_t launch_x(exs_ctx *c, cudaStream_t s)
 {
-    c->x_valid = true;
-    return c->oz_sch.mod ? launch_ring_x(c->params(), c->oz_atom_args(), c->oz_ring, s)
-                         : launch_oz_x(c->params(), c->oz_atom_args(), c->oz_sch, s);
+    const cudaError_t e = c->oz_sch.mod ? launch_ring_x(c->params(), c->oz_atom_args(), c->oz_ring, s)
+                                        : launch_oz_x(c->params(), c->oz_atom_args(), c->oz_sch, s);
+    c->x_valid = e == cudaSuccess;
+    return e;
 }
 }  // namespace exs

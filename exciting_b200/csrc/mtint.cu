@@ -745,6 +745,7 @@ int enqueue_hmlint(exs_ctx *c, MtState &m, int lmaxvr, const double *apwfr, cons
     const size_t naa = (size_t)maxaa * maxaa * nat, nloa = (size_t)maxnlo * maxaa * nat;
     if (want_out) MT_CUDA(grow(&m.d_out, &m.out_cap, naa + nloa));
     // rows and columns past a species' own block stay zero
+    c->x_valid = false;
     MT_CUDA(cudaMemsetAsync(c->d_haa_r, 0, sizeof(double) * nat * c->ldh * c->ldh, s));
     MT_CUDA(cudaMemsetAsync(c->d_haa_i, 0, sizeof(double) * nat * c->ldh * c->ldh, s));
     MT_CUDA(cudaMemsetAsync(c->d_loa_r, 0, sizeof(double) * nat * c->ldlo * maxaa, s));
@@ -766,7 +767,6 @@ int enqueue_hmlint(exs_ctx *c, MtState &m, int lmaxvr, const double *apwfr, cons
     MT_CUDA(launch_radial(a, m, 0, ngroup + 1, 0, a.lmmaxvr + 1, s));   // potential groups + CH_KIN
     mt_angular_kernel<<<dim3((m.maxrows + 31) / 32, (m.maxrows + 7) / 8, nat), 256, 0, s>>>(a);
     MT_CUDA(cudaGetLastError());
-    c->x_valid = false;
     if (c->oz_on() && c->d_xs)
         MT_CUDA(exs::launch_x(c, s));
     return EXS_OK;
