@@ -289,14 +289,15 @@ __global__ void apwalm_to_planes_kernel(DevParams p, int ngp, const exs_complex 
 }
 
 // (I + h1aa) A for the IORA overlap (overlapsetup.f90:72-87):
-// C(f2) = A(f2) + sum_io1 h1aa(io1, io2, l, ias) A(f1), f = (l, m, io).  One
-// block row per (atom, l) (one per atom walks 162 rows in a thread: 80 us for
-// nine k-points of the eight-atom cell, 47 us with l apart).
+// C(f2) = A(f2) + sum_io1 h1aa(io1, io2, l, ias) A(f1), f = (l, m, io).  Blocks
+// per (atom, l) (one per atom walks 162 rows in a thread: 80 us for nine
+// k-points of the eight-atom cell, 47 us with l apart): the l beside the G in
+// the grid's x, which alone goes past 65,535, the atoms in y.
 __global__ void iora_planes_kernel(DevParams p, const KDesc *ks)
 {
     const KDesc k = ks[blockIdx.z];
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    const int ias = blockIdx.y / (p.lmaxmat + 1), l = blockIdx.y % (p.lmaxmat + 1);
+    const int l = blockIdx.x % (p.lmaxmat + 1), ias = blockIdx.y;
+    const int g = blockIdx.x / (p.lmaxmat + 1) * blockDim.x + threadIdx.x;
     if (g >= p.npad) return;
     const AtomDesc &at = p.atoms[ias];
     const int *apw = p.apword + (size_t)(p.lmaxapw + 1) * at.species;
@@ -398,7 +399,7 @@ cudaError_t launch_apwalm_to_planes(const DevParams &p, int ngp, const exs_compl
 cudaError_t launch_iora_planes(const DevParams &p, const KDesc *d_k, int nk, int ngp_max, cudaStream_t s)
 {
     (void)ngp_max;
-    dim3 grid((p.npad + 127) / 128, p.natmtot * (p.lmaxmat + 1), nk);
+    dim3 grid((p.npad + 127) / 128 * (p.lmaxmat + 1), p.natmtot, nk);
     iora_planes_kernel<<<grid, 128, 0, s>>>(p, d_k);
     return cudaGetLastError();
 }
