@@ -382,10 +382,15 @@ __device__ __forceinline__ void ring_pace(int *pace, int me, int ncl, int step)
     st_relaxed_gpu(pace + me, step);
 }
 
-// An arrival that orders nothing but the tensor-memory reads before it, which
-// tcgen05.wait::ld has completed: a release here would make the warp wait
-// until its residue stores are performed (per-atom products of 64 atoms: 2.19 ms
-// with release, 1.36 ms without).
+// An arrival that orders nothing but the tensor-memory reads before it.  Those
+// need no release: the warp waits for its loads (tcgen05.wait::ld), every lane
+// fences them (tcgen05.fence::before_thread_sync), and an mbarrier arrival and a
+// wait, both relaxed at cluster scope, with the issuer's after_thread_sync order
+// them before its MMAs (the pattern that PTX gives for tcgen05.ld and MMAs in
+// different threads).  A release would make the warp wait until its residue
+// stores are performed (per-atom products of 64 atoms: 2.19 ms with release, 1.36 ms
+// without; with a release ahead of the product's own stores, all columns
+// loaded first, 27 k-points of the eight-atom cell still 6.06 against 5.62 ms).
 __device__ __forceinline__ void mbar_arrive_relaxed(uint32_t cluster_addr)
 {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
@@ -624,7 +629,7 @@ oz_plane_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant_
 #pragma unroll
                     for (int o = 0; o < C::NB; o++) {
                         // the epilogues of both CTAs must have read this accumulator's previous product
-                        if (k0 == 0 && use > 0 && !mbar_wait_ab(&acce[buf + o], (use - 1) & 1, abort, rg.wait)) {
+                        if (k0 == 0 && use > 0 && !mbar_wait_ab<true>(&acce[buf + o], (use - 1) & 1, abort, rg.wait)) {
                             bad = true;
                             if (o > 0) {             // H's MMAs of this stage are under way: commit them too
                                 umma_commit_2sm(&empty[st]);

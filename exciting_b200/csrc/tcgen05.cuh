@@ -45,14 +45,32 @@ __device__ __forceinline__ bool mbar_try_suspend(uint64_t *bar, uint32_t parity)
     return ok != 0;
 }
 
+// The pair of an arrival with relaxed.cluster semantics (tcgen05 operations
+// only, see mbar_arrive_relaxed in oz_ring.cu).
+__device__ __forceinline__ bool mbar_try_relaxed(uint64_t *bar, uint32_t parity, uint32_t suspend_ns)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(suspend_ns)
+        : "memory");
+    return ok != 0;
+}
+
 // Bounded wait (limit cycles; 0: OZ_WAIT_CYCLES) that also gives up as soon
 // as another role raised `abort`.
+template <bool RELAXED = false>
 __device__ __forceinline__ bool mbar_wait_ab(uint64_t *bar, uint32_t parity, volatile int *abort, long long limit)
 {
     const long long t0 = clock64();
     const long long lim = limit > 0 ? limit : OZ_WAIT_CYCLES;
     while (true) {
-        if (limit > 0 ? mbar_try(bar, parity) : mbar_try_suspend(bar, parity)) return true;
+        if (RELAXED ? mbar_try_relaxed(bar, parity, limit > 0 ? 0 : 10000)
+                    : (limit > 0 ? mbar_try(bar, parity) : mbar_try_suspend(bar, parity)))
+            return true;
         if (*abort) return false;
         if (clock64() - t0 > lim) {
             *abort = 1;
