@@ -21,7 +21,6 @@ from __future__ import annotations
 
 import argparse
 import json
-import math
 import os
 import statistics
 import subprocess
@@ -179,19 +178,6 @@ def _hbm_peak():
         return 6650.0      # earlier measurement on this pool's B200s
 
 
-# The moduli the products run in (pairwise coprime, every prime factor 1 mod 4: two int8 products per
-# modulus make a complex one), largest first; the fewest that hold products of 2 b bits with one bit of margin.
-RINGS = (241, 233, 229, 221, 205, 197, 193, 181, 173, 157, 149, 137, 113, 109, 101, 97)
-
-
-def rings_for(bits):
-    lm, n = 0.0, 0
-    while lm - 1e-9 < bits + 2:
-        lm += math.log2(RINGS[n])
-        n += 1
-    return n
-
-
 def split_scheme(args, sys_):
     """(int8 planes per operand, int8 products per H/O tile, dtype text,
     precision text) of the split-precision mode args.precision."""
@@ -199,10 +185,10 @@ def split_scheme(args, sys_):
         S = args.slices
         return (S, S * (S + 1) // 2, "i8 slices, f64 recombination",
                 "split int8 x%d slices (tcgen05), FP64 recombination" % S)
-    from exciting_b200.fvsystem import ozaki_moduli
+    from exciting_b200.fvsystem import ozaki_moduli, ozaki_rings
     K = apw_rows(sys_)
     ps, _, b, bx, _ = ozaki_moduli(args.moduli, K, sys_.basis.maxaa)
-    r = rings_for(2 * b)
+    r = len(ozaki_rings(args.moduli, K, sys_.basis.maxaa)[0])       # two int8 products (planes) per modulus
     return (2 * r, 2 * r, "i8 residues mod %d coprime moduli, CRT in 96-bit fixed point, f64 scaling" % r,
             "split int8 (the %d-modulus plan: columns scaled by their 2-norms to %d bits, exact integer products "
             "modulo %d moduli, two per modulus; tcgen05), Chinese-remainder recombination" % (len(ps), b, r))
@@ -371,12 +357,12 @@ def run_reference(args):
     return 0
 
 
-def launches_per_setup(precision, sys_=None, ngp=(), planes=0):
+def launches_per_setup(precision, sys_=None, ngp=(), moduli=0):
     """Kernel launches of one batched setup call.  Moduli: match, the column
     norms and residues of A, the per-atom products and their recombination, the
     norms and residues of B, the H/O products and their recombination, the
     local-orbital blocks; the products in chunks of at most 4 GB of residues
-    (sys_, ngp, planes: more than one for the 216-atom cell).  Slices: match, the
+    (sys_, ngp, moduli: more than one for the 216-atom cell).  Slices: match, the
     A split, the per-atom products, the B split, the H/O tiles, the blocks.
     FP64: match, h_a A, the APW-lo rows, H and O, the blocks."""
     if precision != "ozaki_mod":
@@ -389,8 +375,9 @@ def launches_per_setup(precision, sys_=None, ngp=(), planes=0):
         rows = [b.napw_atom(a) + sum(2 * l + 1 for l in b.lorbl[b.atom_species[a]]) for a in range(sys_.natmtot)]
         blocks = (max(rows) + 255) // 256
         nb = ((max(rows) + blocks - 1) // blocks + 15) // 16 * 16
-        at_planes = planes - 2 if planes == 28 else planes                     # 13 of the 14 moduli at b = 49, bx = 45
-        tile = [planes * 512 * cols, at_planes * 256 * nb]
+        from exciting_b200.fvsystem import ozaki_rings
+        ps, n_atom = ozaki_rings(moduli, K, b.maxaa)
+        tile = [2 * len(ps) * 512 * cols, 2 * n_atom * 256 * nb]
         n = [sum(ho_tiles(g, 256, cols) for g in ngp),
              sum((g + 255) // 256 for g in ngp) * sum((r + nb - 1) // nb for r in rows)]
         top = len(ngp) * ho_tiles(max(ngp), 256, cols)                         # the buffer is sized for ngkmax
@@ -621,7 +608,6 @@ def run_ours(args, emit=True):
     gks = s.gksets()[: args.nk]
     nk = len(gks)
     st = Setup(s, max_batch=nk)
-    planes = 0
     if args.precision != "fp64":
         st.set_precision(args.precision, args.slices if args.precision == "ozaki" else args.moduli)
         planes, products, dtype_text, prec_text = split_scheme(args, s)
@@ -869,7 +855,7 @@ def run_ours(args, emit=True):
                 "sample": f"{cpu_n} k-points of the 27-k set in {cpu_dt:.1f} s by the FP64 CPU "
                           "restatement (C + OpenMP + OpenBLAS zgemm)"},
             "clocks": clocks,
-            "gpu_launches": launches_per_setup(args.precision, s, ngp, planes) * args.steps,
+            "gpu_launches": launches_per_setup(args.precision, s, ngp, args.moduli) * args.steps,
             "setup_flops_per_step": setup_flops(s, gks),
             "accuracy": accuracy,
             "fp64_path_value": fp64_value,
@@ -1400,7 +1386,7 @@ def run_large(args):
                                              "unit": "TFLOP/s", "frac": fl / (mt_ms * 1e-3) / 1e12 / peak64}},
             "cpu_baseline": cpu,
             "clocks": clocks,
-            "gpu_launches": launches_per_setup(prec, s, [gks_all[0].ngp], planes) * args.steps,
+            "gpu_launches": launches_per_setup(prec, s, [gks_all[0].ngp], args.moduli) * args.steps,
             "setup_flops_per_step": setup_flops(s, gks_all) / len(gks_all),
             "accuracy": acc,
             "fp64_path_value": fp64_value,

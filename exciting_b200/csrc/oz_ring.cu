@@ -8,7 +8,8 @@
 // scaled column has norm <= 2^b (1 + eps)); the rows of h_a and loa likewise
 // to bx bits.  By the Cauchy-Schwarz inequality the integer products obey
 // |X| <= 2^(2b) (1 + eps)^2 (H, O) and 2^(b+bx) (1 + eps)^2 (h_a A, loa A),
-// whatever K.  b and bx are the plan's (oz_mod_plan, exs_ozaki_moduli).
+// whatever K.  b and bx are the plan's (oz_mod_plan, exs_ozaki_moduli), the
+// moduli below exs_ozaki_rings'.
 //
 // Products.  The moduli p_m of the table below are pairwise coprime and all
 // their prime factors are 1 mod 4, so an integer i_m with i_m^2 = -1 (mod p_m)
@@ -416,7 +417,7 @@ __device__ __forceinline__ void tma_load_4d_2sm(uint32_t dst, const CUtensorMap 
 template <bool RUNS>
 struct RingUnits {
     int ncl, np, count, tile, P, full_end, rest, rest_tile, rest_P;
-    __device__ RingUnits(int ntiles, int ncl_, int np_, int c) : ncl(ncl_), np(np_)
+    __host__ __device__ RingUnits(int ntiles, int ncl_, int np_, int c) : ncl(ncl_), np(np_)
     {
         const int full = ntiles / ncl;
         full_end = full * ncl;
@@ -424,13 +425,14 @@ struct RingUnits {
         const int pairs = rest * np;                       // rest < ncl
         const int first = RUNS ? (int)((long long)pairs * c / ncl) : c;
         const int mine = RUNS ? (int)((long long)pairs * (c + 1) / ncl) - first : (pairs - c + ncl - 1) / ncl;
+        const int div = rest > 0 ? rest : 1;
         count = full * np + mine;
-        rest_tile = full_end + (RUNS ? first / np : first % max(rest, 1));
-        rest_P = RUNS ? first % np : first / max(rest, 1);
+        rest_tile = full_end + (RUNS ? first / np : first % div);
+        rest_P = RUNS ? first % np : first / div;
         tile = full > 0 ? c : rest_tile;
         P = full > 0 ? 0 : rest_P;
     }
-    __device__ void next()
+    __host__ __device__ void next()
     {
         if (tile >= full_end) {                            // among the remaining tiles
             if (RUNS) {
@@ -1411,5 +1413,16 @@ extern "C" int exs_ozaki_moduli(int n, int K, int kx, int *n_out, int *p, unsign
     if (b) *b = s.b;
     if (bx) *bx = s.bx;
     if (h) *h = s.h;
+    return EXS_OK;
+}
+
+extern "C" int exs_ozaki_rings(int n, int K, int kx, int *n_ho, int *n_atom, int *p)
+{
+    exs::OzScheme s{};
+    exs::OzRing r{};
+    if (exs::oz_mod_plan(n, K, kx, &s) != 0 || exs::oz_ring_plan(s.b, s.bx, &r) != 0) return EXS_ERR_ARG;
+    if (n_ho) *n_ho = r.n;
+    if (n_atom) *n_atom = r.at.n;
+    for (int m = 0; p && m < r.n; m++) p[m] = r.p[m];
     return EXS_OK;
 }

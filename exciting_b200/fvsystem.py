@@ -537,6 +537,18 @@ def ozaki_moduli(n: int, K: int, kx: int):
     return [int(x) for x in p[:m]], [int(x) for x in c[:m]], b.value, bx.value, h.value
 
 
+def ozaki_rings(n: int, K: int, kx: int):
+    """The moduli the device forms that plan's products in, those of H and O;
+    and how many of them, from the first, the per-atom products take."""
+    lib = abi.load()
+    n_ho, n_atom = ctypes.c_int(), ctypes.c_int()
+    p = np.zeros(16, dtype=np.int32)
+    rc = lib.exs_ozaki_rings(int(n), int(K), int(kx), ctypes.byref(n_ho), ctypes.byref(n_atom), _ptr(p))
+    if rc != 0:
+        raise abi.ExsError(rc, "no modular plan for n=%d K=%d kx=%d" % (n, K, kx))
+    return [int(x) for x in p[: n_ho.value]], n_atom.value
+
+
 def multi_graph(setups, batches) -> SetupGraph:
     """One CUDA graph over several contexts (exs_graph_create_multi).
 

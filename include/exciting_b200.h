@@ -166,11 +166,17 @@ int exs_set_precision(exs_ctx *ctx, int mode, int slices);
  * c[m] = round(2^(64+h) y_m / p_m) mod 2^64 with y_m = (M / p_m)^-1 mod p_m
  * and its headroom h (2^(2b + 2) <= M and 2^(b + bx + h + 2) <= M).  The
  * device forms the same integer products exactly modulo a second set of
- * moduli, in which -1 is a square (csrc/oz_ring.cu).  n = 0 picks n as
- * exs_set_precision does; *n_out receives it.  Any output pointer may be
+ * moduli (exs_ozaki_rings).  n = 0 picks n as exs_set_precision does; *n_out receives it.  Any output pointer may be
  * NULL.  Host only. */
 int exs_ozaki_moduli(int n, int K, int kx, int *n_out, int *p, unsigned long long *c, int *b, int *bx,
                      int *h);
+
+/* The moduli in which the device forms the integer products of that plan:
+ * pairwise coprime, -1 a square in each (two int8 products per modulus make a
+ * complex one), largest first: p[0..*n_ho-1] for H and O, the first *n_atom of
+ * them for h_a A and loa A; their products exceed 2^(2b + 2) and 2^(b + bx + 2).
+ * p holds up to 16.  Any output pointer may be NULL.  Host only. */
+int exs_ozaki_rings(int n, int K, int kx, int *n_ho, int *n_atom, int *p);
 
 /* Replaces  call match(ngp, gpc, tpgpc, sfacgp, apwalm)   (src/match.f90:13).
  *   gpc(ngkmax), tpgpc(2, ngkmax), sfacgp(ngkmax, natmtot)  in;
